@@ -213,6 +213,30 @@ __device__ __forceinline__ int sample_action(const GameParams& G, const float* r
   return result;
 }
 
+// sample_action from a row's stored BF16 strategy (four words, two slots each).
+// The running sums of sig over the legal slots are both the total and the
+// cumulative thresholds; they never decrease, so the first legal slot whose
+// threshold reaches r is the number of slots whose threshold does not (an
+// illegal slot repeats the one before it).  A NaN total (infinite regrets) passes
+// no threshold and falls back, as the comparison chain does.
+__device__ __forceinline__ int sample_stored(const GameParams& G, const uint4& st, uint32_t vm, float u) {
+  const uint32_t w[4] = {st.x, st.y, st.z, st.w};
+  float c[kSlots];
+  float total = 0.0f;
+#pragma unroll
+  for (int a = 0; a < kSlots; ++a) {
+    const float sig = __uint_as_float((a & 1) ? (w[a >> 1] & 0xFFFF0000u) : (w[a >> 1] << 16));
+    if ((vm >> a) & 1) total = __fadd_rn(total, sig);
+    c[a] = total;
+  }
+  int result = 0;
+  const float r = __fmul_rn(u, total);
+#pragma unroll
+  for (int a = 0; a < kSlots; ++a) result += !(r <= c[a]);
+  if (total < 1e-7f || result == kSlots) result = passive_fallback(G, vm);
+  return result;
+}
+
 // Regret-matched strategy of a node (cfr_gpu.cu:784-797); illegal slots are 0.
 __device__ __forceinline__ void node_strategy(const float* reg, uint32_t vm, float* strat) {
   float sum_r = 0.0f;

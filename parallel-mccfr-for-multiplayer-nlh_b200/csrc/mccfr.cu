@@ -53,70 +53,99 @@ constexpr int kRefBlock = 128;
 // Folds one player-update's accumulators into the rows it touched and zeroes
 // them (the sparse equivalent of kernel_clamp_regrets, cfr_gpu.cu:1018-1022).
 // Eight lanes per row, lane a owning action slot a: each row field is read and
-// written as one coalesced vector, and the row's regret matching gathers the
-// eight regrets with shuffles and sums them in slot order, like node_strategy.
+// written as one coalesced vector, and sums over slots gather the eight values
+// with shuffles and add them in slot order, like node_strategy.  The rows are
+// random lines of a table of many GB, so the bytes and the dependent reads of a
+// row are what it costs: the first line holds all that an opponents' row needs,
+// da is loaded with it when the list entry says the updating player claimed the
+// row, and only what changed is written.
 // `group`/`ngroups` enumerate the 8-lane groups working on this table.
 __device__ __forceinline__ void apply_rows(const GameParams& G, const TableView& tv, const Sched* sched, double rinv,
                                            unsigned group, unsigned ngroups, bool leader) {
+  __shared__ unsigned s_end[kListShards];  // rows of shards 0..s, so that one index runs over all of them
   const uint32_t uid = update_id(sched, G.N);
+  if (threadIdx.x < kListShards) {
+    unsigned n = *list_count(tv, uid & 1, threadIdx.x);
+#pragma unroll
+    for (int o = 1; o < kListShards; o <<= 1) {
+      const unsigned y = __shfl_up_sync(0xFFFFFFFFu, n, o);
+      if ((int)threadIdx.x >= o) n += y;
+    }
+    s_end[threadIdx.x] = n;
+  }
+  __syncthreads();
+  const unsigned total = s_end[kListShards - 1];
   const size_t per_shard = (tv.mask + 1) / kListShards;
   const double w = G.lcfr ? (double)(float)sched->iteration : 1.0;
   const double s32 = 2.3283064365386962890625e-10;  // 2^-32
   const int a = threadIdx.x & 7;
   const unsigned gmask = 0xFFu << (threadIdx.x & 24);
-  unsigned wide_rows = 0;  // rows whose second line was written back (counted by lane 0 of each group)
-  for (int sh = 0; sh < kListShards; ++sh) {
-  const unsigned n = *list_count(tv, uid & 1, sh);
-  const unsigned* list = tv.touched + (size_t)sh * per_shard;
-  for (unsigned i = group; i < n; i += ngroups) {
-    const unsigned long long slot = list[i];
-    // every field of both lines is loaded at once: a row's accumulators are
-    // zero unless its flags say they were written, so no load waits on another
-    const uint32_t m = (uint32_t)(*row_tag(tv, slot) & 0xFF);
-    const unsigned long long cnt = *row_cnt(tv, slot);
-    const long long canon = (long long)(cnt & 0xFFFFFFFFull);
-    const long long su = (long long)*row_su(tv, slot);
-    const unsigned flags = *row_flags(tv, slot);
+  unsigned wide_rows = 0;  // rows with accumulators on the second line (counted by lane 0 of each group)
+  int sh = 0;
+  for (unsigned i = group; i < total; i += ngroups) {
+    while (i >= s_end[sh]) ++sh;
+    const unsigned e = tv.touched[(size_t)sh * per_shard + (i - (sh ? s_end[sh - 1] : 0u))];
+    const unsigned long long slot = e & ~kListWide;
+    const bool claimed = (e & kListWide) != 0;
     float* regp = reinterpret_cast<float*>(row_reg(tv, slot));
     float* ssp = reinterpret_cast<float*>(row_ssum(tv, slot));
     long long* dap = reinterpret_cast<long long*>(row_da(tv, slot));
     long long* dsp = reinterpret_cast<long long*>(row_ds(tv, slot));
+    long long da_a = 0;
+    if (claimed) da_a = dap[a];
+    const ulonglong2 cs = *reinterpret_cast<const ulonglong2*>(row_cnt(tv, slot));     // cnt, su
+    const ulonglong2 vf = *reinterpret_cast<const ulonglong2*>(row_visits(tv, slot));  // visits, flags
+    const uint32_t m = (uint32_t)(*row_tag(tv, slot) & 0xFF);
     const float r_a = regp[a];
     const float s_a = ssp[a];
-    const long long da_a = dap[a];
-    const long long ds_a = dsp[a];
-    // strategy of the canonical mask from the snapshot regrets (node_strategy)
-    float sum_r = 0.0f;
-#pragma unroll
-    for (int b = 0; b < 8; ++b) {
-      const float rb = __shfl_sync(gmask, r_a, b, 8);
-      if ((m >> b) & 1) sum_r = __fadd_rn(sum_r, fmaxf(0.0f, rb));
-    }
+    const unsigned long long cnt = cs.x;
+    const long long canon = (long long)(cnt & 0xFFFFFFFFull), su = (long long)cs.y;
+    const bool wide = claimed || (cnt >> 32) != (unsigned long long)canon;
+    const bool has_ds = ((unsigned)vf.y & kFlagDs) != 0;
+    if (wide && !claimed) da_a = dap[a];
+    long long dsv = 0;
+    if (has_ds) dsv = dsp[a];
     const bool in = (m >> a) & 1;
-    float strat_a = 0.0f;
-    if (in) strat_a = (sum_r > 1e-7f) ? __fdiv_rn(fmaxf(0.0f, r_a), sum_r) : __fdiv_rn(1.0f, (float)__popc(m));
+    if (canon) {
+      // strategy of the canonical mask from the snapshot regrets (node_strategy)
+      float sum_r = 0.0f;
+#pragma unroll
+      for (int b = 0; b < 8; ++b) {
+        const float rb = __shfl_sync(gmask, r_a, b, 8);
+        if ((m >> b) & 1) sum_r = __fadd_rn(sum_r, fmaxf(0.0f, rb));
+      }
+      float strat_a = 0.0f;
+      if (in) strat_a = (sum_r > 1e-7f) ? __fdiv_rn(fmaxf(0.0f, r_a), sum_r) : __fdiv_rn(1.0f, (float)__popc(m));
+      dsv += in ? canon * fix_s(strat_a) : 0ll;
+    }
     const long long dr = da_a - (in ? su : 0ll);
-    const long long dsv = ds_a + (in ? canon * fix_s(strat_a) : 0ll);
     float r = __fadd_rn(r_a, __double2float_rn(__dmul_rn((double)dr, rinv)));
     if (G.cfr_plus) r = (r < 0.0f) ? 0.0f : r;
-    regp[a] = r;
-    ssp[a] = __fadd_rn(s_a, __double2float_rn(__dmul_rn(__dmul_rn((double)dsv, s32), w)));
-    if (flags & kFlagDa) dap[a] = 0;
-    if (flags & kFlagDs) dsp[a] = 0;
-    if (a == 0) {
-      *row_visits(tv, slot) += cnt >> 32;
-      *row_cnt(tv, slot) = 0;
-      *row_su(tv, slot) = 0;
-      *row_flags(tv, slot) = 0;
-      wide_rows += (flags & (kFlagDa | kFlagDs)) ? 1u : 0u;
+    const float s = __fadd_rn(s_a, __double2float_rn(__dmul_rn(__dmul_rn((double)dsv, s32), w)));
+    if (__float_as_uint(s) != __float_as_uint(s_a)) ssp[a] = s;
+    const bool moved = __float_as_uint(r) != __float_as_uint(r_a);
+    if (moved) regp[a] = r;
+    if (__any_sync(gmask, moved)) {
+      // the row's sampling strategy follows its regrets
+      float sum = 0.0f;
+#pragma unroll
+      for (int b = 0; b < 8; ++b) sum = __fadd_rn(sum, fmaxf(0.0f, __shfl_sync(gmask, r, b, 8)));
+      reinterpret_cast<__nv_bfloat16*>(row_strat(tv, slot))[a] =
+          __float2bfloat16_rn(sum > 1e-7f && r > 0.0f ? __fdiv_rn(r, sum) : 0.0f);
     }
-  }
+    if (da_a) dap[a] = 0;
+    if (has_ds) dsp[a] = 0;
+    if (a == 0) {
+      *reinterpret_cast<ulonglong2*>(row_cnt(tv, slot)) = make_ulonglong2(0ull, 0ull);
+      *reinterpret_cast<ulonglong2*>(row_visits(tv, slot)) = make_ulonglong2(vf.x + (cnt >> 32), 0ull);
+      wide_rows += wide || has_ds ? 1u : 0u;
+    }
   }
   wide_rows = __reduce_add_sync(0xFFFFFFFFu, wide_rows);
   if ((threadIdx.x & 31) == 0 && wide_rows) atomicAdd(wide_count(tv, uid & 1), wide_rows);
   if (leader) {
     const uint32_t next = (uid + 1) & 1;
-    for (int sh = 0; sh < kListShards; ++sh) *list_count(tv, next, sh) = 0;
+    for (int k = 0; k < kListShards; ++k) *list_count(tv, next, k) = 0;
     *wide_count(tv, next) = 0;
   }
 }
@@ -234,6 +263,7 @@ __global__ void k_import_dense(const TableView tv, const float* __restrict__ dr,
     row_reg(tv, slot)[1] = make_float4(r[4], r[5], r[6], r[7]);
     row_ssum(tv, slot)[0] = make_float4(q[0], q[1], q[2], q[3]);
     row_ssum(tv, slot)[1] = make_float4(q[4], q[5], q[6], q[7]);
+    store_strategy(tv, (unsigned long long)slot, r);
   }
 }
 
@@ -251,6 +281,9 @@ __global__ void k_import_rows(const TableView tv, const unsigned long long* __re
     row_ssum(tv, slot)[0] = ssum[2 * i];
     row_ssum(tv, slot)[1] = ssum[2 * i + 1];
     *row_visits(tv, slot) = visits[i];
+    const float4 a = reg[2 * i], b = reg[2 * i + 1];
+    const float r[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+    store_strategy(tv, (unsigned long long)slot, r);
   }
 }
 

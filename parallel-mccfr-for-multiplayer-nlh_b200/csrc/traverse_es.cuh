@@ -274,7 +274,6 @@ __device__ __forceinline__ int es_step(const GameParams& G, const TableView& tv,
         return 2;
       }
       EsFrame& F = fr.at(L.sp++);
-      mark_deltas(tv, (unsigned long long)slot);
       F.st = cur;
       node_strategy(reg, vm, F.strat);
       F.vh = 0.0f;
@@ -291,7 +290,7 @@ __device__ __forceinline__ int es_step(const GameParams& G, const TableView& tv,
                           G.seed_lo, G.seed_hi);
       const int s = sample_action(G, reg, vm, uniform01(d.x));
       if (slot >= 0) {
-        if (touch_row(tv, (unsigned long long)slot, uid, vm)) {
+        if (touch_row(tv, (unsigned long long)slot, uid, vm, 0u)) {
           atomicAdd(row_cnt(tv, slot), (1ull << 32) | 1ull);
         } else {
           atomicAdd(row_cnt(tv, slot), 1ull << 32);
@@ -319,7 +318,7 @@ __device__ __forceinline__ int es_step(const GameParams& G, const TableView& tv,
       const float vh = F.vh;
       const long long fv = fix_r(vh, rscale);
       atomicAdd(row_cnt(tv, F.slot), 1ull << 32);
-      if (touch_row(tv, F.slot, uid, F.vm)) {
+      if (touch_row(tv, F.slot, uid, F.vm, kListWide)) {
         atomicAdd(row_su(tv, F.slot), (unsigned long long)fv);
       } else {
         long long dr[kSlots];

@@ -136,10 +136,10 @@ __device__ __noinline__ float lv_showdown(int N, int up, uint32_t folded, uint32
 
 // A sampled opponent's visit whose mask is not the row's canonical one: its
 // strategy weights go to the accumulators directly.
-__device__ __forceinline__ void lv_off_canonical(const TableView& tv, unsigned long long slot, uint32_t vm,
-                                                 const float* reg) {
+__device__ __noinline__ void lv_off_canonical(const TableView tv, unsigned long long slot, uint32_t vm) {
   atomicAdd(row_cnt(tv, slot), 1ull << 32);
-  float strat[kSlots];
+  float reg[kSlots], strat[kSlots];
+  load_regrets(tv, (long long)slot, reg);
   node_strategy(reg, vm, strat);
   long long dw[kSlots];
 #pragma unroll
@@ -236,17 +236,15 @@ __device__ __forceinline__ int lv_step(const GameParams& G, const TableView& tv,
       return kLvUp;
     }
     const ulonglong2 kt = __ldcg(reinterpret_cast<const ulonglong2*>(row_ptr(tv, rs)));
-    const float4* rp = row_reg(tv, rs);
-    const float4 r0 = __ldg(rp), r1 = __ldg(rp + 1);
+    const uint4 st = __ldg(row_strat(tv, rs));
     const U4 d = philox(U4{cur.aux, uid, (uint32_t)cur.path, (uint32_t)(cur.path >> 32) | 0x80000000u},
                         G.seed_lo, G.seed_hi);
     if (kt.x != key) __stcg(row_key(tv, rs), key);
-    const float reg[kSlots] = {r0.x, r0.y, r0.z, r0.w, r1.x, r1.y, r1.z, r1.w};
-    const int s = sample_action(G, reg, vm, uniform01(d.x));
-    if (touch_row_from(tv, rs, uid, vm, kt.y)) {
+    const int s = sample_stored(G, st, vm, uniform01(d.x));
+    if (touch_row_from(tv, rs, uid, vm, kt.y, 0u)) {
       atomicAdd(row_cnt(tv, rs), (1ull << 32) | 1ull);
     } else {
-      lv_off_canonical(tv, rs, vm, reg);
+      lv_off_canonical(tv, rs, vm);
     }
     pend.player = player;
     pend.action = s;
@@ -259,16 +257,15 @@ __device__ __forceinline__ int lv_step(const GameParams& G, const TableView& tv,
     return kLvUp;
   }
   // sampled opponent: strategy sum, then one action (es_step's opponent branch)
-  float reg[kSlots];
-  load_regrets(tv, slot, reg);
+  const uint4 st = slot >= 0 ? __ldg(row_strat(tv, (unsigned long long)slot)) : make_uint4(0u, 0u, 0u, 0u);
   const U4 d = philox(U4{cur.aux, uid, (uint32_t)cur.path, (uint32_t)(cur.path >> 32) | 0x80000000u}, G.seed_lo,
                       G.seed_hi);
-  const int s = sample_action(G, reg, vm, uniform01(d.x));
+  const int s = sample_stored(G, st, vm, uniform01(d.x));
   if (slot >= 0) {
-    if (touch_row(tv, (unsigned long long)slot, uid, vm)) {
+    if (touch_row(tv, (unsigned long long)slot, uid, vm, 0u)) {
       atomicAdd(row_cnt(tv, slot), (1ull << 32) | 1ull);
     } else {
-      lv_off_canonical(tv, (unsigned long long)slot, vm, reg);
+      lv_off_canonical(tv, (unsigned long long)slot, vm);
     }
   }
   pend.player = player;
@@ -598,7 +595,6 @@ k_level_back(const GameParams G, const TableView tv, const Sched* __restrict__ s
     for (int a = 0; a < kSlots; ++a)
       if ((vm >> a) & 1) vh = __fadd_rn(vh, __fmul_rn(strat[a], v[a]));
     const long long fv = fix_r(vh, rscale);
-    mark_deltas(tv, slot);
 #pragma unroll
     for (int a = 0; a < kSlots; ++a)
       if ((vm >> a) & 1) atomicAdd(row_da(tv, slot) + a, (unsigned long long)(fix_r(v[a], rscale) - fv));
