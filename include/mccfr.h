@@ -130,7 +130,11 @@ typedef struct mccfr_config {
 
 /* Traversal forms (external sampling). */
 enum {
-  MCCFR_FORM_AUTO = 0,   /* the level-synchronous form */
+  /* every warp walks its own traversals' trees, 32 seeds at a time, in one
+     launch per update; games whose paths may hold more than 31 decisions of the
+     updating player (no raise cap and a depth cut above 31, or a cap above 6)
+     take the level-synchronous form */
+  MCCFR_FORM_AUTO = 0,
   /* one lane per traversal, depth first, with an explicit frame stack
      (persistent lanes pulling traversals from a work counter) */
   MCCFR_FORM_LANES = 1,
@@ -291,8 +295,8 @@ int mccfr_eval7(mccfr_handle* h, const uint8_t* cards, uint16_t* ranks, size_t n
 int mccfr_eval7_device(mccfr_handle* h, const uint8_t* dev_cards,
                        uint16_t* dev_ranks, size_t n, float* ms);
 
-/* The level-synchronous form's counts of the handle's last external-sampling
-   update: seeds[L] (level 0: the update's traversals) and updating-player
+/* Level counts of the handle's last external-sampling update in the default or
+   the level-synchronous form: seeds[L] (level 0: the update's traversals) and updating-player
    nodes[L] reached from level L, for L < min(cap, *levels), and the seeds left
    to the depth-first walk because the buffers were full.  *levels = 0 before
    the first such update.  No reference counterpart (a tuning aid). */
@@ -341,7 +345,7 @@ typedef struct mccfr_batch_tuning {
 } mccfr_batch_tuning;
 /* Batch forms.  PERSISTENT: per phase one persistent traversal launch over all
    tables (the fields above tune it).  TABLE_GRAPHS: each table's own update
-   kernels (for external sampling the level-synchronous form) as independent
+   kernels (for external sampling in its configured form) as independent
    branches of one CUDA graph per iteration, so the tables' launches run
    concurrently; the tuning fields above are then unused.  Both give every
    table the rows of training it alone. */

@@ -28,13 +28,17 @@ struct GameParams {
   const uint32_t* range_cdf;    // [N][1326] cumulative range weights, 2^31 scale
   // action slots
   int8_t kind[kSlots];
-  int16_t num[kSlots], den[kSlots];
+  int16_t num[kSlots];
   uint8_t m_fold, m_check, m_call, m_allin, m_raise, m_check_kind;
   uint8_t n_fallback;
   uint8_t fallback[kSlots];
   uint8_t default_slot;
   int stack_base;  // chips behind plus chips already in: stack + (subgame) pot share
-  int8_t den_shift[kSlots];  // log2(den[a]) when den[a] is a power of two, else -1
+  // floor(num * pot / den) of a pot raise as floor(2 * num * pot * frac_mul / 2^32) >> frac_sh
+  // (frac_factors; 0 for a minimum raise, whose target is the minimum itself)
+  uint32_t frac_mul[kSlots];
+  uint8_t frac_sh[kSlots];
+  uint8_t n_raise, raise_slot[kSlots];  // the raise slots in order
 };
 
 // ---------------------------------------------------------------------------
@@ -122,12 +126,29 @@ __host__ __device__ __forceinline__ int min_raise_to(int cb, int lfr, int bb) {
   return (cb == 0) ? imax(1, bb) : cb + imax(lfr, bb);
 }
 
+// Multiplier and shift of an exact division by den for numerators below 2^24
+// (num <= 16, a pot of at most 6 x 65535 chips): with den in [2^l, 2^(l+1)),
+// m = ceil(2^(31+l) / den) fits 32 bits and exceeds 2^(31+l) / den by less than
+// 1, so x * m / 2^(31+l) has x / den's floor while x * den < 2^(31+l), which
+// x < 2^24 and l <= 14 keep.  The factor 2 in the numerator makes den = 1 fit.
+__host__ __device__ __forceinline__ void frac_factors(int den, uint32_t& mul, uint8_t& sh) {
+  mul = 0;
+  sh = 0;
+  if (den <= 0) return;
+  int l = 0;
+  while ((2 << l) <= den) ++l;
+  mul = (uint32_t)(((1ull << (31 + l)) + (unsigned)den - 1) / (unsigned)den);
+  sh = (uint8_t)l;
+}
+
 __host__ __device__ __forceinline__ int raise_target(const GameParams& G, int a, int pot, int cb, int mrt) {
-  if (G.kind[a] == 4 /*RAISE_MIN*/) return mrt;
-  // num * pot >= 0, so a power-of-two denominator is an exact shift
-  const int x = G.num[a] * pot, sh = G.den_shift[a];
-  const int frac = sh >= 0 ? (x >> sh) : x / G.den[a];
-  return imax(mrt, cb + imax(1, frac));
+  const uint32_t x = 2u * (uint32_t)(G.num[a] * pot);
+#ifdef __CUDA_ARCH__
+  const uint32_t q = __umulhi(x, G.frac_mul[a]);
+#else
+  const uint32_t q = (uint32_t)(((uint64_t)x * G.frac_mul[a]) >> 32);
+#endif
+  return imax(mrt, cb + imax(1, (int)(q >> G.frac_sh[a])));
 }
 
 __host__ __device__ __forceinline__ uint32_t valid_mask(const GameParams& G, int pot, int stack, int to_call,
@@ -147,10 +168,11 @@ __host__ __device__ __forceinline__ uint32_t valid_mask(const GameParams& G, int
   const int mrt = min_raise_to(cb, lfr, G.bb);
   const int maxrt = cb + head;
   if (maxrt >= mrt) {
-#pragma unroll
-    for (int a = 0; a < kSlots; ++a)
-      if ((G.m_raise >> a) & 1)
-        if (raise_target(G, a, pot, cb, mrt) <= maxrt) m |= 1u << a;
+#pragma unroll 1
+    for (int i = 0; i < G.n_raise; ++i) {
+      const int a = G.raise_slot[i];
+      if (raise_target(G, a, pot, cb, mrt) <= maxrt) m |= 1u << a;
+    }
   }
   return m | G.m_allin;
 }

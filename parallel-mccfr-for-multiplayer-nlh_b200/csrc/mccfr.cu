@@ -32,6 +32,7 @@
 #include "traverse_ref.cuh"
 #include "traverse_es.cuh"
 #include "traverse_levels.cuh"
+#include "traverse_walk.cuh"
 #include "showdown.cuh"
 #include "batched.cuh"
 #include "best_response.h"
@@ -403,6 +404,12 @@ struct mccfr_handle {
   int level_last_batch = 0;  // traversals of the last update enqueued in the level form
   LevelBufs lb{};
   int grid_expand = 0, grid_back = 0, grid_dfs = 0;  // resident blocks on this handle's device
+  // walk form: every resident warp's node records, and the update's counters
+  void* d_walk = nullptr;
+  int walk_blocks = 0;    // blocks the records were allocated for
+  int walk_resident = 0;  // resident blocks on this handle's device
+  bool last_walk = false;  // the last external-sampling update ran in the walk form
+  WalkBufs wb{};
   // graph of one iteration
   cudaGraphExec_t graph = nullptr;
   int graph_batch = -1;
@@ -530,16 +537,16 @@ void make_params(const mccfr_config& c, GameParams& g) {
   for (int a = 0; a < 8; ++a) {
     g.kind[a] = (int8_t)(a < c.num_actions ? c.action_kind[a] : -1);
     g.num[a] = (int16_t)(a < c.num_actions ? c.action_num[a] : 0);
-    g.den[a] = (int16_t)(a < c.num_actions ? std::max(1, c.action_den[a]) : 1);
-    g.den_shift[a] = -1;
-    for (int k = 0; k < 15; ++k)
-      if (g.den[a] == (1 << k)) g.den_shift[a] = (int8_t)k;
     const int k = g.kind[a];
     if (k == MCCFR_ACT_FOLD) g.m_fold |= 1u << a;
     if (k == MCCFR_ACT_CHECK || k == MCCFR_ACT_CHECK_CALL) g.m_check |= 1u << a;
     if (k == MCCFR_ACT_CALL || k == MCCFR_ACT_CHECK_CALL) g.m_call |= 1u << a;
     if (k == MCCFR_ACT_ALL_IN) g.m_allin |= 1u << a;
-    if (k == MCCFR_ACT_RAISE_MIN || k == MCCFR_ACT_RAISE_POT) g.m_raise |= 1u << a;
+    if (k == MCCFR_ACT_RAISE_MIN || k == MCCFR_ACT_RAISE_POT) {
+      g.m_raise |= 1u << a;
+      g.raise_slot[g.n_raise++] = (uint8_t)a;
+      if (k == MCCFR_ACT_RAISE_POT) frac_factors((int16_t)std::max(1, c.action_den[a]), g.frac_mul[a], g.frac_sh[a]);
+    }
   }
   // Passive fallback order (cfr_gpu.cu:498-508): check, check/call, call, fold,
   // raises in slot order, all-in.
@@ -598,7 +605,9 @@ int record(mccfr_handle* h, cudaEvent_t e, bool capturing) {
   return MCCFR_OK;
 }
 
+bool use_walk(const mccfr_handle* h);
 bool use_levels(const mccfr_handle* h);
+int enqueue_walk(mccfr_handle* h, int batch, float rscale);
 int enqueue_levels(mccfr_handle* h, int batch, float rscale);
 
 // Enqueues one player-update (traverse + apply) reading the device schedule;
@@ -609,7 +618,10 @@ int enqueue_update(mccfr_handle* h, int batch, mccfr_trace* d_trace, cudaEvent_t
   const double rinv = std::ldexp(1.0, -rb);
   HandView hv{h->d_hr, h->d_pre, h->d_cdf};
   if (batch > h->deals_cap) return fail(h, MCCFR_ERR_INVALID_ARG, "deal buffer smaller than the batch");
-  k_deal<<<(batch + 127) / 128, 128, 0, h->stream>>>(h->gp, hv, h->d_sched, batch, h->d_deals);
+  const bool walk = use_walk(h);
+  k_deal<<<(batch + 127) / 128, 128, 0, h->stream>>>(h->gp, hv, h->d_sched, batch, h->d_deals,
+                                                     walk ? reinterpret_cast<uint32_t*>(h->wb.ctl) : nullptr,
+                                                     walk ? (int)(sizeof(WalkCtl) / 4) : 0);
   CK(cudaGetLastError());
   if (ev3 && record(h, ev3[0], capturing)) return MCCFR_ERR_CUDA;
   if (h->cfg.sampling == MCCFR_SAMPLING_REFERENCE) {
@@ -620,8 +632,8 @@ int enqueue_update(mccfr_handle* h, int batch, mccfr_trace* d_trace, cudaEvent_t
     else
       k_traverse_ref<kRefBlock, false><<<grid, kRefBlock, 0, h->stream>>>(h->gp, h->tv, h->d_deals, h->d_sched,
                                                                             batch, rscale, h->d_counters, nullptr);
-  } else if (use_levels(h)) {
-    const int rc = enqueue_levels(h, batch, rscale);
+  } else if (walk || use_levels(h)) {
+    const int rc = walk ? enqueue_walk(h, batch, rscale) : enqueue_levels(h, batch, rscale);
     if (rc) return rc;
   } else {
     launch_traverse_es(h->gp, h->tv, h->d_deals, h->d_sched, batch, rscale, h->d_counters, h->d_work, h->stream,
@@ -635,23 +647,92 @@ int enqueue_update(mccfr_handle* h, int batch, mccfr_trace* d_trace, cudaEvent_t
   return MCCFR_OK;
 }
 
-// Traversal form of the update: the level-synchronous kernels for external
-// sampling unless the config asks for the depth-first lanes.
-bool use_levels(const mccfr_handle* h) {
-  return h->cfg.sampling == MCCFR_SAMPLING_EXTERNAL && h->cfg.traversal_form != MCCFR_FORM_LANES;
-}
-
-// Seed levels of an update: the updating player acts at most raise_cap + 1
-// times per street (once, and once more after each raise of another player),
-// and at most once per node of the depth cut; one more level holds the seeds
-// below its last possible decision.  Capped at kMaxLevels (the deepest level
-// is then walked depth first).
-int level_count(const mccfr_handle* h) {
+// Most decisions of the updating player on a path: at most raise_cap + 1 per
+// street (once, and once more after each raise of another player), and at most
+// one per node of the depth cut.
+int max_decisions(const mccfr_handle* h) {
   const mccfr_config& c = h->cfg;
   const int streets = h->gp.sub_street ? 4 - h->gp.sub_street : 4;
-  int decisions = c.max_depth;
-  if (c.raise_cap > 0) decisions = std::min(decisions, streets * (c.raise_cap + 1));
-  return std::min(decisions + 1, kMaxLevels);
+  return c.raise_cap > 0 ? std::min(c.max_depth, streets * (c.raise_cap + 1)) : c.max_depth;
+}
+
+// Traversal form of an external-sampling update.  The walk form unless the
+// config asks for another; it keeps one node record per decision in reserve, so
+// paths longer than its level counters (no raise cap and a deep depth cut) take
+// the level-synchronous kernels, which leave the deepest level to the depth-first
+// walk.
+bool use_walk(const mccfr_handle* h) {
+  return h->cfg.sampling == MCCFR_SAMPLING_EXTERNAL && h->cfg.traversal_form == MCCFR_FORM_AUTO &&
+         max_decisions(h) < kMaxLevels;
+}
+bool use_levels(const mccfr_handle* h) {
+  return h->cfg.sampling == MCCFR_SAMPLING_EXTERNAL && h->cfg.traversal_form != MCCFR_FORM_LANES && !use_walk(h);
+}
+
+// Seed levels of an update: one per decision and one below the last.  Capped at
+// kMaxLevels (the deepest level is then walked depth first).
+int level_count(const mccfr_handle* h) { return std::min(max_decisions(h) + 1, kMaxLevels); }
+
+void drop_graph(mccfr_handle* h) {
+  if (h->graph) cudaGraphExecDestroy(h->graph);
+  h->graph = nullptr;
+  h->graph_batch = -1;
+}
+
+// Node records of the walk form's warps: as many blocks as are resident, or as
+// the batch has traversals for.  Fewer are tried when the device is short of
+// memory; any number gives the same rows.
+int ensure_walk(mccfr_handle* h, int batch) {
+  if (!h->walk_resident) {
+    int sms = 0, per = 0;
+    CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, h->device));
+    CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_walk<true>, kWalkBlock, 0));
+    h->walk_resident = std::max(1, per) * sms;
+  }
+  const int want = std::min(h->walk_resident, (batch + kWalkWarps - 1) / kWalkWarps);
+  h->wb.decisions = max_decisions(h);
+  if (h->d_walk && h->walk_blocks >= want) return MCCFR_OK;
+  if (h->d_walk) {
+    CK(cudaStreamSynchronize(h->stream));
+    cudaFree(h->d_walk);
+    h->d_walk = nullptr;
+    h->walk_blocks = 0;
+  }
+  drop_graph(h);  // the graph captured the old buffers
+  for (int blocks = want;; blocks = (blocks + 1) / 2) {
+    const size_t nodes = (size_t)blocks * kWalkWarps * kWalkNodes;
+    const cudaError_t e = cudaMalloc(&h->d_walk, nodes * sizeof(WalkNode) + sizeof(WalkCtl));
+    if (e == cudaSuccess) {
+      h->wb.nodes = static_cast<WalkNode*>(h->d_walk);
+      h->wb.ctl = reinterpret_cast<WalkCtl*>(h->wb.nodes + nodes);
+      h->walk_blocks = blocks;
+      return MCCFR_OK;
+    }
+    cudaGetLastError();  // clear the allocation error
+    if (e != cudaErrorMemoryAllocation || blocks == 1)
+      return fail(h, MCCFR_ERR_OOM, "walk buffers: %s", cudaGetErrorString(e));
+  }
+}
+
+// Buffers of the handle's external-sampling form for updates of `batch` traversals.
+int ensure_levels(mccfr_handle* h, int batch);
+int ensure_form(mccfr_handle* h, int batch) {
+  if (use_walk(h)) return ensure_walk(h, batch);
+  return use_levels(h) ? ensure_levels(h, batch) : MCCFR_OK;
+}
+
+int enqueue_walk(mccfr_handle* h, int batch, float rscale) {
+  h->last_walk = true;
+  h->level_last_batch = batch;
+  const int blocks = std::min(h->walk_blocks, (batch + kWalkWarps - 1) / kWalkWarps);
+  WalkBufs wb = h->wb;
+  // a warp takes up to 32 roots at a time, fewer while that would leave other
+  // warps of the launch without
+  wb.grab = std::max(1, std::min(32, batch / (4 * blocks * kWalkWarps)));
+  auto kern = h->tv.direct ? k_walk<true> : k_walk<false>;
+  kern<<<blocks, kWalkBlock, 0, h->stream>>>(h->gp, h->tv, h->d_deals, h->d_sched, batch, rscale, wb, h->d_counters);
+  CK(cudaGetLastError());
+  return MCCFR_OK;
 }
 
 // Node and seed buffers for updates of `batch` traversals: 2^level_log2 node
@@ -739,6 +820,7 @@ int ensure_levels(mccfr_handle* h, int batch) {
 // recorded showdowns evaluated in one pass, the values returned bottom up.
 int enqueue_levels(mccfr_handle* h, int batch, float rscale) {
   const LevelBufs& lb = h->lb;
+  h->last_walk = false;
   h->level_last_batch = batch;
   CK(cudaMemsetAsync(lb.ctl, 0, sizeof(LevelCtl), h->stream));
   k_level_expand<128, 1, true><<<h->grid_expand, 128, 0, h->stream>>>(h->gp, h->tv, h->d_deals, h->d_sched, batch,
@@ -780,7 +862,7 @@ int ensure_deals(mccfr_handle* h, int batch) {
 int ensure_graph(mccfr_handle* h, int batch) {
   {
     int rc = ensure_deals(h, batch);
-    if (!rc && use_levels(h)) rc = ensure_levels(h, batch);
+    if (!rc) rc = ensure_form(h, batch);
     if (rc) return rc;
   }
   if (h->graph && h->graph_batch == batch) return MCCFR_OK;
@@ -933,6 +1015,7 @@ void release(mccfr_handle* h) {
   cudaFree(h->d_counters);
   cudaFree(h->d_work);
   cudaFree(h->d_level);
+  cudaFree(h->d_walk);
   if (h->stream) cudaStreamDestroy(h->stream);
   delete h;
 }
@@ -1255,7 +1338,7 @@ int mccfr_step(mccfr_handle* h, long long iteration, int player, int batch, mccf
     CK(cudaMemsetAsync(d_trace, 0, (size_t)batch * sizeof(mccfr_trace), h->stream));
   }
   int rc = ensure_deals(h, batch);
-  if (rc == MCCFR_OK && use_levels(h)) rc = ensure_levels(h, batch);
+  if (rc == MCCFR_OK) rc = ensure_form(h, batch);
   if (rc == MCCFR_OK) rc = set_sched(h, iteration, player);
   if (rc == MCCFR_OK) rc = enqueue_update(h, batch, d_trace, h->ev);
   if (rc == MCCFR_OK) {
@@ -1747,8 +1830,19 @@ int mccfr_level_counts(mccfr_handle* h, uint32_t* seeds, uint32_t* nodes, int ca
   if (!h || !levels || cap < 0 || (cap && (!seeds || !nodes))) return MCCFR_ERR_INVALID_ARG;
   *levels = 0;
   if (deferred) *deferred = 0;
-  if (!h->d_level) return MCCFR_OK;
+  if (h->last_walk ? !h->d_walk : !h->d_level) return MCCFR_OK;
   CK(cudaSetDevice(h->device));
+  if (h->last_walk) {
+    WalkCtl w;
+    CK(cudaMemcpyAsync(&w, h->wb.ctl, sizeof(w), cudaMemcpyDeviceToHost, h->stream));
+    CK(cudaStreamSynchronize(h->stream));
+    *levels = level_count(h);
+    for (int L = 0; L < *levels && L < cap; ++L) {
+      seeds[L] = L == 0 ? (uint32_t)h->level_last_batch : w.seeds[L - 1];
+      nodes[L] = w.nodes[L];
+    }
+    return MCCFR_OK;
+  }
   static thread_local LevelCtl c;
   CK(cudaMemcpyAsync(&c, h->lb.ctl, sizeof(c), cudaMemcpyDeviceToHost, h->stream));
   CK(cudaStreamSynchronize(h->stream));
@@ -1945,7 +2039,7 @@ int batch_prepare_table_graphs(mccfr_batch* b) {
   for (size_t i = 0; i < b->tables.size(); ++i) {
     mccfr_handle* h = b->tables[i];
     int rc = ensure_deals(h, b->traversals[i]);
-    if (!rc && use_levels(h)) rc = ensure_levels(h, b->traversals[i]);
+    if (!rc) rc = ensure_form(h, b->traversals[i]);
     if (rc) return bfail(b, rc, "table buffers for the batch graph");
   }
   return MCCFR_OK;

@@ -266,8 +266,13 @@ __device__ __forceinline__ void deal_one(const GameParams& G, const int32_t* __r
   for (int i = 0; i < 4; ++i) dst[i] = src[i];
 }
 
+// `ctl`: 128-byte blocks of counters of the traversal that follows, zeroed here
+// so that the update needs no launch for it (may be null).
 __global__ void __launch_bounds__(128) k_deal(const GameParams G, const HandView hv, const Sched* __restrict__ sched,
-                                              int batch, DealRec* __restrict__ out) {
+                                              int batch, DealRec* __restrict__ out, uint32_t* __restrict__ ctl,
+                                              int ctl_words) {
+  if (blockIdx.x == 0)
+    for (int i = threadIdx.x; i < ctl_words; i += blockDim.x) ctl[i] = 0;
   __shared__ uint8_t s_pre[52 * 52];
   for (int i = threadIdx.x; i < 52 * 52 / 4; i += blockDim.x)
     reinterpret_cast<uint32_t*>(s_pre)[i] = __ldg(reinterpret_cast<const uint32_t*>(hv.pre) + i);

@@ -1,0 +1,515 @@
+// traverse_walk.cuh — external-sampling traversal, every warp on its own trees.
+//
+// The same player-update as k_traverse_es and the level kernels (a traversal's
+// tree, cfr_gpu.cu:644-860, cut into *seeds* at the updating player's decision
+// nodes: a traversal's root, or a node's state after one of its legal actions),
+// in one launch.  A warp takes roots from a counter and keeps everything its
+// trees need to itself:
+//   * a stack of seeds in shared memory; an idle lane takes the newest one, loads
+//     its parent's 128-byte record and walks the opponents' sampled nodes until a
+//     terminal or the next updating-player node;
+//   * a pool of node records (betting state, row, children's values) in global
+//     memory that stays in L1/L2 because the newest records are reused first;
+//   * per open node a count of children still out; the lane that delivers the
+//     last value lists the node as ready.  32 ready nodes at a time are regret
+//     matched, added to their rows and handed to their own parents;
+//   * a queue of showdowns, evaluated 32 at a time.
+// So no lane waits for a level of the whole update, no counter in global memory
+// is shared but the roots', and an update is one launch whatever its depth,
+// which is what small updates cost in the level form (38 dependent launches).
+// Taking the newest seed first bounds the pool: a seed is taken only while the
+// pool could still hold one node for every lane that walks and one per remaining
+// decision; with no lane walking one seed at a time always fits (depth first).
+//
+// A step of the warp: fill idle lanes, apply the lanes' pending actions and sort
+// out terminals (their lanes are filled again, until enough lanes stand at a
+// decision), then the decisions together: legal mask, key, and for opponents the
+// row's sector, the draw and the sampled action.  The betting state is packed
+// two seats to a word and the seats still to act are a mask searched from the
+// seat after the last actor (seats act in cyclic order), so that no per-player
+// array is indexed.
+//
+// Every sum that reaches the table is an integer (fixed point) and every draw is
+// keyed by the node's action path, so the rows after an update are those of the
+// other forms, bit for bit, whatever the order of the walks.
+#pragma once
+#include "game.cuh"
+#include "table.cuh"
+#include "traverse_ref.cuh"
+#include "traverse_es.cuh"
+#include "traverse_levels.cuh"
+
+namespace mccfr {
+
+constexpr int kWalkBlock = 128;
+constexpr int kWalkWarps = kWalkBlock / 32;
+constexpr int kWalkNodes = 192;                  // open updating-player nodes of a warp
+constexpr int kWalkSeeds = kSlots * kWalkNodes;  // their children not yet taken
+constexpr int kWalkShow = 64;                    // queued showdowns: 31 left over + 32 of one step
+constexpr uint32_t kWalkRoot = 0xFFFFu;          // parent of a traversal's root
+
+// Counters of one update, zeroed by the deal that precedes the walk.
+struct WalkCtl {
+  unsigned work;                // traversals handed out
+  unsigned pad[31];
+  uint32_t nodes[kMaxLevels];   // updating-player nodes reached from each level's seeds
+  uint32_t seeds[kMaxLevels];   // their children (seeds of the next level)
+};
+
+// Betting state of a lane's walk.
+//   seats = folded | all-in << 8 | still to act << 16 | seat to search from << 24
+//   prog  = street | dealer << 4 | raises << 8 | depth << 16 | level << 24
+struct WalkState {
+  uint32_t inv0, inv1, inv2, bet0, bet1, bet2;  // chips in the hand and in this street, two seats per word
+  int pot, cb;
+  uint64_t path;
+  int lfr;
+  uint32_t abits;
+  uint32_t aux;  // traversal
+  uint32_t seats, prog;
+};
+
+// An open updating-player node: its state, row, own seed, and children's values.
+struct __align__(128) WalkNode {
+  uint4 s0;  // inv0, inv1, inv2, bet0
+  uint4 s1;  // bet1, bet2, pot, cb
+  uint4 s2;  // path, lfr, abits
+  uint4 s3;  // aux, seats, prog, row slot
+  uint4 own; // parent record << 3 | action (its own seed), legal mask
+  float v[kSlots];
+  uint4 pad;
+};
+static_assert(sizeof(WalkNode) == 128, "a node record is one line");
+
+struct WalkShowdown {
+  uint32_t ref, aux, inv0, inv1, inv2;  // ref: seed | folded << 16
+};
+
+// A warp's own lists.
+struct WalkWarp {
+  uint16_t seeds[kWalkSeeds];          // record << 3 | action
+  uint16_t spare[kWalkNodes];          // free records
+  uint16_t ready[kWalkNodes];          // nodes whose children are all in
+  uint32_t out[kWalkNodes / 8];        // children still out, 4 bits per record
+  WalkShowdown show[kWalkShow];
+};
+
+struct WalkBufs {
+  WalkNode* nodes;  // [warps][kWalkNodes]
+  WalkCtl* ctl;
+  int decisions;    // most updating-player decisions on a path
+  int grab;         // traversals a warp takes at a time
+};
+
+__device__ __forceinline__ int seat16(uint32_t w0, uint32_t w1, uint32_t w2, int p) {
+  const uint32_t w = p < 2 ? w0 : (p < 4 ? w1 : w2);
+  return (int)((w >> ((p & 1) << 4)) & 0xFFFFu);
+}
+
+// Adds x to seat p's half word (sums stay below 2^16).
+__device__ __forceinline__ void seat16_add(uint32_t& w0, uint32_t& w1, uint32_t& w2, int p, uint32_t x) {
+  const uint32_t d = x << ((p & 1) << 4);
+  w0 += p < 2 ? d : 0u;
+  w1 += (p >> 1) == 1 ? d : 0u;
+  w2 += p >= 4 ? d : 0u;
+}
+
+// Root state of traversal t (es_begin).
+__device__ __forceinline__ void walk_root(const GameParams& G, const DealRec* D, uint32_t t, WalkState& s) {
+  const int N = G.N;
+  const int dealer = D->dealer;
+  const uint32_t all = (1u << N) - 1;
+  s.aux = t;
+  s.inv0 = s.inv1 = s.inv2 = s.bet0 = s.bet1 = s.bet2 = 0;
+  s.abits = 0;
+  s.path = kPathSeed;
+  s.lfr = G.bb;
+  if (G.sub_street) {
+    const uint32_t x = (uint32_t)(G.sub_pot / N), xx = x | (x << 16);
+    s.inv0 = xx;
+    s.inv1 = N > 3 ? xx : (N > 2 ? x : 0u);
+    s.inv2 = N > 5 ? xx : (N > 4 ? x : 0u);
+    s.pot = G.sub_pot;
+    s.cb = 0;
+    s.seats = (all << 16) | ((uint32_t)seat_after(dealer, 1, N) << 24);
+    s.prog = (uint32_t)G.sub_street | ((uint32_t)dealer << 4);
+  } else {
+    const int next = seat_after(dealer, 1, N);
+    const int sbp = N == 2 ? dealer : next;
+    const int bbp = N == 2 ? next : seat_after(next, 1, N);
+    const int sba = min(G.sb, G.stack), bba = min(G.bb, G.stack);
+    seat16_add(s.bet0, s.bet1, s.bet2, sbp, (uint32_t)sba);
+    seat16_add(s.bet0, s.bet1, s.bet2, bbp, (uint32_t)bba);
+    s.inv0 = s.bet0;
+    s.inv1 = s.bet1;
+    s.inv2 = s.bet2;
+    s.pot = sba + bba;
+    s.cb = bba;
+    uint32_t allin = 0;
+    if (G.stack == sba) allin |= 1u << sbp;
+    if (G.stack == bba) allin |= 1u << bbp;
+    s.seats = (allin << 8) | ((all & ~allin) << 16) | ((uint32_t)seat_after(bbp, 1, N) << 24);
+    s.prog = (uint32_t)dealer << 4;
+  }
+}
+
+// Next seat to act: the first of `mask` at or after `from`, cyclically.
+__device__ __forceinline__ int walk_next(uint32_t seats, int N) {
+  const uint32_t mask = (seats >> 16) & 0xFFu;
+  const int from = (int)(seats >> 24);
+  return seat_after(from, __ffs((int)((mask | (mask << N)) >> from)) - 1, N);
+}
+
+// Applies action a of `player` (es_apply).
+__device__ __forceinline__ void walk_apply(const GameParams& G, WalkState& s, int player, int a) {
+  const int N = G.N;
+  const uint32_t bit = 1u << player;
+  const int after = seat_after(player, 1, N);
+  s.abits = ((s.abits << 3) | (uint32_t)a) & 0x3FFFFFFFu;
+  s.path = path_step(s.path, a);
+  s.prog += 1u << 16;  // depth
+  uint32_t folded = s.seats & 0xFFu, allin = (s.seats >> 8) & 0xFFu, act = ((s.seats >> 16) & 0xFFu) & ~bit;
+  const int k = G.kind[a];
+  if (k == 0) {
+    folded |= bit;
+  } else if (k != 1) {
+    const int pbet = seat16(s.bet0, s.bet1, s.bet2, player);
+    const int pstack = G.stack_base - seat16(s.inv0, s.inv1, s.inv2, player);
+    const int chips = chips_for(G, a, s.pot, pstack, s.cb - pbet, s.cb, s.lfr);
+    seat16_add(s.bet0, s.bet1, s.bet2, player, (uint32_t)chips);
+    seat16_add(s.inv0, s.inv1, s.inv2, player, (uint32_t)chips);
+    s.pot += chips;
+    if (pstack == chips) allin |= bit;
+    const int nbet = pbet + chips;
+    if (nbet > s.cb) {
+      const int rs = nbet - s.cb;
+      if (rs >= s.lfr || s.cb == 0) s.lfr = rs;
+      s.cb = nbet;
+      s.prog = (s.prog & ~0xFF00u) | ((s.prog + 0x100u) & 0xFF00u);  // raises, modulo 256
+      act = ((1u << N) - 1) & ~(folded | allin | bit);
+    }
+  }
+  s.seats = folded | (allin << 8) | (act << 16) | ((uint32_t)after << 24);
+}
+
+// Sorts out what follows an applied action: kLvDone with the terminal's value,
+// kLvShow for a showdown, kLvGoOn at a decision node (after a street change
+// where one is due).
+__device__ __forceinline__ int walk_events(const GameParams& G, WalkState& s, int up, float& value) {
+  const int N = G.N;
+  const uint32_t live = ((1u << N) - 1) & ~s.seats;
+  value = 0.0f;
+  if ((int)((s.prog >> 16) & 0xFFu) >= G.max_depth) return kLvDone;
+  if ((live & (live - 1)) == 0) {
+    const int inv_up = seat16(s.inv0, s.inv1, s.inv2, up);
+    value = (live >> up) & 1 ? (float)(s.pot - inv_up) : (float)(-inv_up);
+    return kLvDone;
+  }
+  if (s.seats & 0x00FF0000u) return kLvGoOn;
+  if ((s.prog & 0xFu) >= 3u) return kLvShow;
+  const uint32_t act = live & ~(s.seats >> 8);
+  if (!act) return kLvShow;
+  s.bet0 = s.bet1 = s.bet2 = 0;
+  s.cb = 0;
+  s.lfr = G.bb;
+  s.prog = (s.prog + 1u + (1u << 16)) & ~0xFF00u;  // street and depth on, no raises
+  s.seats = (s.seats & 0xFFFFu) | (act << 16) | ((uint32_t)seat_after((int)((s.prog >> 4) & 0xFu), 1, N) << 24);
+  return (int)((s.prog >> 16) & 0xFFu) >= G.max_depth ? kLvDone : kLvGoOn;
+}
+
+template <bool DIRECT>
+__global__ void __launch_bounds__(kWalkBlock, 8)
+k_walk(const GameParams G, const TableView tv, const DealRec* __restrict__ deals, const Sched* __restrict__ sched,
+       int batch, float rscale, const WalkBufs wb, Counters* __restrict__ counters) {
+  __shared__ WalkWarp s_warp[kWalkWarps];
+  __shared__ uint32_t s_nodes[kMaxLevels], s_seeds[kMaxLevels];
+  const int lane = threadIdx.x & 31;
+  const unsigned below = (1u << lane) - 1u;
+  WalkWarp& W = s_warp[threadIdx.x >> 5];
+  WalkNode* const pool = wb.nodes + (size_t)(blockIdx.x * kWalkWarps + (threadIdx.x >> 5)) * kWalkNodes;
+  if (threadIdx.x < kMaxLevels) s_nodes[threadIdx.x] = s_seeds[threadIdx.x] = 0;
+  for (int i = lane; i < kWalkNodes; i += 32) W.spare[i] = (uint16_t)(kWalkNodes - 1 - i);
+  for (int i = lane; i < kWalkNodes / 8; i += 32) W.out[i] = 0;
+  __syncthreads();
+  const int N = G.N;
+  const int up = sched->player;
+  const uint32_t uid = update_id(sched, N);
+  // warp-uniform list lengths and counters
+  int n_seeds = 0, n_spare = kWalkNodes, n_ready = 0, n_show = 0;
+  unsigned c_trav = 0, c_vis = 0, c_upd = 0, c_term = 0;
+  bool more = true;  // roots may be left
+  int stalled = 0;
+  // the lane's walk: idle, an action to apply, or standing at a decision
+  enum { kIdle = 0, kApply = 1, kDecide = 2 };
+  int st = kIdle;
+  WalkState s;
+  uint32_t ref = kWalkRoot;  // its seed
+  int pl = -1, pa = 0;       // pending action (pl < 0: a root, nothing to apply)
+
+  // Hands lane values to their parents (ref), listing nodes whose last child it was.
+  auto deliver = [&](bool on, float v) {
+    const bool has = on && ref != kWalkRoot;
+    if (has) pool[ref >> 3].v[ref & 7] = v;
+    __syncwarp();
+    bool last = false;
+    if (has) {
+      const unsigned sh = 4u * ((ref >> 3) & 7u);
+      last = ((atomicSub(&W.out[ref >> 6], 1u << sh) >> sh) & 15u) == 1u;
+    }
+    const unsigned m = __ballot_sync(0xFFFFFFFFu, last);
+    if (last) W.ready[n_ready + __popc(m & below)] = (uint16_t)(ref >> 3);
+    n_ready += __popc(m);
+    __syncwarp();
+  };
+
+  for (;;) {
+    const unsigned idlem = __ballot_sync(0xFFFFFFFFu, st == kIdle);
+    const int n_idle = __popc(idlem);
+    const bool starved = n_idle == 32 && n_seeds == 0 && !more;
+    // seeds the pool has room for: every walking lane may still open one node,
+    // and one seed walked depth first opens one per decision
+    const int room = n_spare - (32 - n_idle) - wb.decisions;
+    const bool low = room < 1;
+
+    if (n_show >= 32 || (n_show && (starved || low))) {
+      // showdowns, one per lane
+      const int nb = min(32, n_show);
+      n_show -= nb;
+      const bool on = lane < nb;
+      const WalkShowdown r = W.show[n_show + (on ? lane : 0)];
+      const uint32_t keep = ref;
+      float v = 0.0f;
+      if (on) {
+        v = lv_showdown(N, up, r.ref >> 16, r.inv0, r.inv1, r.inv2, deals + r.aux);
+        ref = r.ref & 0xFFFFu;
+      }
+      deliver(on, v);
+      ref = keep;
+      continue;
+    }
+    if (n_ready >= 32 || (n_ready && (starved || low))) {
+      // ready nodes, one per lane: regret matching, row sums, own value
+      const int nb = min(32, n_ready);
+      n_ready -= nb;
+      const bool on = lane < nb;
+      const uint32_t keep = ref;
+      float vh = 0.0f;
+      uint32_t id = 0;
+      if (on) {
+        id = W.ready[n_ready + lane];
+        const WalkNode* nd = pool + id;
+        const unsigned long long slot = nd->s3.w;
+        const uint4 own = nd->own;
+        const uint32_t vm = own.y;
+        if (DIRECT) {  // the row's key, which the walk left to this pass
+          const unsigned long long k = __ldcg(row_key(tv, slot));
+          if (k != slot + 1) __stcg(row_key(tv, slot), slot + 1);
+        }
+        claim_row(tv, slot, uid);
+        float reg[kSlots], strat[kSlots], v[kSlots];
+        load_regrets(tv, (long long)slot, reg);
+        const float4 v0 = *reinterpret_cast<const float4*>(nd->v), v1 = *reinterpret_cast<const float4*>(nd->v + 4);
+        v[0] = v0.x; v[1] = v0.y; v[2] = v0.z; v[3] = v0.w;
+        v[4] = v1.x; v[5] = v1.y; v[6] = v1.z; v[7] = v1.w;
+        node_strategy(reg, vm, strat);
+#pragma unroll
+        for (int a = 0; a < kSlots; ++a)
+          if ((vm >> a) & 1) vh = __fadd_rn(vh, __fmul_rn(strat[a], v[a]));
+        const long long fv = fix_r(vh, rscale);
+#pragma unroll
+        for (int a = 0; a < kSlots; ++a)
+          if ((vm >> a) & 1) atomicAdd(row_da(tv, slot) + a, (unsigned long long)(fix_r(v[a], rscale) - fv));
+        atomicAdd(row_cnt(tv, slot), 1ull << 32);
+        ref = own.x;
+      }
+      __syncwarp();
+      if (on) W.spare[n_spare + lane] = (uint16_t)id;
+      n_spare += nb;
+      c_upd += nb;
+      deliver(on, vh);
+      ref = keep;
+      continue;
+    }
+    if (starved) break;
+
+    // ---- fill idle lanes: the newest seeds, else new roots
+    bool filled = false;
+    if (n_idle) {
+      const int allowed = n_idle == 32 ? max(room, 1) : room;
+      const int rank = __popc(idlem & below);
+      const int take = min(min(n_idle, n_seeds), allowed);
+      if (take > 0) {
+        n_seeds -= take;
+        if (st == kIdle && rank < take) {
+          ref = W.seeds[n_seeds + take - 1 - rank];
+          const WalkNode* nd = pool + (ref >> 3);
+          const uint4 a = nd->s0, b = nd->s1, c = nd->s2, d = nd->s3;
+          s.inv0 = a.x; s.inv1 = a.y; s.inv2 = a.z; s.bet0 = a.w;
+          s.bet1 = b.x; s.bet2 = b.y; s.pot = (int)b.z; s.cb = (int)b.w;
+          s.path = (uint64_t)c.x | ((uint64_t)c.y << 32);
+          s.lfr = (int)c.z; s.abits = c.w;
+          s.aux = d.x; s.seats = d.y; s.prog = d.z;
+          s.prog += 1u << 24;  // one level down
+          pl = up;
+          pa = (int)(ref & 7u);
+          st = kApply;
+        }
+        filled = true;
+      } else if (n_seeds == 0 && more && allowed > 0) {
+        const int want = min(min(n_idle, allowed), wb.grab);
+        unsigned base = 0;
+        if (lane == 0) base = atomicAdd(&wb.ctl->work, (unsigned)want);
+        base = __shfl_sync(0xFFFFFFFFu, base, 0);
+        const int got = base < (unsigned)batch ? min(want, (int)((unsigned)batch - base)) : 0;
+        if (got < want) more = false;
+        if (st == kIdle && rank < got) {
+          walk_root(G, deals + base + rank, base + (uint32_t)rank, s);
+          ref = kWalkRoot;
+          pl = -1;
+          st = kApply;
+        }
+        c_trav += got;
+        filled = got > 0;
+      }
+    }
+
+    // ---- pending actions and what follows from them
+    if (__any_sync(0xFFFFFFFFu, st == kApply)) {
+      stalled = 0;
+      int r = -1;
+      float v = 0.0f;
+      if (st == kApply) {
+        if (pl >= 0) walk_apply(G, s, pl, pa);
+        r = walk_events(G, s, up, v);
+        st = r == kLvGoOn ? kDecide : kIdle;
+      }
+      const unsigned showm = __ballot_sync(0xFFFFFFFFu, r == kLvShow);
+      const unsigned donem = __ballot_sync(0xFFFFFFFFu, r == kLvDone);
+      c_term += __popc(showm) + __popc(donem);
+      if (r == kLvShow) {
+        WalkShowdown& q = W.show[n_show + __popc(showm & below)];
+        q.ref = ref | (s.seats << 16);
+        q.aux = s.aux;
+        q.inv0 = s.inv0;
+        q.inv1 = s.inv1;
+        q.inv2 = s.inv2;
+      }
+      n_show += __popc(showm);
+      if (donem) deliver(r == kLvDone, v);
+      __syncwarp();
+    }
+    // lanes freed by terminals are filled again before the decisions run
+    const unsigned decm = __ballot_sync(0xFFFFFFFFu, st == kDecide);
+    if (filled && __popc(decm) < 28 && (n_seeds > 0 || more)) continue;
+    if (!decm) {
+      // every round of the loop above takes, fills or finishes something; a round
+      // that does not would never end
+      if (++stalled > 8) {
+        if (lane == 0) atomicOr(tv.err, kErrStackOverflow);
+        break;
+      }
+      continue;
+    }
+
+    // ---- decisions
+    bool isup = false;
+    uint32_t vm = 0;
+    long long slot = -1;
+    c_vis += __popc(decm);
+    if (st == kDecide) {
+      const int player = walk_next(s.seats, N);
+      const int street = (int)(s.prog & 0xFu);
+      const uint32_t cw = __ldg(deals[s.aux].ctx + player);
+      const int to_call = s.cb - seat16(s.bet0, s.bet1, s.bet2, player);
+      vm = valid_mask(G, s.pot, G.stack_base - seat16(s.inv0, s.inv1, s.inv2, player), to_call, s.cb, s.lfr,
+                      (int)((s.prog >> 8) & 0xFFu));
+      uint32_t hb, bkt;
+      if (G.sub_street) {  // exact combo; the river card once it is dealt
+        hb = cw & 0xFFFF;
+        bkt = (street == 3 && G.sub_street == 2) ? (cw >> 16) : 0u;
+      } else {
+        hb = cw & 0xFF;
+        bkt = street ? ((cw >> (8 * street)) & 0xFF) : 0u;
+      }
+      const unsigned long long key = info_key(G, player, hb, bkt, street, s.abits, s.path);
+      isup = player == up;
+      // in a direct-mapped table the updating player's row is left to the ready pass
+      slot = DIRECT ? (long long)(key - 1) : table_insert<1>(tv, key);
+      if (!isup) {
+        const bool ok = DIRECT || slot >= 0;
+        ulonglong2 kt = make_ulonglong2(0ull, 0ull);
+        uint4 sg = make_uint4(0u, 0u, 0u, 0u);
+        if (ok) {
+          kt = __ldcg(reinterpret_cast<const ulonglong2*>(row_ptr(tv, (unsigned long long)slot)));
+          sg = __ldcg(row_strat(tv, (unsigned long long)slot));
+        }
+        const U4 d = philox(U4{s.aux, uid, (uint32_t)s.path, (uint32_t)(s.path >> 32) | 0x80000000u}, G.seed_lo,
+                            G.seed_hi);
+        if (DIRECT && kt.x != key) __stcg(row_key(tv, (unsigned long long)slot), key);
+        pl = player;
+        pa = sample_stored(G, sg, vm, uniform01(d.x));
+        st = kApply;
+        if (ok) {
+          if (touch_row_from(tv, (unsigned long long)slot, uid, vm, kt.y, 0u))
+            atomicAdd(row_cnt(tv, (unsigned long long)slot), (1ull << 32) | 1ull);
+          else
+            lv_off_canonical(tv, (unsigned long long)slot, vm);
+        }
+      }
+    }
+    // ---- updating-player nodes: a record and one seed per legal action
+    if (__any_sync(0xFFFFFFFFu, isup)) {
+      const unsigned full = __ballot_sync(0xFFFFFFFFu, isup && slot < 0);  // no row: nothing to update
+      bool open = isup && slot >= 0;
+      unsigned upm = __ballot_sync(0xFFFFFFFFu, open);
+      if (__popc(upm) > n_spare) {  // cannot happen while seeds are taken within `room`
+        if (lane == 0) atomicOr(tv.err, kErrStackOverflow);
+        open = false;
+        upm = 0;
+      }
+      const int k = open ? __popc(vm) : 0;
+      int before = 0, total = 0;
+#pragma unroll
+      for (int b = 0; b < 4; ++b) {
+        const unsigned kb = __ballot_sync(0xFFFFFFFFu, (k >> b) & 1);
+        before += __popc(kb & below) << b;
+        total += __popc(kb) << b;
+      }
+      const int cnt = __popc(upm);
+      if (open) {
+        const uint32_t id = W.spare[n_spare - 1 - __popc(upm & below)];
+        WalkNode* nd = pool + id;
+        nd->s0 = make_uint4(s.inv0, s.inv1, s.inv2, s.bet0);
+        nd->s1 = make_uint4(s.bet1, s.bet2, (uint32_t)s.pot, (uint32_t)s.cb);
+        nd->s2 = make_uint4((uint32_t)s.path, (uint32_t)(s.path >> 32), (uint32_t)s.lfr, s.abits);
+        nd->s3 = make_uint4(s.aux, s.seats, s.prog, (uint32_t)slot);
+        nd->own = make_uint4(ref, vm, 0u, 0u);
+        atomicAdd(&W.out[id >> 3], (unsigned)k << (4u * (id & 7u)));
+        int o = n_seeds + before;
+        for (uint32_t left = vm; left; left &= left - 1) W.seeds[o++] = (uint16_t)((id << 3) | (uint32_t)(__ffs(left) - 1));
+        const int level = (int)(s.prog >> 24);
+        atomicAdd(&s_nodes[level], 1u);
+        atomicAdd(&s_seeds[level], (unsigned)k);
+      }
+      n_spare -= cnt;
+      n_seeds += total;
+      __syncwarp();
+      if (full) deliver(isup && slot < 0, 0.0f);
+      if (isup) st = kIdle;
+    }
+  }
+  if (lane == 0) {
+    if (c_trav) atomicAdd(&counters->traversals, (unsigned long long)c_trav);
+    if (c_vis) atomicAdd(&counters->visits, (unsigned long long)c_vis);
+    if (c_upd) atomicAdd(&counters->updates, (unsigned long long)c_upd);
+    if (c_term) atomicAdd(&counters->terminals, (unsigned long long)c_term);
+    if (c_trav) atomicAdd(&counters->evals, (unsigned long long)c_trav * (unsigned)N);
+  }
+  __syncthreads();
+  if (threadIdx.x < kMaxLevels) {
+    if (s_nodes[threadIdx.x]) atomicAdd(&wb.ctl->nodes[threadIdx.x], s_nodes[threadIdx.x]);
+    if (s_seeds[threadIdx.x]) atomicAdd(&wb.ctl->seeds[threadIdx.x], s_seeds[threadIdx.x]);
+  }
+}
+
+}  // namespace mccfr
