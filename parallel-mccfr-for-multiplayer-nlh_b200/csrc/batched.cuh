@@ -60,6 +60,7 @@ __global__ void __launch_bounds__(128) k_deal_batched(const TableDesc* __restric
   for (int i = threadIdx.x; i < (int)(sizeof(PhaseDesc) / 4); i += blockDim.x)
     reinterpret_cast<uint32_t*>(&P)[i] = reinterpret_cast<const uint32_t*>(phase)[i];
   __syncthreads();
+  if (blockIdx.x == 0 && (int)threadIdx.x < P.n) *table_epoch(tables[P.table[threadIdx.x]].tv) += 1;
   const unsigned long long total = P.off[P.n];
   for (unsigned long long g = blockIdx.x * (unsigned long long)blockDim.x + threadIdx.x; g < total;
        g += (unsigned long long)gridDim.x * blockDim.x) {
@@ -110,7 +111,7 @@ k_traverse_batched(const __grid_constant__ PhaseParams P, const DealRec* __restr
   fr.stride = BLOCK;
   const int lane = threadIdx.x & 31;
   int cur_j = -1, up = 0;
-  uint32_t uid = 0;
+  uint32_t uid = 0, epoch = 0;
   unsigned long long c_trav = 0;
   EsCounts c{0, 0, 0};
   auto flush = [&]() {
@@ -163,6 +164,7 @@ k_traverse_batched(const __grid_constant__ PhaseParams P, const DealRec* __restr
         cur_j = j;
         uid = update_id(P.T[j].sched, P.T[j].G.N);
         up = P.T[j].sched->player;
+        epoch = *table_epoch(P.T[j].tv);
       }
       es_begin(P.T[j].G, deals + g, (uint32_t)(g - P.off[j]), L);
       have = true;
@@ -171,7 +173,7 @@ k_traverse_batched(const __grid_constant__ PhaseParams P, const DealRec* __restr
     if (!__any_sync(0xFFFFFFFFu, have || more)) break;
     if (have) {
       const TableDesc& D = P.T[cur_j];
-      if (es_step<W>(D.G, D.tv, uid, up, D.rscale, fr, L, c)) have = false;
+      if (es_step<W>(D.G, D.tv, uid, epoch, up, D.rscale, fr, L, c)) have = false;
     }
   }
   flush();

@@ -53,116 +53,183 @@ constexpr int kRefBlock = 128;
 
 // Folds one player-update's accumulators into the rows it touched and zeroes
 // them (the sparse equivalent of kernel_clamp_regrets, cfr_gpu.cu:1018-1022).
-// Eight lanes per row, lane a owning action slot a: each row field is read and
-// written as one coalesced vector, and sums over slots gather the eight values
-// with shuffles and add them in slot order, like node_strategy.  The rows are
-// random lines of a table of many GB, so the bytes and the dependent reads of a
-// row are what it costs: the first line holds all that an opponents' row needs,
-// da is loaded with it when the list entry says the updating player claimed the
-// row, and only what changed is written.
-// `group`/`ngroups` enumerate the 8-lane groups working on this table.
+// A warp takes 32 words of the bitmaps at a time (the next ones in flight
+// meanwhile), lists the rows marked there in shared memory, rows of sampled visits
+// from the front and wide ones from the back, and folds 32 rows of one kind at a
+// time, one lane per row in nearly ascending address order.  The bytes of the rows
+// are what it costs: a lane has its row's whole first line in flight at once (and
+// da for a wide row), and writes only what changed.
+// `group` of `ngroups`: the warps working on this table.
+constexpr int kApplyBlock = 256;
+constexpr int kApplyList = 1024 + 64;  // rows of 32 words and up to 31 left over of each kind
+
+template <bool WIDE>
+__device__ __forceinline__ void fold_row(const GameParams& G, const TableView& tv, unsigned long long slot, double rinv,
+                                         double w, unsigned& wide_rows) {
+  const double s32 = 2.3283064365386962890625e-10;  // 2^-32
+  void* const cp = row_cnt(tv, slot);  // cnt, su, visits, flags
+  void* const rp = row_reg(tv, slot);
+  void* const sp = row_ssum(tv, slot);
+  unsigned char* const dp = reinterpret_cast<unsigned char*>(row_da(tv, slot));
+  const Sector c = ld_sector(cp), rs = ld_sector(rp), ss = ld_sector(sp);
+  const uint32_t m = (uint32_t)(__ldcg(row_tag(tv, slot)) & 0xFF);
+  long long da[8];
+  if (WIDE) {
+    const Sector d0 = ld_sector(dp), d1 = ld_sector(dp + 32);
+    da[0] = (long long)d0.x; da[1] = (long long)d0.y; da[2] = (long long)d0.z; da[3] = (long long)d0.w;
+    da[4] = (long long)d1.x; da[5] = (long long)d1.y; da[6] = (long long)d1.z; da[7] = (long long)d1.w;
+  }
+  float r[8] = {lo_float(rs.x), hi_float(rs.x), lo_float(rs.y), hi_float(rs.y),
+                lo_float(rs.z), hi_float(rs.z), lo_float(rs.w), hi_float(rs.w)};
+  float s[8] = {lo_float(ss.x), hi_float(ss.x), lo_float(ss.y), hi_float(ss.y),
+                lo_float(ss.z), hi_float(ss.z), lo_float(ss.w), hi_float(ss.w)};
+  const long long canon = (long long)(c.x & 0xFFFFFFFFull), su = (long long)c.y;
+  const bool has_ds = ((unsigned)c.w & kFlagDs) != 0;
+  unsigned moved_s = 0;
+  if (canon || has_ds) {
+    // canonical visits: their count times the strategy of the canonical mask from
+    // the snapshot regrets (node_strategy); the others' weights from ds
+    float sum = 0.0f;
+#pragma unroll
+    for (int a = 0; a < 8; ++a)
+      if ((m >> a) & 1) sum = __fadd_rn(sum, fmaxf(0.0f, r[a]));
+    const float uni = sum > 1e-7f ? 0.0f : __fdiv_rn(1.0f, (float)__popc(m));
+    long long* dsp = reinterpret_cast<long long*>(row_ds(tv, slot));
+#pragma unroll
+    for (int a = 0; a < 8; ++a) {
+      long long d = 0;
+      if (has_ds) {
+        d = dsp[a];
+        if (d) dsp[a] = 0;
+      }
+      if (canon && ((m >> a) & 1)) {
+        float st = uni;
+        if (sum > 1e-7f) st = r[a] > 0.0f ? __fdiv_rn(r[a], sum) : 0.0f;
+        d += canon * fix_s(st);
+      }
+      const float x = __fadd_rn(s[a], __double2float_rn(__dmul_rn(__dmul_rn((double)d, s32), w)));
+      moved_s |= __float_as_uint(x) ^ __float_as_uint(s[a]);
+      s[a] = x;
+    }
+  } else {
+#pragma unroll
+    for (int a = 0; a < 8; ++a) {
+      const float x = __fadd_rn(s[a], 0.0f);
+      moved_s |= __float_as_uint(x) ^ __float_as_uint(s[a]);
+      s[a] = x;
+    }
+  }
+  if (moved_s) {
+    st_sector(sp, Sector{two_floats(s[0], s[1]), two_floats(s[2], s[3]), two_floats(s[4], s[5]),
+                         two_floats(s[6], s[7])});
+  }
+  unsigned moved = 0;
+#pragma unroll
+  for (int a = 0; a < 8; ++a) {
+    // only a wide row has regret terms
+    float x = 0.0f;
+    if (WIDE) x = __double2float_rn(__dmul_rn((double)(da[a] - (((m >> a) & 1) ? su : 0ll)), rinv));
+    x = __fadd_rn(r[a], x);
+    if (G.cfr_plus) x = x < 0.0f ? 0.0f : x;
+    moved |= __float_as_uint(x) ^ __float_as_uint(r[a]);
+    r[a] = x;
+  }
+  if (moved) {
+    st_sector(rp, Sector{two_floats(r[0], r[1]), two_floats(r[2], r[3]), two_floats(r[4], r[5]),
+                         two_floats(r[6], r[7])});
+    __stcg(row_strat(tv, slot), pack_strategy(r));  // the sampling strategy follows the regrets
+  }
+  if (WIDE) {
+    st_sector(dp, Sector{0ull, 0ull, 0ull, 0ull});
+    st_sector(dp + 32, Sector{0ull, 0ull, 0ull, 0ull});
+  }
+  st_sector(cp, Sector{0ull, 0ull, c.z + (c.x >> 32), 0ull});
+  wide_rows += WIDE || has_ds ? 1u : 0u;
+}
+
 __device__ __forceinline__ void apply_rows(const GameParams& G, const TableView& tv, const Sched* sched, double rinv,
                                            unsigned group, unsigned ngroups, bool leader) {
-  __shared__ unsigned s_end[kListShards];  // rows of shards 0..s, so that one index runs over all of them
-  const uint32_t uid = update_id(sched, G.N);
-  if (threadIdx.x < kListShards) {
-    unsigned n = *list_count(tv, uid & 1, threadIdx.x);
-#pragma unroll
-    for (int o = 1; o < kListShards; o <<= 1) {
-      const unsigned y = __shfl_up_sync(0xFFFFFFFFu, n, o);
-      if ((int)threadIdx.x >= o) n += y;
-    }
-    s_end[threadIdx.x] = n;
-  }
-  __syncthreads();
-  const unsigned total = s_end[kListShards - 1];
-  const size_t per_shard = (tv.mask + 1) / kListShards;
+  __shared__ unsigned s_rows[kApplyBlock / 32][kApplyList];
+  unsigned* const list = s_rows[threadIdx.x >> 5];
+  const uint32_t epoch = *table_epoch(tv);
   const double w = G.lcfr ? (double)(float)sched->iteration : 1.0;
-  const double s32 = 2.3283064365386962890625e-10;  // 2^-32
-  const int a = threadIdx.x & 7;
-  const unsigned gmask = 0xFFu << (threadIdx.x & 24);
-  unsigned wide_rows = 0;  // rows with accumulators on the second line (counted by lane 0 of each group)
-  int sh = 0;
-  for (unsigned i = group; i < total; i += ngroups) {
-    while (i >= s_end[sh]) ++sh;
-    const unsigned e = tv.touched[(size_t)sh * per_shard + (i - (sh ? s_end[sh - 1] : 0u))];
-    const unsigned long long slot = e & ~kListWide;
-    const bool claimed = (e & kListWide) != 0;
-    float* regp = reinterpret_cast<float*>(row_reg(tv, slot));
-    float* ssp = reinterpret_cast<float*>(row_ssum(tv, slot));
-    long long* dap = reinterpret_cast<long long*>(row_da(tv, slot));
-    long long* dsp = reinterpret_cast<long long*>(row_ds(tv, slot));
-    long long da_a = 0;
-    if (claimed) da_a = dap[a];
-    const ulonglong2 cs = *reinterpret_cast<const ulonglong2*>(row_cnt(tv, slot));     // cnt, su
-    const ulonglong2 vf = *reinterpret_cast<const ulonglong2*>(row_visits(tv, slot));  // visits, flags
-    const uint32_t m = (uint32_t)(*row_tag(tv, slot) & 0xFF);
-    const float r_a = regp[a];
-    const float s_a = ssp[a];
-    const unsigned long long cnt = cs.x;
-    const long long canon = (long long)(cnt & 0xFFFFFFFFull), su = (long long)cs.y;
-    const bool wide = claimed || (cnt >> 32) != (unsigned long long)canon;
-    const bool has_ds = ((unsigned)vf.y & kFlagDs) != 0;
-    if (wide && !claimed) da_a = dap[a];
-    long long dsv = 0;
-    if (has_ds) dsv = dsp[a];
-    const bool in = (m >> a) & 1;
-    if (canon) {
-      // strategy of the canonical mask from the snapshot regrets (node_strategy)
-      float sum_r = 0.0f;
+  const int lane = threadIdx.x & 31;
+  const unsigned n_words = tv.n_words;
+  unsigned* const wide_bits = tv.bits + n_words;
+  unsigned rows = 0, wide_rows = 0;
+  // words per run: short runs while the table is small, so that every warp has one
+  unsigned run = 32;
+  while (run > 1 && (unsigned long long)run * ngroups > n_words) run >>= 1;
+  const unsigned runs = (n_words + run - 1) / run;
+  unsigned q = group;
+  unsigned word = q * run + lane;
+  bool on = q < runs && lane < run && word < n_words;
+  unsigned b = on ? __ldcg(tv.bits + word) : 0u, bw = on ? __ldcg(wide_bits + word) : 0u;
+  int n_s = 0, n_w = 0;  // rows listed: sampled only, wide
+  for (; q < runs; q += ngroups) {
+    const unsigned cur = word;
+    const unsigned cb = b & ~bw, cw = bw;
+    if (b) __stcg(tv.bits + cur, 0u);
+    if (bw) __stcg(wide_bits + cur, 0u);
+    word = (q + ngroups) * run + lane;
+    on = q + ngroups < runs && lane < run && word < n_words;
+    b = on ? __ldcg(tv.bits + word) : 0u;
+    bw = on ? __ldcg(wide_bits + word) : 0u;
+    const unsigned mine = (unsigned)__popc(cb) | (unsigned)__popc(cw) << 16;
+    unsigned at = mine;
 #pragma unroll
-      for (int b = 0; b < 8; ++b) {
-        const float rb = __shfl_sync(gmask, r_a, b, 8);
-        if ((m >> b) & 1) sum_r = __fadd_rn(sum_r, fmaxf(0.0f, rb));
-      }
-      float strat_a = 0.0f;
-      if (in) strat_a = (sum_r > 1e-7f) ? __fdiv_rn(fmaxf(0.0f, r_a), sum_r) : __fdiv_rn(1.0f, (float)__popc(m));
-      dsv += in ? canon * fix_s(strat_a) : 0ll;
+    for (int o = 1; o < 32; o <<= 1) {
+      const unsigned y = __shfl_up_sync(0xFFFFFFFFu, at, o);
+      if (lane >= o) at += y;
     }
-    const long long dr = da_a - (in ? su : 0ll);
-    float r = __fadd_rn(r_a, __double2float_rn(__dmul_rn((double)dr, rinv)));
-    if (G.cfr_plus) r = (r < 0.0f) ? 0.0f : r;
-    const float s = __fadd_rn(s_a, __double2float_rn(__dmul_rn(__dmul_rn((double)dsv, s32), w)));
-    if (__float_as_uint(s) != __float_as_uint(s_a)) ssp[a] = s;
-    const bool moved = __float_as_uint(r) != __float_as_uint(r_a);
-    if (moved) regp[a] = r;
-    if (__any_sync(gmask, moved)) {
-      // the row's sampling strategy follows its regrets
-      float sum = 0.0f;
-#pragma unroll
-      for (int b = 0; b < 8; ++b) sum = __fadd_rn(sum, fmaxf(0.0f, __shfl_sync(gmask, r, b, 8)));
-      reinterpret_cast<__nv_bfloat16*>(row_strat(tv, slot))[a] =
-          __float2bfloat16_rn(sum > 1e-7f && r > 0.0f ? __fdiv_rn(r, sum) : 0.0f);
+    const unsigned all = __shfl_sync(0xFFFFFFFFu, at, 31);
+    if (all == 0) continue;
+    at -= mine;
+    unsigned o = n_s + (at & 0xFFFFu);
+    for (unsigned left = cb; left; left &= left - 1) list[o++] = (cur << 5) | (unsigned)(__ffs((int)left) - 1);
+    o = kApplyList - 1 - (n_w + (at >> 16));
+    for (unsigned left = cw; left; left &= left - 1) list[o--] = (cur << 5) | (unsigned)(__ffs((int)left) - 1);
+    n_s += (int)(all & 0xFFFFu);
+    n_w += (int)(all >> 16);
+    rows += (unsigned)__popc(cb) + (unsigned)__popc(cw);
+    __syncwarp();
+    while (n_s >= 32) {
+      n_s -= 32;
+      fold_row<false>(G, tv, list[n_s + lane], rinv, w, wide_rows);
     }
-    if (da_a) dap[a] = 0;
-    if (has_ds) dsp[a] = 0;
-    if (a == 0) {
-      *reinterpret_cast<ulonglong2*>(row_cnt(tv, slot)) = make_ulonglong2(0ull, 0ull);
-      *reinterpret_cast<ulonglong2*>(row_visits(tv, slot)) = make_ulonglong2(vf.x + (cnt >> 32), 0ull);
-      wide_rows += wide || has_ds ? 1u : 0u;
+    while (n_w >= 32) {
+      n_w -= 32;
+      fold_row<true>(G, tv, list[kApplyList - 1 - (n_w + lane)], rinv, w, wide_rows);
     }
+    __syncwarp();
   }
+  if (lane < n_s) fold_row<false>(G, tv, list[lane], rinv, w, wide_rows);
+  if (lane < n_w) fold_row<true>(G, tv, list[kApplyList - 1 - lane], rinv, w, wide_rows);
+  __syncwarp();
+  rows = __reduce_add_sync(0xFFFFFFFFu, rows);
   wide_rows = __reduce_add_sync(0xFFFFFFFFu, wide_rows);
-  if ((threadIdx.x & 31) == 0 && wide_rows) atomicAdd(wide_count(tv, uid & 1), wide_rows);
+  if (lane == 0 && rows) {
+    atomicAdd(touched_count(tv, epoch), rows);
+    if (wide_rows) atomicAdd(wide_count(tv, epoch), wide_rows);
+  }
   if (leader) {
-    const uint32_t next = (uid + 1) & 1;
-    for (int k = 0; k < kListShards; ++k) *list_count(tv, next, k) = 0;
-    *wide_count(tv, next) = 0;
+    *touched_count(tv, epoch + 1) = 0;
+    *wide_count(tv, epoch + 1) = 0;
   }
 }
 
-__global__ void __launch_bounds__(256) k_apply(const GameParams G, const TableView tv,
+__global__ void __launch_bounds__(kApplyBlock) k_apply(const GameParams G, const TableView tv,
                                                const Sched* __restrict__ sched, double rinv) {
-  apply_rows(G, tv, sched, rinv, (blockIdx.x * blockDim.x + threadIdx.x) >> 3, (gridDim.x * blockDim.x) >> 3,
+  apply_rows(G, tv, sched, rinv, (blockIdx.x * blockDim.x + threadIdx.x) >> 5, (gridDim.x * blockDim.x) >> 5,
              blockIdx.x == 0 && threadIdx.x == 0);
 }
 
 // Apply of every table in a phase: blockIdx.y selects the table.
-__global__ void __launch_bounds__(256) k_apply_batched(const TableDesc* __restrict__ tables,
+__global__ void __launch_bounds__(kApplyBlock) k_apply_batched(const TableDesc* __restrict__ tables,
                                                        const PhaseDesc* __restrict__ phase) {
   const TableDesc& D = tables[phase->table[blockIdx.y]];
-  apply_rows(D.G, D.tv, D.sched, D.rinv, (blockIdx.x * blockDim.x + threadIdx.x) >> 3,
-             (gridDim.x * blockDim.x) >> 3, blockIdx.x == 0 && threadIdx.x == 0);
+  apply_rows(D.G, D.tv, D.sched, D.rinv, (blockIdx.x * blockDim.x + threadIdx.x) >> 5,
+             (gridDim.x * blockDim.x) >> 5, blockIdx.x == 0 && threadIdx.x == 0);
 }
 
 __global__ void k_advance(Sched* s, int N) {
@@ -264,7 +331,7 @@ __global__ void k_import_dense(const TableView tv, const float* __restrict__ dr,
     row_reg(tv, slot)[1] = make_float4(r[4], r[5], r[6], r[7]);
     row_ssum(tv, slot)[0] = make_float4(q[0], q[1], q[2], q[3]);
     row_ssum(tv, slot)[1] = make_float4(q[4], q[5], q[6], q[7]);
-    store_strategy(tv, (unsigned long long)slot, r);
+    *row_strat(tv, slot) = pack_strategy(r);
   }
 }
 
@@ -284,7 +351,7 @@ __global__ void k_import_rows(const TableView tv, const unsigned long long* __re
     *row_visits(tv, slot) = visits[i];
     const float4 a = reg[2 * i], b = reg[2 * i + 1];
     const float r[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
-    store_strategy(tv, (unsigned long long)slot, r);
+    *row_strat(tv, slot) = pack_strategy(r);
   }
 }
 
@@ -567,6 +634,14 @@ void make_params(const mccfr_config& c, GameParams& g) {
     }
 }
 
+// The table's direct map, and the bitmap words of the rows that keys can own.
+void set_direct(mccfr_handle* h) {
+  h->tv.direct = direct_map(h->cfg);
+  const int kb = h->cfg.key_mode == MCCFR_KEY_FNV26 ? 26 : h->cfg.key_bits;
+  const unsigned long long rows = h->tv.direct ? 1ull << kb : h->cap;
+  h->tv.n_words = (unsigned)((rows + 31) / 32);
+}
+
 int grid_for(long long work, int block) {
   long long g = (work + block - 1) / block;
   return (int)std::max(1LL, std::min(g, 148LL * 64));
@@ -585,16 +660,15 @@ int check_device_error(mccfr_handle* h) {
   return MCCFR_OK;
 }
 
-// Rows the player-update of parity `par` listed (all shards) and folded wide.
-int read_touched(mccfr_handle* h, uint32_t par) {
+// Rows the last player-update touched and folded wide.
+int read_touched(mccfr_handle* h) {
   unsigned c[kCounterBytes / 4];
-  CK(cudaMemcpy(c, h->tv.n_touched, sizeof(c), cudaMemcpyDeviceToHost));
+  CK(cudaMemcpy(c, h->tv.counters, sizeof(c), cudaMemcpyDeviceToHost));
   TableView hv = h->tv;
-  hv.n_touched = c;
-  long long n = 0;
-  for (int sh = 0; sh < kListShards; ++sh) n += *list_count(hv, par, sh);
-  h->touched_last = n;
-  h->wide_last = *wide_count(hv, par);
+  hv.counters = c;
+  const uint32_t epoch = *table_epoch(hv);
+  h->touched_last = *touched_count(hv, epoch);
+  h->wide_last = *wide_count(hv, epoch);
   return MCCFR_OK;
 }
 
@@ -620,6 +694,7 @@ int enqueue_update(mccfr_handle* h, int batch, mccfr_trace* d_trace, cudaEvent_t
   if (batch > h->deals_cap) return fail(h, MCCFR_ERR_INVALID_ARG, "deal buffer smaller than the batch");
   const bool walk = use_walk(h);
   k_deal<<<(batch + 127) / 128, 128, 0, h->stream>>>(h->gp, hv, h->d_sched, batch, h->d_deals,
+                                                     table_epoch(h->tv),
                                                      walk ? reinterpret_cast<uint32_t*>(h->wb.ctl) : nullptr,
                                                      walk ? (int)(sizeof(WalkCtl) / 4) : 0);
   CK(cudaGetLastError());
@@ -641,7 +716,7 @@ int enqueue_update(mccfr_handle* h, int batch, mccfr_trace* d_trace, cudaEvent_t
   }
   CK(cudaGetLastError());
   if (ev3 && record(h, ev3[1], capturing)) return MCCFR_ERR_CUDA;
-  k_apply<<<148 * 8, 256, 0, h->stream>>>(h->gp, h->tv, h->d_sched, rinv);
+  k_apply<<<148 * 3, kApplyBlock, 0, h->stream>>>(h->gp, h->tv, h->d_sched, rinv);
   CK(cudaGetLastError());
   if (ev3 && record(h, ev3[2], capturing)) return MCCFR_ERR_CUDA;
   return MCCFR_OK;
@@ -1193,22 +1268,22 @@ int mccfr_create(const mccfr_config* cfg, mccfr_handle** out) {
   CKC(cudaMemset(h->d_counters, 0, sizeof(Counters)));
   CKC(cudaMalloc(&h->d_work, 256));
   CKC(cudaMemset(h->d_work, 0, 256));
-  // Table rows, the touched list and small counters in one allocation.
+  // Table rows, the touched-row bitmaps and small counters in one allocation.
   h->cap = 1ull << cfg->table_log2;
   const unsigned long long C = h->cap;
-  const size_t bytes_rows = C * kRowBytes, bytes_touch = C * 4, bytes_misc = kCounterBytes;
-  h->block_bytes = bytes_rows + bytes_touch + bytes_misc;
-  CKC(cudaMalloc(&h->d_block, bytes_rows + bytes_touch + bytes_misc));
-  CKC(cudaMemset(h->d_block, 0, bytes_rows + bytes_touch + bytes_misc));
+  const size_t bytes_rows = C * kRowBytes, bytes_bits = C / 4, bytes_misc = kCounterBytes;
+  h->block_bytes = bytes_rows + bytes_bits + bytes_misc;
+  CKC(cudaMalloc(&h->d_block, h->block_bytes));
+  CKC(cudaMemset(h->d_block, 0, h->block_bytes));
   char* base = static_cast<char*>(h->d_block);
   h->tv.rows = reinterpret_cast<unsigned char*>(base);
-  h->tv.touched = reinterpret_cast<unsigned int*>(base + bytes_rows);
-  char* misc = base + bytes_rows + bytes_touch;
-  h->tv.n_touched = reinterpret_cast<unsigned int*>(misc);
+  h->tv.bits = reinterpret_cast<unsigned int*>(base + bytes_rows);
+  char* misc = base + bytes_rows + bytes_bits;
+  h->tv.counters = reinterpret_cast<unsigned int*>(misc);
   h->tv.err = reinterpret_cast<int*>(misc + kCounterBytes - 128);
   h->tv.mask = C - 1;
   h->tv.log2cap = cfg->table_log2;
-  h->tv.direct = direct_map(*cfg);
+  set_direct(h);
   *out = h;
   return MCCFR_OK;
 #undef CKC
@@ -1354,8 +1429,7 @@ int mccfr_step(mccfr_handle* h, long long iteration, int player, int batch, mccf
     h->traverse_ms += t1;
     h->apply_ms += t2;
     h->launches++;
-    // the apply kernel resets the other parity's counters, not this one's
-    read_touched(h, (uint32_t)((iteration - 1) * h->cfg.num_players + player) & 1);
+    read_touched(h);
     rc = check_device_error(h);
   }
   if (rc == MCCFR_OK && trace) {
@@ -1395,9 +1469,8 @@ int mccfr_train(mccfr_handle* h, long long iters, int batch, int verbose, const 
         h->last_apply_ms = t2;
       }
       if (i + 1 == iters) {
-        // rows touched by this iteration's last player-update (its parity's counter
-        // is reset only by the next update's apply)
-        if (read_touched(h, (uint32_t)((base + i) * np + np - 1) & 1)) return MCCFR_ERR_CUDA;
+        // rows touched by this iteration's last player-update
+        if (read_touched(h)) return MCCFR_ERR_CUDA;
       }
     }
     h->launches += h->cfg.num_players;
@@ -1731,7 +1804,7 @@ int mccfr_load_checkpoint_v2(mccfr_handle* h, const char* path) {
       return fail(h, MCCFR_ERR_FORMAT, "%s: row %llu has an invalid key", path, (unsigned long long)i);
   CK(cudaSetDevice(h->device));
   CK(cudaStreamSynchronize(h->stream));
-  CK(cudaMemsetAsync(h->d_block, 0, h->block_bytes, h->stream));  // rows, touched list, counters
+  CK(cudaMemsetAsync(h->d_block, 0, h->block_bytes, h->stream));  // rows, bitmaps, counters
   int rc = MCCFR_OK;
   if (n) {
     std::vector<unsigned long long> keys(n), vis(n);
@@ -2455,11 +2528,11 @@ int mccfr_subgame_reset(mccfr_handle* h, const mccfr_config* cfg, const mccfr_su
   build_preflop_lut(cfg->preflop_mode, cfg->preflop_buckets, pre);
   CK(cudaMemcpyAsync(h->d_pre, pre, sizeof(pre), cudaMemcpyHostToDevice, h->stream));
   CK(cudaMemcpyAsync(h->d_ranges, cdf.data(), cdf.size() * 4, cudaMemcpyHostToDevice, h->stream));
-  CK(cudaMemsetAsync(h->d_block, 0, h->block_bytes, h->stream));  // rows, touched list, counters
+  CK(cudaMemsetAsync(h->d_block, 0, h->block_bytes, h->stream));  // rows, bitmaps, counters
   CK(cudaMemsetAsync(h->d_counters, 0, sizeof(Counters), h->stream));
   CK(cudaStreamSynchronize(h->stream));
   h->cfg = *cfg;
-  h->tv.direct = direct_map(*cfg);
+  set_direct(h);
   make_params(*cfg, h->gp);
   set_subgame_params(h, cfg, sg, nb);
   if (h->graph) {

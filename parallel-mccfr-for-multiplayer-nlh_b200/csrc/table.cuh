@@ -6,7 +6,8 @@
 // is folded from its first line alone:
 //     0  key    u64   0 = empty; linear probing from the key's home slot, or row k-1
 //                       for key k when every key fits (direct map)
-//     8  tag    u64   ((update id + 1) << 8) | canonical action mask of that update
+//     8  tag    u64   (epoch of the last update with sampled visits) << 8 | canonical
+//                       action mask: that of the update's first sampled visit
 //    16  strat[8] bf16  current strategy max(0, reg) / sum over all slots, rounded to
 //                       BF16 as sampling takes it (0 while the sum is at most 1e-7)
 //    32  cnt    u64   (all visits << 32) | visits whose mask is the canonical one
@@ -17,11 +18,13 @@
 //    96  ssum[8] f32  average-strategy sums
 //   128  da[8]  i64   per-action regret deltas, 2^-rb units
 //   192  ds[8]  i64   strategy weights of non-canonical visits, 2^-32 units
-// tag/cnt/su/da/ds/flags are per-update accumulators, zeroed by the apply
-// kernel.  strat follows reg: whoever writes regrets stores it (store_strategy,
-// the apply kernel), so a sampled visit reads one 32-byte sector and divides
-// nothing.  da is non-zero only in a row that the updating player visited: its
-// list entry then carries kListWide, or its visits outnumber its canonical ones.
+// cnt/su/da/ds/flags are per-update accumulators, zeroed by the apply kernel.
+// strat follows reg: whoever writes regrets stores it (pack_strategy), so a sampled visit reads one 32-byte sector and divides nothing.
+//
+// Touched rows are marked in two bitmaps, one bit per row: rows with sampled
+// visits, and rows whose da was added to ("wide": the updating player's).  A mark
+// is a plain OR whose result nobody waits for, the bitmaps fit L2, and the apply
+// kernel meets the rows in address order.
 #pragma once
 #include <cstdint>
 #include <cuda_bf16.h>
@@ -32,23 +35,14 @@ constexpr int kRowBytes = 256;
 constexpr int kOffKey = 0, kOffTag = 8, kOffStrat = 16, kOffCnt = 32, kOffSu = 40, kOffVisits = 48, kOffFlags = 56,
               kOffReg = 64, kOffSsum = 96, kOffDa = 128, kOffDs = 192;
 constexpr unsigned kFlagDs = 1u;
-// Touched-list entry of a row claimed by its updating player (slots use 31 bits):
-// the apply kernel then loads da together with the row's first line.
-constexpr unsigned kListWide = 0x80000000u;
-
-// The touched-row list is cut into kListShards shards by the slot's low bits:
-// shard s holds slots s, s + S, s + 2S, ..., so it never holds more than cap / S
-// rows, and appends spread over S counters instead of queueing on one address.
-constexpr int kListShards = 32;
-constexpr int kCounterStride = 32;  // counters 128 bytes apart (separate lines)
-
 struct TableView {
   unsigned char* rows;       // [cap][256]
-  unsigned int* touched;     // [kListShards][cap / kListShards] rows touched by the update
-  // counters, kCounterStride words apart: entries of each shard by update-id
-  // parity (index parity * kListShards + shard), then, by parity, rows whose
-  // second line the apply kernel folded (index 2 * kListShards + parity)
-  unsigned int* n_touched;
+  unsigned int* bits;        // [2][n_words] touched rows: sampled visits, wide
+  unsigned int n_words;      // words of one bitmap: one bit per row that a key can own
+  // counters, kCounterStride words apart, by epoch parity: touched rows (0, 1) and
+  // wide ones among them (2, 3) of the update, then the epoch (4): updates dealt
+  // since the table was cleared, advanced by the deal that starts each update
+  unsigned int* counters;
   unsigned long long mask;   // cap - 1
   int log2cap;
   int direct;                // every key is at most cap: key k owns row k-1, no probing
@@ -62,6 +56,7 @@ enum : int {
 };
 
 constexpr int kProbeLimit = 1 << 14;
+constexpr int kCounterStride = 32;  // counters 128 bytes apart (separate lines)
 
 __device__ __forceinline__ unsigned char* row_ptr(const TableView& tv, unsigned long long s) {
   return tv.rows + (s << 8);
@@ -71,6 +66,10 @@ __device__ __forceinline__ unsigned long long* row_key(const TableView& tv, unsi
 }
 __device__ __forceinline__ unsigned long long* row_tag(const TableView& tv, unsigned long long s) {
   return reinterpret_cast<unsigned long long*>(row_ptr(tv, s) + kOffTag);
+}
+// Key and tag.
+__device__ __forceinline__ ulonglong2* row_head(const TableView& tv, unsigned long long s) {
+  return reinterpret_cast<ulonglong2*>(row_ptr(tv, s));
 }
 __device__ __forceinline__ uint4* row_strat(const TableView& tv, unsigned long long s) {
   return reinterpret_cast<uint4*>(row_ptr(tv, s) + kOffStrat);
@@ -155,63 +154,72 @@ __device__ __forceinline__ long long table_insert(const TableView& tv, unsigned 
   return -1;
 }
 
-__host__ __device__ __forceinline__ unsigned int* list_count(const TableView& tv, uint32_t parity, int shard) {
-  return tv.n_touched + (size_t)kCounterStride * (parity * kListShards + shard);
+__host__ __device__ __forceinline__ unsigned int* touched_count(const TableView& tv, uint32_t epoch) {
+  return tv.counters + (size_t)kCounterStride * (epoch & 1);
 }
-__host__ __device__ __forceinline__ unsigned int* wide_count(const TableView& tv, uint32_t parity) {
-  return tv.n_touched + (size_t)kCounterStride * (2 * kListShards + parity);
+__host__ __device__ __forceinline__ unsigned int* wide_count(const TableView& tv, uint32_t epoch) {
+  return tv.counters + (size_t)kCounterStride * (2 + (epoch & 1));
 }
-// Bytes of the counter block (list counters, wide-row counters, error flag).
-constexpr size_t kCounterBytes = (size_t)kCounterStride * 4 * (2 * kListShards + 2) + 128;
+__host__ __device__ __forceinline__ unsigned int* table_epoch(const TableView& tv) {
+  return tv.counters + (size_t)kCounterStride * 4;
+}
+// Bytes of the counter block (the five above, then the error flag).
+constexpr size_t kCounterBytes = (size_t)kCounterStride * 4 * 5 + 128;
 
-__device__ __forceinline__ void list_row(const TableView& tv, unsigned long long slot, uint32_t uid, unsigned wide) {
-  const int shard = (int)(slot & (kListShards - 1));
-  const unsigned int i = atomicAdd(list_count(tv, uid & 1, shard), 1u);
-  tv.touched[(size_t)shard * ((tv.mask + 1) / kListShards) + i] = (unsigned int)slot | wide;
+__device__ __forceinline__ void mark_wide(const TableView& tv, unsigned long long slot) {
+  atomicOr(tv.bits + tv.n_words + (unsigned)(slot >> 5), 1u << (slot & 31));
 }
 
-// Marks the row as touched by update `uid`; returns whether `vm` is the
-// update's canonical mask for that row (the first visitor sets it).  `old` is
-// the row's tag as the caller read it (any earlier value will do: a stale one
-// only makes the compare-and-swap fail and return the current tag).  `wide` is
-// kListWide when the visitor adds to da.
-__device__ __forceinline__ bool touch_row_from(const TableView& tv, unsigned long long slot, uint32_t uid,
-                                               uint32_t vm, unsigned long long old, unsigned wide) {
-  const unsigned long long want = ((unsigned long long)(uid + 1) << 8) | vm;
-  unsigned long long* tag = row_tag(tv, slot);
-  if ((old >> 8) != (unsigned long long)(uid + 1)) {
-    const unsigned long long r = atomicCAS(tag, old, want);
-    if (r == old) {
-      list_row(tv, slot, uid, wide);
+// Marks the row as sampled in the update of `epoch` and returns whether `vm` is
+// its canonical mask there (the first visitor's).  `tag` is the row's as the
+// caller read it; a stale one only makes the compare-and-swap fail, and then the
+// row belongs to this update already.
+__device__ __forceinline__ bool touch_row_from(const TableView& tv, unsigned long long slot, uint32_t epoch,
+                                               uint32_t vm, unsigned long long tag) {
+  if ((tag >> 8) != epoch) {
+    tag = atomicCAS(row_tag(tv, slot), tag, ((unsigned long long)epoch << 8) | vm);
+    if ((tag >> 8) != epoch) {
+      atomicOr(tv.bits + (unsigned)(slot >> 5), 1u << (slot & 31));
       return true;
     }
-    old = r;
   }
-  return (uint32_t)(old & 0xFF) == vm;
+  return (uint32_t)(tag & 0xFF) == vm;
 }
-__device__ __forceinline__ bool touch_row(const TableView& tv, unsigned long long slot, uint32_t uid,
-                                          uint32_t vm, unsigned wide) {
-  return touch_row_from(tv, slot, uid, vm, __ldcg(row_tag(tv, slot)), wide);
-}
-
-// Marks the row as touched by update `uid` without claiming a canonical mask
-// (mask 0: every later visitor takes the direct path), for a visitor that adds
-// its whole regret terms to the per-action accumulators; one atomic whose
-// result only decides the list entry.  Update ids only grow, so the maximum
-// leaves a tag of this update (claimed or not) as it is.
-__device__ __forceinline__ void claim_row(const TableView& tv, unsigned long long slot, uint32_t uid) {
-  const unsigned long long old = atomicMax(row_tag(tv, slot), (unsigned long long)(uid + 1) << 8);
-  if ((old >> 8) < (unsigned long long)(uid + 1)) list_row(tv, slot, uid, kListWide);
+__device__ __forceinline__ bool touch_row(const TableView& tv, unsigned long long slot, uint32_t epoch, uint32_t vm) {
+  return touch_row_from(tv, slot, epoch, vm, __ldcg(row_tag(tv, slot)));
 }
 
-// BF16 strategy of a row whose regrets were written from outside an update
-// (imports): the sums and roundings of sampling (cfr_gpu.cu:318-351).
-__device__ __forceinline__ void store_strategy(const TableView& tv, unsigned long long slot, const float* reg) {
+// One 32-byte sector by one lane (256-bit accesses; L2 only).
+struct __align__(32) Sector {
+  unsigned long long x, y, z, w;
+};
+__device__ __forceinline__ Sector ld_sector(const void* p) {
+  Sector s;
+  asm volatile("ld.global.cg.v4.u64 {%0, %1, %2, %3}, [%4];"
+               : "=l"(s.x), "=l"(s.y), "=l"(s.z), "=l"(s.w) : "l"(__cvta_generic_to_global(p)) : "memory");
+  return s;
+}
+__device__ __forceinline__ void st_sector(void* p, const Sector& s) {
+  asm volatile("st.global.cg.v4.u64 [%0], {%1, %2, %3, %4};"
+               :: "l"(__cvta_generic_to_global(p)), "l"(s.x), "l"(s.y), "l"(s.z), "l"(s.w) : "memory");
+}
+__device__ __forceinline__ float lo_float(unsigned long long v) { return __uint_as_float((unsigned)v); }
+__device__ __forceinline__ float hi_float(unsigned long long v) { return __uint_as_float((unsigned)(v >> 32)); }
+__device__ __forceinline__ unsigned long long two_floats(float lo, float hi) {
+  return (unsigned long long)__float_as_uint(lo) | (unsigned long long)__float_as_uint(hi) << 32;
+}
+
+// A row's BF16 sampling strategy from its regrets: the sums and roundings of
+// sampling (cfr_gpu.cu:318-351).
+__device__ __forceinline__ uint4 pack_strategy(const float* reg) {
   float sum = 0.0f;
+#pragma unroll
   for (int a = 0; a < 8; ++a) sum = __fadd_rn(sum, fmaxf(0.0f, reg[a]));
-  __nv_bfloat16* st = reinterpret_cast<__nv_bfloat16*>(row_strat(tv, slot));
+  uint32_t h[8];
+#pragma unroll
   for (int a = 0; a < 8; ++a)
-    st[a] = __float2bfloat16_rn(sum > 1e-7f && reg[a] > 0.0f ? __fdiv_rn(reg[a], sum) : 0.0f);
+    h[a] = __bfloat16_as_ushort(__float2bfloat16_rn(sum > 1e-7f && reg[a] > 0.0f ? __fdiv_rn(reg[a], sum) : 0.0f));
+  return make_uint4(h[0] | h[1] << 16, h[2] | h[3] << 16, h[4] | h[5] << 16, h[6] | h[7] << 16);
 }
 
 // Adds one visit whose legal mask differs from the row's canonical one: every

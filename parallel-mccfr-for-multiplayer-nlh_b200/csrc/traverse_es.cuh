@@ -201,8 +201,8 @@ __device__ __forceinline__ int es_peek(const GameParams& G, const EsLane& L, int
 // stopped on a full table or frame stack (the error flag is set).  The updating
 // player's subtree is walked depth-first, opponents sampled.
 template <int W, class Frames>
-__device__ __forceinline__ int es_step(const GameParams& G, const TableView& tv, uint32_t uid, int up, float rscale,
-                                       Frames& fr, EsLane& L, EsCounts& cnt) {
+__device__ __forceinline__ int es_step(const GameParams& G, const TableView& tv, uint32_t uid, uint32_t epoch, int up,
+                                       float rscale, Frames& fr, EsLane& L, EsCounts& cnt) {
   const int N = G.N;
   const uint32_t all_players = (1u << N) - 1;
   EsState& cur = L.cur;
@@ -290,7 +290,7 @@ __device__ __forceinline__ int es_step(const GameParams& G, const TableView& tv,
                           G.seed_lo, G.seed_hi);
       const int s = sample_action(G, reg, vm, uniform01(d.x));
       if (slot >= 0) {
-        if (touch_row(tv, (unsigned long long)slot, uid, vm, 0u)) {
+        if (touch_row(tv, (unsigned long long)slot, epoch, vm)) {
           atomicAdd(row_cnt(tv, slot), (1ull << 32) | 1ull);
         } else {
           atomicAdd(row_cnt(tv, slot), 1ull << 32);
@@ -318,7 +318,8 @@ __device__ __forceinline__ int es_step(const GameParams& G, const TableView& tv,
       const float vh = F.vh;
       const long long fv = fix_r(vh, rscale);
       atomicAdd(row_cnt(tv, F.slot), 1ull << 32);
-      if (touch_row(tv, F.slot, uid, F.vm, kListWide)) {
+      mark_wide(tv, F.slot);
+      if (touch_row(tv, F.slot, epoch, F.vm)) {
         atomicAdd(row_su(tv, F.slot), (unsigned long long)fv);
       } else {
         long long dr[kSlots];
@@ -354,7 +355,7 @@ k_traverse_es(const GameParams G, const TableView tv, const DealRec* __restrict_
               int batch, float rscale, Counters* __restrict__ counters, unsigned* __restrict__ work) {
   extern __shared__ EsFrame s_frames[];  // [K][BLOCK]
   const int up = sched->player;
-  const uint32_t uid = update_id(sched, G.N);
+  const uint32_t uid = update_id(sched, G.N), epoch = *table_epoch(tv);
   FrameStack<K> fr;
   fr.smem = s_frames + threadIdx.x;
   fr.stride = BLOCK;
@@ -406,7 +407,7 @@ k_traverse_es(const GameParams G, const TableView tv, const DealRec* __restrict_
     if (forced) pick = __shfl_sync(0xFFFFFFFFu, ty, __ffs(forced) - 1);
     if (have && (ty == pick || ty == 4)) {
       waited = 0;
-      if (es_step<W>(G, tv, uid, up, rscale, fr, L, c)) have = false;
+      if (es_step<W>(G, tv, uid, epoch, up, rscale, fr, L, c)) have = false;
     } else if (have) {
       waited++;
     }

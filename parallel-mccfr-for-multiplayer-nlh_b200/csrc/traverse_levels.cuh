@@ -27,10 +27,8 @@
 //              snapshot the update does not change), reads its children's values,
 //              forms v_h = sum_a strat[a] * v[a] in slot order as the depth-first
 //              walk does, adds fix(v[a]) - fix(v_h) to every legal action's
-//              accumulator and hands v_h to its own seed.  The row is claimed for
-//              the update by one atomic maximum on its tag, with no canonical
-//              mask (the whole regret term goes to the accumulators), so no
-//              thread waits on a compare-and-swap.
+//              accumulator and hands v_h to its own seed.  The row is marked wide
+//              (the whole regret term goes to the accumulators).
 //
 // Every sum that reaches the table is an integer (fixed point) and every draw
 // is keyed by the node's action path, so the rows after an update are
@@ -136,7 +134,7 @@ __device__ __noinline__ float lv_showdown(int N, int up, uint32_t folded, uint32
 
 // A sampled opponent's visit whose mask is not the row's canonical one: its
 // strategy weights go to the accumulators directly.
-__device__ __noinline__ void lv_off_canonical(const TableView tv, unsigned long long slot, uint32_t vm) {
+__device__ __noinline__ void lv_off_canonical(const TableView& tv, unsigned long long slot, uint32_t vm) {
   atomicAdd(row_cnt(tv, slot), 1ull << 32);
   float reg[kSlots], strat[kSlots];
   load_regrets(tv, (long long)slot, reg);
@@ -163,7 +161,8 @@ struct LvPending {
 // action is left pending); at an updating-player node the walk stops with the
 // node's mask and row slot (its regrets are read in back).
 template <int W>
-__device__ __forceinline__ int lv_step(const GameParams& G, const TableView& tv, uint32_t uid, int up, EsState& cur,
+__device__ __forceinline__ int lv_step(const GameParams& G, const TableView& tv, uint32_t uid, uint32_t epoch, int up,
+                                       EsState& cur,
                                        const DealRec* D, LvPending& pend, float& value, uint32_t& vm_out,
                                        long long& slot_out, uint4& sd, EsCounts& cnt) {
   const int N = G.N;
@@ -235,13 +234,13 @@ __device__ __forceinline__ int lv_step(const GameParams& G, const TableView& tv,
       slot_out = (long long)rs;
       return kLvUp;
     }
-    const ulonglong2 kt = __ldcg(reinterpret_cast<const ulonglong2*>(row_ptr(tv, rs)));
+    const ulonglong2 head = __ldcg(row_head(tv, rs));
     const uint4 st = __ldg(row_strat(tv, rs));
     const U4 d = philox(U4{cur.aux, uid, (uint32_t)cur.path, (uint32_t)(cur.path >> 32) | 0x80000000u},
                         G.seed_lo, G.seed_hi);
-    if (kt.x != key) __stcg(row_key(tv, rs), key);
+    if (head.x != key) __stcg(row_key(tv, rs), key);
     const int s = sample_stored(G, st, vm, uniform01(d.x));
-    if (touch_row_from(tv, rs, uid, vm, kt.y, 0u)) {
+    if (touch_row_from(tv, rs, epoch, vm, head.y)) {
       atomicAdd(row_cnt(tv, rs), (1ull << 32) | 1ull);
     } else {
       lv_off_canonical(tv, rs, vm);
@@ -262,7 +261,7 @@ __device__ __forceinline__ int lv_step(const GameParams& G, const TableView& tv,
                       G.seed_hi);
   const int s = sample_stored(G, st, vm, uniform01(d.x));
   if (slot >= 0) {
-    if (touch_row(tv, (unsigned long long)slot, uid, vm, 0u)) {
+    if (touch_row(tv, (unsigned long long)slot, epoch, vm)) {
       atomicAdd(row_cnt(tv, slot), (1ull << 32) | 1ull);
     } else {
       lv_off_canonical(tv, (unsigned long long)slot, vm);
@@ -322,7 +321,7 @@ k_level_expand(const GameParams G, const TableView tv, const DealRec* __restrict
   const LevelBase B = s_base;
   if (B.count == 0) return;
   const int up = sched->player;
-  const uint32_t uid = update_id(sched, G.N);
+  const uint32_t uid = update_id(sched, G.N), epoch = *table_epoch(tv);
   const bool last = L + 1 >= lb.nlev;
   const int lane = threadIdx.x & 31;
   // room check at pick-up: every lane of the launch may hold a seed meanwhile
@@ -402,7 +401,7 @@ k_level_expand(const GameParams G, const TableView tv, const DealRec* __restrict
     float v = 0.0f;
     uint4 sd = make_uint4(0u, 0u, 0u, 0u);
     if (have) {
-      r = lv_step<W>(G, tv, uid, up, cur, D, pend, v, vm, slot, sd, c);
+      r = lv_step<W>(G, tv, uid, epoch, up, cur, D, pend, v, vm, slot, sd, c);
       if (r == kLvDone) {
         lb.value[seed] = v;
         have = false;
@@ -487,7 +486,7 @@ k_level_dfs(const GameParams G, const TableView tv, const DealRec* __restrict__ 
   __syncthreads();
   const uint32_t total = s_total;
   const int up = sched->player;
-  const uint32_t uid = update_id(sched, G.N);
+  const uint32_t uid = update_id(sched, G.N), epoch = *table_epoch(tv);
   FrameStack<K> fr;
   fr.smem = s_frames + threadIdx.x;
   fr.stride = BLOCK;
@@ -536,7 +535,7 @@ k_level_dfs(const GameParams G, const TableView tv, const DealRec* __restrict__ 
     }
     if (!__any_sync(0xFFFFFFFFu, have || more)) break;
     if (have) {
-      const int r = es_step<W>(G, tv, uid, up, rscale, fr, Ln, c);
+      const int r = es_step<W>(G, tv, uid, epoch, up, rscale, fr, Ln, c);
       if (r) {
         lb.value[seed] = r == 1 ? Ln.value : 0.0f;
         have = false;
@@ -570,20 +569,16 @@ k_level_back(const GameParams G, const TableView tv, const Sched* __restrict__ s
   if (threadIdx.x == 0) s_base = level_base(lb, L, batch);
   __syncthreads();
   const uint32_t nb = s_base.node;
-  const uint32_t uid = update_id(sched, G.N);
   unsigned upd = 0;
   for (uint32_t i = blockIdx.x * BLOCK + threadIdx.x; i < n; i += gridDim.x * BLOCK) {
     const uint4 m = __ldcg(lb.meta + nb + i);
     const uint32_t vm = m.w;
     if (!vm) continue;
     const unsigned long long slot = m.x;
-    // independent of each other: the claim, the row's regrets, the children's
-    // values, and (direct map) the row's key, which the expand pass left to this pass
-    if (tv.direct) {
-      const unsigned long long k = __ldcg(row_key(tv, slot));
-      if (k != slot + 1) __stcg(row_key(tv, slot), slot + 1);
-    }
-    claim_row(tv, slot, uid);
+    // independent of each other: the row's key (in a direct map it is left to this
+    // pass), its regrets, the children's values
+    if (tv.direct && __ldcg(row_key(tv, slot)) != slot + 1) __stcg(row_key(tv, slot), slot + 1);
+    mark_wide(tv, slot);
     float reg[kSlots], strat[kSlots], v[kSlots];
     load_regrets(tv, (long long)slot, reg);
     uint32_t o = m.z;

@@ -266,13 +266,16 @@ __device__ __forceinline__ void deal_one(const GameParams& G, const int32_t* __r
   for (int i = 0; i < 4; ++i) dst[i] = src[i];
 }
 
-// `ctl`: 128-byte blocks of counters of the traversal that follows, zeroed here
-// so that the update needs no launch for it (may be null).
+// The deal starts an update: it advances the table's epoch and zeroes `ctl`, the
+// counters of the traversal that follows (may be null), so that neither needs a
+// launch of its own.
 __global__ void __launch_bounds__(128) k_deal(const GameParams G, const HandView hv, const Sched* __restrict__ sched,
-                                              int batch, DealRec* __restrict__ out, uint32_t* __restrict__ ctl,
-                                              int ctl_words) {
-  if (blockIdx.x == 0)
+                                              int batch, DealRec* __restrict__ out, uint32_t* __restrict__ epoch,
+                                              uint32_t* __restrict__ ctl, int ctl_words) {
+  if (blockIdx.x == 0) {
+    if (threadIdx.x == 0) *epoch += 1;
     for (int i = threadIdx.x; i < ctl_words; i += blockDim.x) ctl[i] = 0;
+  }
   __shared__ uint8_t s_pre[52 * 52];
   for (int i = threadIdx.x; i < 52 * 52 / 4; i += blockDim.x)
     reinterpret_cast<uint32_t*>(s_pre)[i] = __ldg(reinterpret_cast<const uint32_t*>(hv.pre) + i);
@@ -365,7 +368,7 @@ k_traverse_ref(const GameParams G, const TableView tv, const DealRec* __restrict
   if (t >= (uint32_t)batch) return;
   const int N = G.N;
   const int up = sched->player;
-  const uint32_t uid = update_id(sched, N);
+  const uint32_t uid = update_id(sched, N), epoch = *table_epoch(tv);
 
   const DealRec& D = deals[t];
   const int dealer = D.dealer;
@@ -539,7 +542,8 @@ k_traverse_ref(const GameParams G, const TableView tv, const DealRec* __restrict
     const int s = (int)(sv & 0xFF);
     const uint32_t vm = sv >> 8;
     const long long dsamp = fix_r(__fsub_rn(__fdiv_rn(u, s_rec_q[i][tid]), u), rscale);
-    if (touch_row(tv, slot, uid, vm, kListWide)) {
+    mark_wide(tv, slot);
+    if (touch_row(tv, slot, epoch, vm)) {
       atomicAdd(row_cnt(tv, slot), (1ull << 32) | 1ull);
       atomicAdd(row_su(tv, slot), (unsigned long long)fu);
       atomicAdd(row_da(tv, slot) + s, (unsigned long long)(dsamp + fu));

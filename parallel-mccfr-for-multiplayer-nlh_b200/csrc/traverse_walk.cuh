@@ -13,7 +13,8 @@
 //   * per open node a count of children still out; the lane that delivers the
 //     last value lists the node as ready.  32 ready nodes at a time are regret
 //     matched, added to their rows and handed to their own parents;
-//   * a queue of showdowns, evaluated 32 at a time.
+//   * queues of showdowns and of visits off a row's canonical mask, worked off 32 at
+//     a time: each takes hundreds of instructions that few lanes of a step need.
 // So no lane waits for a level of the whole update, no counter in global memory
 // is shared but the roots', and an update is one launch whatever its depth,
 // which is what small updates cost in the level form (38 dependent launches).
@@ -45,7 +46,8 @@ constexpr int kWalkBlock = 128;
 constexpr int kWalkWarps = kWalkBlock / 32;
 constexpr int kWalkNodes = 192;                  // open updating-player nodes of a warp
 constexpr int kWalkSeeds = kSlots * kWalkNodes;  // their children not yet taken
-constexpr int kWalkShow = 64;                    // queued showdowns: 31 left over + 32 of one step
+constexpr int kWalkQueue = 64;                   // queue entries: 31 left over + 32 of one step
+constexpr int kWalkReady = 28;                   // lanes at a decision that end the filling of a step
 constexpr uint32_t kWalkRoot = 0xFFFFu;          // parent of a traversal's root
 
 // Counters of one update, zeroed by the deal that precedes the walk.
@@ -79,6 +81,7 @@ struct __align__(128) WalkNode {
   float v[kSlots];
   uint4 pad;
 };
+static_assert(kMaxLevels == 32, "one lane per level");
 static_assert(sizeof(WalkNode) == 128, "a node record is one line");
 
 struct WalkShowdown {
@@ -91,7 +94,9 @@ struct WalkWarp {
   uint16_t spare[kWalkNodes];          // free records
   uint16_t ready[kWalkNodes];          // nodes whose children are all in
   uint32_t out[kWalkNodes / 8];        // children still out, 4 bits per record
-  WalkShowdown show[kWalkShow];
+  WalkShowdown show[kWalkQueue];
+  uint2 off[kWalkQueue];               // row slot, legal mask
+  unsigned roots;                      // traversals this warp took
 };
 
 struct WalkBufs {
@@ -217,8 +222,35 @@ __device__ __forceinline__ int walk_events(const GameParams& G, WalkState& s, in
   return (int)((s.prog >> 16) & 0xFFu) >= G.max_depth ? kLvDone : kLvGoOn;
 }
 
+// Side-pot payoff of the updating player (side_pot_payoff).  A folded player, or
+// one beaten by a live seat with at least its chips, loses what it put in; one
+// that no live seat ties or beats takes its share of every seat's chips (sums of
+// whole chips below 2^24, exact in any order).  Only ties, and wins over some of
+// the side pots, need the pots one by one.
+__device__ __forceinline__ float walk_showdown(int N, int up, uint32_t folded, uint32_t inv0, uint32_t inv1,
+                                               uint32_t inv2, const DealRec* D) {
+  const uint2 k01 = __ldg(reinterpret_cast<const uint2*>(D->rank));
+  const uint32_t k2 = __ldg(reinterpret_cast<const uint32_t*>(D->rank + 4));
+  const int mine = seat16(inv0, inv1, inv2, up), rank = seat16(k01.x, k01.y, k2, up);
+  bool beaten = (folded >> up) & 1, contested = false;
+  int take = 0;
+#pragma unroll
+  for (int q = 0; q < kMaxPlayers; ++q) {
+    if (q >= N) break;
+    const int iq = (int)(((q < 2 ? inv0 : q < 4 ? inv1 : inv2) >> (16 * (q & 1))) & 0xFFFFu);
+    const int rq = (int)(((q < 2 ? k01.x : q < 4 ? k01.y : k2) >> (16 * (q & 1))) & 0xFFFFu);
+    const bool live = q != up && !((folded >> q) & 1);
+    take += min(iq, mine);
+    contested |= live && rq >= rank;
+    beaten |= live && rq > rank && iq >= mine;
+  }
+  if (beaten) return (float)(-mine);
+  if (!contested) return (float)(take - mine);
+  return lv_showdown(N, up, folded, inv0, inv1, inv2, D);
+}
+
 template <bool DIRECT>
-__global__ void __launch_bounds__(kWalkBlock, 8)
+__global__ void __launch_bounds__(kWalkBlock, 6)
 k_walk(const GameParams G, const TableView tv, const DealRec* __restrict__ deals, const Sched* __restrict__ sched,
        int batch, float rscale, const WalkBufs wb, Counters* __restrict__ counters) {
   __shared__ WalkWarp s_warp[kWalkWarps];
@@ -227,16 +259,19 @@ k_walk(const GameParams G, const TableView tv, const DealRec* __restrict__ deals
   const unsigned below = (1u << lane) - 1u;
   WalkWarp& W = s_warp[threadIdx.x >> 5];
   WalkNode* const pool = wb.nodes + (size_t)(blockIdx.x * kWalkWarps + (threadIdx.x >> 5)) * kWalkNodes;
+  __shared__ unsigned s_full;  // updating-player nodes that found no row
   if (threadIdx.x < kMaxLevels) s_nodes[threadIdx.x] = s_seeds[threadIdx.x] = 0;
+  if (threadIdx.x == 0) s_full = 0;
   for (int i = lane; i < kWalkNodes; i += 32) W.spare[i] = (uint16_t)(kWalkNodes - 1 - i);
   for (int i = lane; i < kWalkNodes / 8; i += 32) W.out[i] = 0;
+  if (lane == 0) W.roots = 0;
   __syncthreads();
   const int N = G.N;
   const int up = sched->player;
-  const uint32_t uid = update_id(sched, N);
+  const uint32_t uid = update_id(sched, N), epoch = *table_epoch(tv);
   // warp-uniform list lengths and counters
-  int n_seeds = 0, n_spare = kWalkNodes, n_ready = 0, n_show = 0;
-  unsigned c_trav = 0, c_vis = 0, c_upd = 0, c_term = 0;
+  int n_seeds = 0, n_spare = kWalkNodes, n_ready = 0, n_show = 0, n_off = 0;
+  unsigned c_vis = 0;
   bool more = true;  // roots may be left
   int stalled = 0;
   // the lane's walk: idle, an action to apply, or standing at a decision
@@ -244,7 +279,8 @@ k_walk(const GameParams G, const TableView tv, const DealRec* __restrict__ deals
   int st = kIdle;
   WalkState s;
   uint32_t ref = kWalkRoot;  // its seed
-  int pl = -1, pa = 0;       // pending action (pl < 0: a root, nothing to apply)
+  int pl = -1, pa = 0;       // pending action (pl < 0: a root, nothing to apply), or the seat to act
+  uint32_t cw = 0;           // that seat's cards (DealRec::ctx)
 
   // Hands lane values to their parents (ref), listing nodes whose last child it was.
   auto deliver = [&](bool on, float v) {
@@ -280,7 +316,7 @@ k_walk(const GameParams G, const TableView tv, const DealRec* __restrict__ deals
       const uint32_t keep = ref;
       float v = 0.0f;
       if (on) {
-        v = lv_showdown(N, up, r.ref >> 16, r.inv0, r.inv1, r.inv2, deals + r.aux);
+        v = walk_showdown(N, up, r.ref >> 16, r.inv0, r.inv1, r.inv2, deals + r.aux);
         ref = r.ref & 0xFFFFu;
       }
       deliver(on, v);
@@ -301,16 +337,15 @@ k_walk(const GameParams G, const TableView tv, const DealRec* __restrict__ deals
         const unsigned long long slot = nd->s3.w;
         const uint4 own = nd->own;
         const uint32_t vm = own.y;
-        if (DIRECT) {  // the row's key, which the walk left to this pass
-          const unsigned long long k = __ldcg(row_key(tv, slot));
-          if (k != slot + 1) __stcg(row_key(tv, slot), slot + 1);
-        }
-        claim_row(tv, slot, uid);
+        const unsigned long long k = __ldcg(row_key(tv, slot));
         float reg[kSlots], strat[kSlots], v[kSlots];
         load_regrets(tv, (long long)slot, reg);
         const float4 v0 = *reinterpret_cast<const float4*>(nd->v), v1 = *reinterpret_cast<const float4*>(nd->v + 4);
         v[0] = v0.x; v[1] = v0.y; v[2] = v0.z; v[3] = v0.w;
         v[4] = v1.x; v[5] = v1.y; v[6] = v1.z; v[7] = v1.w;
+        // a direct-mapped row's key was left to this pass
+        if (DIRECT && k != slot + 1) __stcg(row_key(tv, slot), slot + 1);
+        mark_wide(tv, slot);
         node_strategy(reg, vm, strat);
 #pragma unroll
         for (int a = 0; a < kSlots; ++a)
@@ -325,9 +360,29 @@ k_walk(const GameParams G, const TableView tv, const DealRec* __restrict__ deals
       __syncwarp();
       if (on) W.spare[n_spare + lane] = (uint16_t)id;
       n_spare += nb;
-      c_upd += nb;
       deliver(on, vh);
       ref = keep;
+      continue;
+    }
+    if (n_off >= 32 || (n_off && starved)) {
+      // visits off the canonical mask: every legal slot's strategy weight
+      const int nb = min(32, n_off);
+      n_off -= nb;
+      if (lane < nb) {
+        const uint2 e = W.off[n_off + lane];
+        float reg[kSlots], strat[kSlots];
+        load_regrets(tv, (long long)e.x, reg);
+        node_strategy(reg, e.y, strat);
+        atomicOr(row_flags(tv, e.x), kFlagDs);
+        atomicAdd(row_cnt(tv, e.x), 1ull << 32);
+#pragma unroll
+        for (int a = 0; a < kSlots; ++a)
+          if ((e.y >> a) & 1) {
+            const long long d = fix_s(strat[a]);
+            if (d) atomicAdd(row_ds(tv, e.x) + a, (unsigned long long)d);
+          }
+      }
+      __syncwarp();
       continue;
     }
     if (starved) break;
@@ -368,7 +423,7 @@ k_walk(const GameParams G, const TableView tv, const DealRec* __restrict__ deals
           pl = -1;
           st = kApply;
         }
-        c_trav += got;
+        if (lane == 0) W.roots += got;
         filled = got > 0;
       }
     }
@@ -381,11 +436,15 @@ k_walk(const GameParams G, const TableView tv, const DealRec* __restrict__ deals
       if (st == kApply) {
         if (pl >= 0) walk_apply(G, s, pl, pa);
         r = walk_events(G, s, up, v);
-        st = r == kLvGoOn ? kDecide : kIdle;
+        st = kIdle;
+        if (r == kLvGoOn) {
+          st = kDecide;
+          pl = walk_next(s.seats, N);
+          cw = __ldg(deals[s.aux].ctx + pl);
+        }
       }
       const unsigned showm = __ballot_sync(0xFFFFFFFFu, r == kLvShow);
       const unsigned donem = __ballot_sync(0xFFFFFFFFu, r == kLvDone);
-      c_term += __popc(showm) + __popc(donem);
       if (r == kLvShow) {
         WalkShowdown& q = W.show[n_show + __popc(showm & below)];
         q.ref = ref | (s.seats << 16);
@@ -400,7 +459,7 @@ k_walk(const GameParams G, const TableView tv, const DealRec* __restrict__ deals
     }
     // lanes freed by terminals are filled again before the decisions run
     const unsigned decm = __ballot_sync(0xFFFFFFFFu, st == kDecide);
-    if (filled && __popc(decm) < 28 && (n_seeds > 0 || more)) continue;
+    if (filled && __popc(decm) < kWalkReady && (n_seeds > 0 || more)) continue;
     if (!decm) {
       // every round of the loop above takes, fills or finishes something; a round
       // that does not would never end
@@ -412,14 +471,13 @@ k_walk(const GameParams G, const TableView tv, const DealRec* __restrict__ deals
     }
 
     // ---- decisions
-    bool isup = false;
+    bool isup = false, off = false;
     uint32_t vm = 0;
     long long slot = -1;
     c_vis += __popc(decm);
     if (st == kDecide) {
-      const int player = walk_next(s.seats, N);
+      const int player = pl;
       const int street = (int)(s.prog & 0xFu);
-      const uint32_t cw = __ldg(deals[s.aux].ctx + player);
       const int to_call = s.cb - seat16(s.bet0, s.bet1, s.bet2, player);
       vm = valid_mask(G, s.pot, G.stack_base - seat16(s.inv0, s.inv1, s.inv2, player), to_call, s.cb, s.lfr,
                       (int)((s.prog >> 8) & 0xFFu));
@@ -437,26 +495,28 @@ k_walk(const GameParams G, const TableView tv, const DealRec* __restrict__ deals
       slot = DIRECT ? (long long)(key - 1) : table_insert<1>(tv, key);
       if (!isup) {
         const bool ok = DIRECT || slot >= 0;
-        ulonglong2 kt = make_ulonglong2(0ull, 0ull);
+        ulonglong2 head = make_ulonglong2(0ull, 0ull);
         uint4 sg = make_uint4(0u, 0u, 0u, 0u);
         if (ok) {
-          kt = __ldcg(reinterpret_cast<const ulonglong2*>(row_ptr(tv, (unsigned long long)slot)));
+          head = __ldcg(row_head(tv, (unsigned long long)slot));
           sg = __ldcg(row_strat(tv, (unsigned long long)slot));
         }
         const U4 d = philox(U4{s.aux, uid, (uint32_t)s.path, (uint32_t)(s.path >> 32) | 0x80000000u}, G.seed_lo,
                             G.seed_hi);
-        if (DIRECT && kt.x != key) __stcg(row_key(tv, (unsigned long long)slot), key);
-        pl = player;
+        if (DIRECT && head.x != key) __stcg(row_key(tv, (unsigned long long)slot), key);
         pa = sample_stored(G, sg, vm, uniform01(d.x));
         st = kApply;
         if (ok) {
-          if (touch_row_from(tv, (unsigned long long)slot, uid, vm, kt.y, 0u))
+          if (touch_row_from(tv, (unsigned long long)slot, epoch, vm, head.y))
             atomicAdd(row_cnt(tv, (unsigned long long)slot), (1ull << 32) | 1ull);
           else
-            lv_off_canonical(tv, (unsigned long long)slot, vm);
+            off = true;
         }
       }
     }
+    const unsigned offm = __ballot_sync(0xFFFFFFFFu, off);
+    if (off) W.off[n_off + __popc(offm & below)] = make_uint2((uint32_t)slot, vm);
+    n_off += __popc(offm);
     // ---- updating-player nodes: a record and one seed per legal action
     if (__any_sync(0xFFFFFFFFu, isup)) {
       const unsigned full = __ballot_sync(0xFFFFFFFFu, isup && slot < 0);  // no row: nothing to update
@@ -476,6 +536,12 @@ k_walk(const GameParams G, const TableView tv, const DealRec* __restrict__ deals
         total += __popc(kb) << b;
       }
       const int cnt = __popc(upm);
+      // the lanes go on with their node's first action while the pool is far from full
+      const bool go_on = n_spare - cnt - 32 >= wb.decisions;
+      if (go_on) {
+        before -= __popc(upm & below);
+        total -= cnt;
+      }
       if (open) {
         const uint32_t id = W.spare[n_spare - 1 - __popc(upm & below)];
         WalkNode* nd = pool + id;
@@ -486,27 +552,47 @@ k_walk(const GameParams G, const TableView tv, const DealRec* __restrict__ deals
         nd->own = make_uint4(ref, vm, 0u, 0u);
         atomicAdd(&W.out[id >> 3], (unsigned)k << (4u * (id & 7u)));
         int o = n_seeds + before;
-        for (uint32_t left = vm; left; left &= left - 1) W.seeds[o++] = (uint16_t)((id << 3) | (uint32_t)(__ffs(left) - 1));
+        uint32_t left = vm;
+        if (go_on) left &= left - 1;
+        for (; left; left &= left - 1) W.seeds[o++] = (uint16_t)((id << 3) | (uint32_t)(__ffs(left) - 1));
         const int level = (int)(s.prog >> 24);
         atomicAdd(&s_nodes[level], 1u);
         atomicAdd(&s_seeds[level], (unsigned)k);
+        if (go_on) {
+          pa = __ffs((int)vm) - 1;
+          ref = (id << 3) | (uint32_t)pa;
+          s.prog += 1u << 24;
+        }
       }
       n_spare -= cnt;
       n_seeds += total;
       __syncwarp();
-      if (full) deliver(isup && slot < 0, 0.0f);
-      if (isup) st = kIdle;
+      if (full) {
+        deliver(isup && slot < 0, 0.0f);
+        if (lane == 0) atomicAdd(&s_full, (unsigned)__popc(full));
+      }
+      if (isup) st = open && go_on ? kApply : kIdle;
     }
   }
   if (lane == 0) {
-    if (c_trav) atomicAdd(&counters->traversals, (unsigned long long)c_trav);
+    if (W.roots) {
+      atomicAdd(&counters->traversals, (unsigned long long)W.roots);
+      atomicAdd(&counters->evals, (unsigned long long)W.roots * (unsigned)N);
+    }
     if (c_vis) atomicAdd(&counters->visits, (unsigned long long)c_vis);
-    if (c_upd) atomicAdd(&counters->updates, (unsigned long long)c_upd);
-    if (c_term) atomicAdd(&counters->terminals, (unsigned long long)c_term);
-    if (c_trav) atomicAdd(&counters->evals, (unsigned long long)c_trav * (unsigned)N);
   }
   __syncthreads();
-  if (threadIdx.x < kMaxLevels) {
+  if (threadIdx.x < 32) {
+    // every root and seed ended at a terminal, an updating-player node, or a node
+    // that found no row
+    const unsigned nodes = __reduce_add_sync(0xFFFFFFFFu, s_nodes[threadIdx.x]);
+    const unsigned seeds = __reduce_add_sync(0xFFFFFFFFu, s_seeds[threadIdx.x]);
+    const unsigned ends = (threadIdx.x < kWalkWarps ? s_warp[threadIdx.x].roots : 0u);
+    const unsigned roots = __reduce_add_sync(0xFFFFFFFFu, ends);
+    if (threadIdx.x == 0 && roots) {
+      atomicAdd(&counters->updates, (unsigned long long)nodes);
+      atomicAdd(&counters->terminals, (unsigned long long)roots + seeds - nodes - s_full);
+    }
     if (s_nodes[threadIdx.x]) atomicAdd(&wb.ctl->nodes[threadIdx.x], s_nodes[threadIdx.x]);
     if (s_seeds[threadIdx.x]) atomicAdd(&wb.ctl->seeds[threadIdx.x], s_seeds[threadIdx.x]);
   }
