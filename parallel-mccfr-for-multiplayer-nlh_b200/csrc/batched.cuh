@@ -53,21 +53,32 @@ __device__ __forceinline__ int phase_table_of(const PhaseDesc& P, unsigned long 
   return lo;
 }
 
+// Deals of a phase: full games (one thread per traversal) or subgames (SUB, eight
+// lanes each); a phase that holds both takes both launches, each skipping the
+// other's items.  The first launch of a phase advances its tables' epochs.
+template <bool SUB>
 __global__ void __launch_bounds__(128) k_deal_batched(const TableDesc* __restrict__ tables,
                                                       const PhaseDesc* __restrict__ phase,
-                                                      const int32_t* __restrict__ T, DealRec* __restrict__ out) {
+                                                      const int32_t* __restrict__ T, DealRec* __restrict__ out,
+                                                      int first) {
   __shared__ PhaseDesc P;
+  __shared__ uint32_t s_deck[SUB ? 1 : 128 * kDeckWords];
   for (int i = threadIdx.x; i < (int)(sizeof(PhaseDesc) / 4); i += blockDim.x)
     reinterpret_cast<uint32_t*>(&P)[i] = reinterpret_cast<const uint32_t*>(phase)[i];
   __syncthreads();
-  if (blockIdx.x == 0 && (int)threadIdx.x < P.n) *table_epoch(tables[P.table[threadIdx.x]].tv) += 1;
+  if (first && blockIdx.x == 0 && (int)threadIdx.x < P.n) *table_epoch(tables[P.table[threadIdx.x]].tv) += 1;
   const unsigned long long total = P.off[P.n];
-  for (unsigned long long g = blockIdx.x * (unsigned long long)blockDim.x + threadIdx.x; g < total;
-       g += (unsigned long long)gridDim.x * blockDim.x) {
+  constexpr int kLanes = SUB ? kDealGroup : 1;
+  const unsigned gmask = ((1u << kDealGroup) - 1u) << ((threadIdx.x & 31) & ~(kDealGroup - 1));
+  for (unsigned long long g = (blockIdx.x * (unsigned long long)blockDim.x + threadIdx.x) / kLanes; g < total;
+       g += (unsigned long long)gridDim.x * blockDim.x / kLanes) {
     const int j = phase_table_of(P, g);
     const TableDesc& D = tables[P.table[j]];
+    if ((D.G.sub_street != 0) != SUB) continue;
     const uint32_t t = (uint32_t)(g - P.off[j]);
-    deal_one(D.G, T, D.pre, D.cdf, t, update_id(D.sched, D.G.N), out + g);
+    const uint32_t uid = update_id(D.sched, D.G.N);
+    if (SUB) deal_subgame(D.G, T, t, uid, out + g, (int)threadIdx.x & (kDealGroup - 1), gmask);
+    else deal_one(D.G, T, D.pre, D.cdf, t, uid, out + g, s_deck + kDeckWords * threadIdx.x);
   }
 }
 

@@ -306,10 +306,18 @@ __device__ __forceinline__ int combo_index(int a, int b) {
   return hi * (hi - 1) / 2 + lo;
 }
 __device__ __forceinline__ void combo_cards(int idx, int& lo, int& hi) {
-  int h = 1;
-  while ((h + 1) * h / 2 <= idx) ++h;
+  // the largest h with h(h-1)/2 <= idx: a square root, corrected by one where its
+  // rounding needs it
+  int h = (int)((1.0f + sqrtf((float)(8 * idx + 1))) * 0.5f);
+  if (h * (h - 1) / 2 > idx) --h;
+  if ((h + 1) * h / 2 <= idx) ++h;
   hi = h;
   lo = idx - h * (h - 1) / 2;
+}
+__device__ __forceinline__ uint64_t combo_bits(int idx) {
+  int lo, hi;
+  combo_cards(idx, lo, hi);
+  return (1ull << lo) | (1ull << hi);
 }
 
 // Reference info-set slot (cfr_gpu.cu:165-179).

@@ -433,6 +433,21 @@ __global__ void k_rank_hist(const int32_t* __restrict__ T, int ncards, unsigned 
     if (sh[i]) atomicAdd(&hist[i], (unsigned long long)sh[i]);
 }
 
+// Buckets of the rank table's 5- and 6-card states (kStateBuckets), one warp per
+// state: the row of a 5-card state leads to states (far above 16 bits), that of a
+// 6-card state to packed ranks; both hold their own packed rank at offset 0.
+__global__ void k_state_buckets(const int32_t* __restrict__ T, uint8_t* __restrict__ cdf) {
+  const int lane = threadIdx.x & 31;
+  for (int k = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5); k < kStates;
+       k += (int)((gridDim.x * blockDim.x) >> 5)) {
+    const int32_t* row = T + 53ll * k;
+    const int a = __ldg(row + 1 + lane), b = lane < 20 ? __ldg(row + 33 + lane) : 0;
+    const bool five = __reduce_max_sync(0xFFFFFFFFu, max(a, b)) > 0xFFFF;
+    const uint32_t rank = decode16((uint32_t)__ldg(row) & 0xFFFF);
+    if (lane == 0) cdf[kStateBuckets + k] = rank < 7463u ? cdf[(five ? 0 : 7463) + rank] : 0;
+  }
+}
+
 }  // namespace
 
 // ---------------------------------------------------------------------------
@@ -679,6 +694,22 @@ int record(mccfr_handle* h, cudaEvent_t e, bool capturing) {
   return MCCFR_OK;
 }
 
+// Blocks of the full-game deal: 16 per SM, so that a large deal fills the preflop
+// LUT of a block once and not once per 128 traversals.
+constexpr int kDealBlocks = 148 * 16;
+
+// Deals of a phase's tables into `out` (k_deal_batched).
+cudaError_t launch_deals(const TableDesc* d_tables, const PhaseDesc* d_phase, const int32_t* T, DealRec* out,
+                         unsigned long long items, bool full, bool sub, cudaStream_t stream) {
+  const auto blocks = [](unsigned long long threads) {
+    return (int)std::max<unsigned long long>(1, std::min<unsigned long long>((threads + 127) / 128, 148ull * 64));
+  };
+  if (full) k_deal_batched<false><<<blocks(items), 128, 0, stream>>>(d_tables, d_phase, T, out, 1);
+  if (sub)
+    k_deal_batched<true><<<blocks(items * kDealGroup), 128, 0, stream>>>(d_tables, d_phase, T, out, full ? 0 : 1);
+  return cudaGetLastError();
+}
+
 bool use_walk(const mccfr_handle* h);
 bool use_levels(const mccfr_handle* h);
 int enqueue_walk(mccfr_handle* h, int batch, float rscale);
@@ -693,10 +724,14 @@ int enqueue_update(mccfr_handle* h, int batch, mccfr_trace* d_trace, cudaEvent_t
   HandView hv{h->d_hr, h->d_pre, h->d_cdf};
   if (batch > h->deals_cap) return fail(h, MCCFR_ERR_INVALID_ARG, "deal buffer smaller than the batch");
   const bool walk = use_walk(h);
-  k_deal<<<(batch + 127) / 128, 128, 0, h->stream>>>(h->gp, hv, h->d_sched, batch, h->d_deals,
-                                                     table_epoch(h->tv),
-                                                     walk ? reinterpret_cast<uint32_t*>(h->wb.ctl) : nullptr,
-                                                     walk ? (int)(sizeof(WalkCtl) / 4) : 0);
+  uint32_t* const ctl = walk ? reinterpret_cast<uint32_t*>(h->wb.ctl) : nullptr;
+  const int ctl_words = walk ? (int)(sizeof(WalkCtl) / 4) : 0;
+  if (h->gp.sub_street)
+    k_deal<true><<<(int)(((long long)batch * kDealGroup + 127) / 128), 128, 0, h->stream>>>(
+        h->gp, hv, h->d_sched, batch, h->d_deals, table_epoch(h->tv), ctl, ctl_words);
+  else
+    k_deal<false><<<std::min((batch + 127) / 128, kDealBlocks), 128, 0, h->stream>>>(
+        h->gp, hv, h->d_sched, batch, h->d_deals, table_epoch(h->tv), ctl, ctl_words);
   CK(cudaGetLastError());
   if (ev3 && record(h, ev3[0], capturing)) return MCCFR_ERR_CUDA;
   if (h->cfg.sampling == MCCFR_SAMPLING_REFERENCE) {
@@ -1260,8 +1295,8 @@ int mccfr_create(const mccfr_config* cfg, mccfr_handle** out) {
   build_preflop_lut(cfg->preflop_mode, cfg->preflop_buckets, pre);
   CKC(cudaMalloc(&h->d_pre, sizeof(pre)));
   CKC(cudaMemcpy(h->d_pre, pre, sizeof(pre), cudaMemcpyHostToDevice));
-  CKC(cudaMalloc(&h->d_cdf, 3 * 7463));
-  CKC(cudaMemset(h->d_cdf, 0, 3 * 7463));
+  CKC(cudaMalloc(&h->d_cdf, kCdfBytes));
+  CKC(cudaMemset(h->d_cdf, 0, kCdfBytes));
   CKC(cudaMalloc(&h->d_sched, sizeof(Sched)));
   CKC(cudaMallocHost(&h->h_sched, sizeof(Sched)));
   CKC(cudaMalloc(&h->d_counters, sizeof(Counters)));
@@ -1341,6 +1376,9 @@ int mccfr_set_hand_table(mccfr_handle* h, const int32_t* table, size_t n) {
     }
     cudaFree(d_hist);
     CK(cudaMemcpy(h->d_cdf, lut, sizeof(lut), cudaMemcpyHostToDevice));
+    k_state_buckets<<<148 * 8, 256, 0, h->stream>>>(h->d_hr, h->d_cdf);
+    CK(cudaGetLastError());
+    CK(cudaStreamSynchronize(h->stream));
   }
   // A persisting L2 access-policy window over the rank table is set only on
   // request (MCCFR_L2_PERSIST=1): the table (130 MB) is larger than the
@@ -2059,9 +2097,9 @@ int batch_enqueue_iteration(mccfr_batch* b, bool capturing) {
     const PhaseDesc& P = b->phases[p];
     const unsigned long long items = P.off[P.n];
     BCK(cudaMemsetAsync(b->d_work + p, 0, sizeof(unsigned long long), b->stream));
-    const int dgrid = (int)std::min<unsigned long long>((items + 127) / 128, 148ull * 64);
-    k_deal_batched<<<std::max(1, dgrid), 128, 0, b->stream>>>(b->d_tables, b->d_phases + p, T, b->d_deals);
-    BCK(cudaGetLastError());
+    bool full = false, sub = false;
+    for (int j = 0; j < P.n; ++j) (b->tables[P.table[j]]->gp.sub_street ? sub : full) = true;
+    BCK(launch_deals(b->d_tables, b->d_phases + p, T, b->d_deals, items, full, sub, b->stream));
     BCK(rec(b->ev_ph[2 * p]));
     kern<<<grid, t.block, smem, b->stream>>>(b->params[p], b->d_deals, b->d_work + p, t.grab, t.warp_sync);
     BCK(cudaGetLastError());
@@ -2557,7 +2595,7 @@ int mccfr_share_hand_table(mccfr_handle* h, mccfr_handle* src) {
     if (src->cfg.postflop_mode != MCCFR_POSTFLOP_RANK_CDF ||
         std::memcmp(src->cfg.postflop_buckets, h->cfg.postflop_buckets, sizeof(h->cfg.postflop_buckets)))
       return fail(h, MCCFR_ERR_INVALID_ARG, "rank-CDF buckets differ from the source table's");
-    CK(cudaMemcpy(h->d_cdf, src->d_cdf, 3 * 7463, cudaMemcpyDeviceToDevice));
+    CK(cudaMemcpy(h->d_cdf, src->d_cdf, kCdfBytes, cudaMemcpyDeviceToDevice));
   }
   if (h->d_hr && !h->shared_hr) cudaFree(h->d_hr);
   h->d_hr = src->d_hr;
@@ -2650,9 +2688,9 @@ int mccfr_batch_round(mccfr_handle* const* tables, int n, const int* traversals,
   BCK(cudaMemcpyAsync(R.d_tables, descs.data(), n * sizeof(TableDesc), cudaMemcpyHostToDevice, R.stream));
   BCK(cudaMemcpyAsync(R.d_phase, &P, sizeof(P), cudaMemcpyHostToDevice, R.stream));
   BCK(cudaMemsetAsync(R.d_work, 0, sizeof(unsigned long long), R.stream));
-  const int dgrid = (int)std::min<unsigned long long>((off + 127) / 128, 148ull * 64);
-  k_deal_batched<<<std::max(1, dgrid), 128, 0, R.stream>>>(R.d_tables, R.d_phase, tables[0]->d_hr, R.d_deals);
-  BCK(cudaGetLastError());
+  bool full = false, sub = false;
+  for (int i = 0; i < n; ++i) (tables[i]->gp.sub_street ? sub : full) = true;
+  BCK(launch_deals(R.d_tables, R.d_phase, tables[0]->d_hr, R.d_deals, off, full, sub, R.stream));
   BatchedKernel kern = pick_kernel(t);
   const size_t smem = batched_smem(t);
   BCK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));

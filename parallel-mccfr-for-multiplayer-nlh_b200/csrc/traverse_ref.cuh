@@ -35,8 +35,15 @@ struct Sched {
 struct HandView {
   const int32_t* hr;      // rank table
   const uint8_t* pre;     // preflop LUT [52*52]
-  const uint8_t* cdf;     // rank-CDF LUTs [3][7463]
+  const uint8_t* cdf;     // rank-CDF LUTs [3][7463], then the states' buckets
 };
+
+// Rank-CDF buckets of the rank table's 5- and 6-card states, one byte per state
+// (613 KB beside the LUTs): a flop or turn bucket is one gather from a small
+// table instead of the state's rank from the 130 MB one and then its LUT.
+constexpr int kStateBuckets = 22400;  // offset: 3 * 7463 rounded up
+constexpr int kStates = MCCFR_HAND_TABLE_ENTRIES / 53;
+constexpr size_t kCdfBytes = kStateBuckets + kStates;
 
 // One traversal's deal.  ctx[p] = hole bucket | flop << 8 | turn << 16 | river << 24.
 struct DealRec {
@@ -77,174 +84,191 @@ __device__ __forceinline__ uint32_t update_id(const Sched* s, int N) {
   return (uint32_t)((s->iteration - 1) * N + s->player);
 }
 
-// First combo whose cumulative weight exceeds w (w < 2^31), by bisection.
-__device__ __forceinline__ int sample_combo(const uint32_t* __restrict__ cdf, uint32_t w) {
-  int lo = 0, hi = 1325;
-  while (lo < hi) {
-    const int mid = (lo + hi) >> 1;
-    if (w < __ldg(cdf + mid)) hi = mid;
-    else lo = mid + 1;
-  }
-  return lo;
-}
-
 // Subgame deal: every player's hole combo from its range, all combos drawn
 // together and redrawn (up to 16 times) until no two share a card; after that,
 // player by player, the drawn combo or the next one of positive weight that
 // fits.  On the turn the river card is then uniform among the unused cards.
 // ctx[p] = combo | (river card + 1) << 16 (the river card enters the river keys).
+//
+// Eight lanes per traversal (`gl` = lane of the group): they draw eight attempts
+// at once and keep the first that fits, then lane p writes player p's fields.  The
+// draws are chains of dependent range lookups (11 per combo), and with six players
+// three of four attempts collide, so one thread per traversal spent most of a
+// small update here (1,024 six-player turn deals: 236 us).
+constexpr int kDealGroup = 8;
+
 __device__ __forceinline__ void deal_subgame(const GameParams& G, const int32_t* __restrict__ T, uint32_t t,
-                                             uint32_t uid, DealRec* __restrict__ out) {
+                                             uint32_t uid, DealRec* __restrict__ out, int gl, unsigned gmask) {
   const int N = G.N;
   const int nb = G.sub_street == 2 ? 4 : 5;
   uint64_t used_board = 0;
   for (int i = 0; i < nb; ++i) used_board |= 1ull << G.sub_board[i];
-  int combo[kMaxPlayers];
+  int combo[kMaxPlayers], first[kMaxPlayers];  // this attempt's combos, the first round's
   uint64_t used = used_board;
-  bool ok = false;
-  for (int a = 0; a < 16 && !ok; ++a) {
-    const U4 w0 = philox(U4{t, uid, 0x100u + (uint32_t)a, 0u}, G.seed_lo, G.seed_hi);
-    const U4 w1 = philox(U4{t, uid, 0x100u + (uint32_t)a, 1u}, G.seed_lo, G.seed_hi);
-    const uint32_t words[8] = {w0.x, w0.y, w0.z, w0.w, w1.x, w1.y, w1.z, w1.w};
-    used = used_board;
-    ok = true;
-    for (int p = 0; p < N && ok; ++p) {
-      combo[p] = sample_combo(G.range_cdf + 1326 * p, words[p] >> 1);
-      int lo, hi;
-      combo_cards(combo[p], lo, hi);
-      const uint64_t m = (1ull << lo) | (1ull << hi);
-      if (used & m) ok = false;
-      used |= m;
+  int winner = -1;
+  for (int round = 0; round < 16 / kDealGroup && winner < 0; ++round) {
+    const uint32_t attempt = 0x100u + (uint32_t)(round * kDealGroup + gl);
+    const U4 w0 = philox(U4{t, uid, attempt, 0u}, G.seed_lo, G.seed_hi);
+    const U4 w1 = philox(U4{t, uid, attempt, 1u}, G.seed_lo, G.seed_hi);
+    const uint32_t words[kMaxPlayers] = {w0.x >> 1, w0.y >> 1, w0.z >> 1, w0.w >> 1, w1.x >> 1, w1.y >> 1};
+    // each player's first combo whose cumulative weight exceeds its word, by
+    // bisection, the players' side by side
+    int lo[kMaxPlayers], hi[kMaxPlayers];
+#pragma unroll
+    for (int p = 0; p < kMaxPlayers; ++p) {
+      lo[p] = 0;
+      hi[p] = p < N ? 1325 : 0;
     }
-  }
-  if (!ok) {
-    const U4 w0 = philox(U4{t, uid, 0x100u, 0u}, G.seed_lo, G.seed_hi);
-    const U4 w1 = philox(U4{t, uid, 0x100u, 1u}, G.seed_lo, G.seed_hi);
-    const uint32_t words[8] = {w0.x, w0.y, w0.z, w0.w, w1.x, w1.y, w1.z, w1.w};
+    for (int step = 0; step < 11; ++step) {
+#pragma unroll
+      for (int p = 0; p < kMaxPlayers; ++p)
+        if (lo[p] < hi[p]) {
+          const int mid = (lo[p] + hi[p]) >> 1;
+          if (words[p] < __ldg(G.range_cdf + 1326 * p + mid)) hi[p] = mid;
+          else lo[p] = mid + 1;
+        }
+    }
     used = used_board;
-    for (int p = 0; p < N; ++p) {
-      const uint32_t* cdf = G.range_cdf + 1326 * p;
-      const int start = sample_combo(cdf, words[p] >> 1);
-      int pick = -1;
-      for (int k = 0; k < 1326 && pick < 0; ++k) {
-        const int c = (start + k) % 1326;
-        const uint32_t prev = c ? __ldg(cdf + c - 1) : 0u;
-        if (__ldg(cdf + c) == prev) continue;  // zero weight
-        int lo, hi;
-        combo_cards(c, lo, hi);
-        if (!(used & ((1ull << lo) | (1ull << hi)))) pick = c;
+    bool ok = true;
+#pragma unroll
+    for (int p = 0; p < kMaxPlayers; ++p) {
+      combo[p] = lo[p];
+      if (round == 0) first[p] = lo[p];
+      if (p < N) {
+        const uint64_t m = combo_bits(lo[p]);
+        ok &= (used & m) == 0;
+        used |= m;
       }
-      if (pick < 0) pick = start;  // range exhausted by card removal: keep the draw
-      combo[p] = pick;
-      int lo, hi;
-      combo_cards(pick, lo, hi);
-      used |= (1ull << lo) | (1ull << hi);
     }
+    const unsigned fit = __ballot_sync(gmask, ok) & gmask;
+    if (fit) winner = __ffs((int)fit) - 1;
   }
-  DealRec r;
-  for (int i = 0; i < 10; ++i) r.pad[i] = 0;
-  for (int i = 0; i < 5; ++i) r.board[i] = (i < nb) ? G.sub_board[i] : 0;
-  int river = -1;
+  if (winner < 0) {
+    winner = __ffs((int)gmask) - 1;
+    if (gl == 0) {
+      used = used_board;
+#pragma unroll
+      for (int p = 0; p < kMaxPlayers; ++p) {
+        if (p >= N) break;
+        const uint32_t* cdf = G.range_cdf + 1326 * p;
+        const int start = first[p];  // attempt 0 is this lane's
+        int pick = -1;
+        for (int k = 0; k < 1326 && pick < 0; ++k) {
+          const int c = start + k < 1326 ? start + k : start + k - 1326;
+          const uint32_t prev = c ? __ldg(cdf + c - 1) : 0u;
+          if (__ldg(cdf + c) == prev) continue;  // zero weight
+          if (!(used & combo_bits(c))) pick = c;
+        }
+        if (pick < 0) pick = start;  // range exhausted by card removal: keep the draw
+        combo[p] = pick;
+        used |= combo_bits(pick);
+      }
+    }
+    __syncwarp(gmask);
+  }
+  int mine = 0;
+#pragma unroll
+  for (int p = 0; p < kMaxPlayers; ++p) {
+    const int c = __shfl_sync(gmask, combo[p], winner);
+    if (p == gl) mine = c;
+  }
+  used = (uint64_t)__shfl_sync(gmask, (unsigned)used, winner) |
+         (uint64_t)__shfl_sync(gmask, (unsigned)(used >> 32), winner) << 32;
+  int river = nb == 4 ? 0 : -1, fifth = G.sub_board[4];
   if (nb == 4) {
     const U4 w = philox(U4{t, uid, 0x200u, 0u}, G.seed_lo, G.seed_hi);
-    const int free_cards = 52 - __popcll(used);
-    int k = (int)(((unsigned long long)w.x * (unsigned long long)free_cards) >> 32);
-    for (int c = 0; c < 52; ++c) {
-      if ((used >> c) & 1) continue;
-      if (k-- == 0) {
-        river = c;
-        break;
-      }
+    uint64_t spare = ~used & ((1ull << 52) - 1);
+    int k = (int)(((unsigned long long)w.x * (unsigned long long)__popcll(spare)) >> 32);
+    for (; k > 0; --k) spare &= spare - 1;
+    river = __ffsll((long long)spare) - 1;
+    fifth = river;
+  }
+  uint32_t* const words = reinterpret_cast<uint32_t*>(out);
+  if (gl < kMaxPlayers) {
+    uint32_t ctx = 0;
+    uint16_t rank = 0, hole = 0;
+    if (gl < N) {
+      int32_t b = __ldg(T + 53 + to_rm(G.sub_board[0]));
+      for (int i = 1; i < 4; ++i) b = __ldg(T + b + to_rm(G.sub_board[i]));
+      b = __ldg(T + b + to_rm(fifth));
+      int lo, hi;
+      combo_cards(mine, lo, hi);
+      const int32_t s6 = __ldg(T + b + to_rm(lo));
+      rank = (uint16_t)decode16((uint32_t)__ldg(T + s6 + to_rm(hi)) & 0xFFFF);
+      ctx = (uint32_t)mine | ((uint32_t)(river + 1) << 16);
+      hole = (uint16_t)(lo | hi << 8);
     }
-    r.board[4] = (uint8_t)river;
+    words[gl] = ctx;
+    out->rank[gl] = rank;
+    reinterpret_cast<uint16_t*>(out->hole)[gl] = hole;
+  } else if (gl == kMaxPlayers) {
+    words[12] = (uint32_t)G.sub_board[0] | (uint32_t)G.sub_board[1] << 8 | (uint32_t)G.sub_board[2] << 16 |
+                (uint32_t)G.sub_board[3] << 24;
+    words[13] = (uint32_t)fifth | (uint32_t)(N - 1) << 8;  // river card, dealer
+  } else {
+    words[14] = words[15] = 0;
   }
-  r.dealer = (uint8_t)(N - 1);
-  int32_t b = __ldg(T + 53 + to_rm(r.board[0]));
-  for (int i = 1; i < 5; ++i) b = __ldg(T + b + to_rm(r.board[i]));
-  for (int p = 0; p < kMaxPlayers; ++p) {
-    r.ctx[p] = 0;
-    r.rank[p] = 0;
-    r.hole[2 * p] = r.hole[2 * p + 1] = 0;
-    if (p >= N) continue;
-    int lo, hi;
-    combo_cards(combo[p], lo, hi);
-    r.hole[2 * p] = (uint8_t)lo;
-    r.hole[2 * p + 1] = (uint8_t)hi;
-    const int32_t s6 = __ldg(T + b + to_rm(lo));
-    r.rank[p] = (uint16_t)decode16((uint32_t)__ldg(T + s6 + to_rm(hi)) & 0xFFFF);
-    r.ctx[p] = (uint32_t)combo[p] | ((uint32_t)(river + 1) << 16);
-  }
-  const uint4* src = reinterpret_cast<const uint4*>(&r);
-  uint4* dst = reinterpret_cast<uint4*>(out);
-#pragma unroll
-  for (int i = 0; i < 4; ++i) dst[i] = src[i];
 }
 
 // Deal, buckets and river ranks of traversal t of update `uid`
 // (cfr_gpu.cu:460-470, 476-489, 942-952, 963).  `pre` is the 52x52 preflop LUT
-// (shared or global memory), `cdf` the rank-CDF LUTs.
+// (shared or global memory), `cdf` the rank-CDF LUTs, `row` this thread's 13 words
+// of shared memory for the deck: a shuffle indexes it by card, and as an array of
+// the thread it lived in local memory (2^18 six-player deals: 98 us).
+constexpr int kDeckWords = 13;  // an odd stride: a warp's decks lie in different banks
+
 __device__ __forceinline__ void deal_one(const GameParams& G, const int32_t* __restrict__ T, const uint8_t* pre,
                                          const uint8_t* __restrict__ cdf, uint32_t t, uint32_t uid,
-                                         DealRec* __restrict__ out) {
-  if (G.sub_street) {
-    deal_subgame(G, T, t, uid, out);
-    return;
-  }
+                                         DealRec* __restrict__ out, uint32_t* row) {
+  uint8_t* const deck = reinterpret_cast<uint8_t*>(row);
   const int N = G.N;
   const int n_deal = 2 * N + 5;
-  uint32_t words[24];
-  const int nblk = (n_deal + 1 + 3) / 4;
 #pragma unroll
-  for (int j = 0; j < 6; ++j) {
-    if (j < nblk) {
-      const U4 o = philox(U4{t, uid, 0u, (uint32_t)j}, G.seed_lo, G.seed_hi);
-      words[4 * j + 0] = o.x;
-      words[4 * j + 1] = o.y;
-      words[4 * j + 2] = o.z;
-      words[4 * j + 3] = o.w;
+  for (int w = 0; w < kDeckWords; ++w) row[w] = 0x03020100u + 0x04040404u * (uint32_t)w;  // cards 4w .. 4w+3
+  uint32_t dealer = 0;
+  for (int blk = 0; 4 * blk <= n_deal; ++blk) {
+    const U4 o = philox(U4{t, uid, 0u, (uint32_t)blk}, G.seed_lo, G.seed_hi);
+    const uint32_t wv[4] = {o.x, o.y, o.z, o.w};
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      const int i = 4 * blk + e;
+      if (i < n_deal) {
+        const int j = i + (int)__umulhi(wv[e], (uint32_t)(52 - i));
+        const uint8_t tmp = deck[i];
+        deck[i] = deck[j];
+        deck[j] = tmp;
+      } else if (i == n_deal) {
+        dealer = wv[e] % (uint32_t)N;
+      }
     }
   }
-  uint8_t deck[52];
+  int board[5];
 #pragma unroll
-  for (int i = 0; i < 52; ++i) deck[i] = (uint8_t)i;
-  for (int i = 0; i < n_deal; ++i) {
-    const int j = i + (int)(((unsigned long long)words[i] * (unsigned long long)(52 - i)) >> 32);
-    const uint8_t tmp = deck[i];
-    deck[i] = deck[j];
-    deck[j] = tmp;
-  }
-  DealRec r;
-#pragma unroll
-  for (int i = 0; i < 2 * kMaxPlayers; ++i) r.hole[i] = (i < 2 * N) ? deck[i] : 0;
-#pragma unroll
-  for (int i = 0; i < 5; ++i) r.board[i] = deck[2 * N + i];
-  r.dealer = (uint8_t)(words[n_deal] % (uint32_t)N);
-#pragma unroll
-  for (int i = 0; i < 10; ++i) r.pad[i] = 0;
-
-  int32_t b = __ldg(T + 53 + to_rm(r.board[0]));
-  b = __ldg(T + b + to_rm(r.board[1]));
-  b = __ldg(T + b + to_rm(r.board[2]));
+  for (int i = 0; i < 5; ++i) board[i] = deck[2 * N + i];
+  int32_t b = __ldg(T + 53 + to_rm(board[0]));
+  b = __ldg(T + b + to_rm(board[1]));
+  b = __ldg(T + b + to_rm(board[2]));
   int32_t s5[kMaxPlayers], s6[kMaxPlayers], r7[kMaxPlayers], s4[kMaxPlayers];
 #pragma unroll
   for (int p = 0; p < kMaxPlayers; ++p)
-    if (p < N) s4[p] = __ldg(T + b + to_rm(r.hole[2 * p]));
+    if (p < N) s4[p] = __ldg(T + b + to_rm(deck[2 * p]));
 #pragma unroll
   for (int p = 0; p < kMaxPlayers; ++p)
-    if (p < N) s5[p] = __ldg(T + s4[p] + to_rm(r.hole[2 * p + 1]));
-  const int rm3 = to_rm(r.board[3]), rm4 = to_rm(r.board[4]);
+    if (p < N) s5[p] = __ldg(T + s4[p] + to_rm(deck[2 * p + 1]));
+  const int rm3 = to_rm(board[3]), rm4 = to_rm(board[4]);
 #pragma unroll
   for (int p = 0; p < kMaxPlayers; ++p)
     if (p < N) s6[p] = __ldg(T + s5[p] + rm3);
 #pragma unroll
   for (int p = 0; p < kMaxPlayers; ++p)
     if (p < N) r7[p] = __ldg(T + s6[p] + rm4);
+  uint32_t ctx[kMaxPlayers], rank[kMaxPlayers];
 #pragma unroll
   for (int p = 0; p < kMaxPlayers; ++p) {
-    r.ctx[p] = 0;
-    r.rank[p] = 0;
+    ctx[p] = 0;
+    rank[p] = 0;
     if (p >= N) continue;
-    const uint32_t hb = pre[r.hole[2 * p] * 52 + r.hole[2 * p + 1]];
+    const uint32_t hb = pre[deck[2 * p] * 52 + deck[2 * p + 1]];
     const uint32_t rr = decode16((uint32_t)r7[p] & 0xFFFF);
     uint32_t b1, b2, b3;
     if (G.postflop_mode == 0) {
@@ -253,22 +277,28 @@ __device__ __forceinline__ void deal_one(const GameParams& G, const int32_t* __r
       b2 = ref_linear_bucket(decode16((uint32_t)s6[p] & 0xFFFF), G.post_b[1]);
       b3 = ref_linear_bucket(rr, G.post_b[2]);
     } else {
-      b1 = __ldg(cdf + decode16((uint32_t)__ldg(T + s5[p]) & 0xFFFF));
-      b2 = __ldg(cdf + 7463 + decode16((uint32_t)__ldg(T + s6[p]) & 0xFFFF));
+      b1 = __ldg(cdf + kStateBuckets + (uint32_t)s5[p] / 53u);
+      b2 = __ldg(cdf + kStateBuckets + (uint32_t)s6[p] / 53u);
       b3 = __ldg(cdf + 2 * 7463 + rr);
     }
-    r.ctx[p] = hb | (b1 << 8) | (b2 << 16) | (b3 << 24);
-    r.rank[p] = (uint16_t)rr;
+    ctx[p] = hb | (b1 << 8) | (b2 << 16) | (b3 << 24);
+    rank[p] = rr;
   }
-  const uint4* src = reinterpret_cast<const uint4*>(&r);
-  uint4* dst = reinterpret_cast<uint4*>(out);
-#pragma unroll
-  for (int i = 0; i < 4; ++i) dst[i] = src[i];
+  // the record, whole: ctx, ranks, hole cards (the deck's first 2N), board, dealer
+  uint4* const dst = reinterpret_cast<uint4*>(out);
+  dst[0] = make_uint4(ctx[0], ctx[1], ctx[2], ctx[3]);
+  dst[1] = make_uint4(ctx[4], ctx[5], rank[0] | rank[1] << 16, rank[2] | rank[3] << 16);
+  const uint32_t h1 = N == 2 ? 0u : N == 3 ? row[1] & 0xFFFFu : row[1];
+  const uint32_t h2 = N <= 4 ? 0u : N == 5 ? row[2] & 0xFFFFu : row[2];
+  dst[2] = make_uint4(rank[4] | rank[5] << 16, row[0], h1, h2);
+  dst[3] = make_uint4((uint32_t)board[0] | (uint32_t)board[1] << 8 | (uint32_t)board[2] << 16 |
+                          (uint32_t)board[3] << 24, (uint32_t)board[4] | dealer << 8, 0u, 0u);
 }
 
 // The deal starts an update: it advances the table's epoch and zeroes `ctl`, the
 // counters of the traversal that follows (may be null), so that neither needs a
-// launch of its own.
+// launch of its own.  SUB: a subgame (eight lanes per traversal).
+template <bool SUB>
 __global__ void __launch_bounds__(128) k_deal(const GameParams G, const HandView hv, const Sched* __restrict__ sched,
                                               int batch, DealRec* __restrict__ out, uint32_t* __restrict__ epoch,
                                               uint32_t* __restrict__ ctl, int ctl_words) {
@@ -276,13 +306,22 @@ __global__ void __launch_bounds__(128) k_deal(const GameParams G, const HandView
     if (threadIdx.x == 0) *epoch += 1;
     for (int i = threadIdx.x; i < ctl_words; i += blockDim.x) ctl[i] = 0;
   }
+  if (SUB) {
+    const uint32_t t = blockIdx.x * (128 / kDealGroup) + threadIdx.x / kDealGroup;
+    if (t >= (uint32_t)batch) return;  // whole groups
+    const int gl = (int)threadIdx.x & (kDealGroup - 1);
+    deal_subgame(G, hv.hr, t, update_id(sched, G.N), out + t, gl,
+                 ((1u << kDealGroup) - 1u) << ((threadIdx.x & 31) & ~(kDealGroup - 1)));
+    return;
+  }
   __shared__ uint8_t s_pre[52 * 52];
+  __shared__ uint32_t s_deck[128 * kDeckWords];
   for (int i = threadIdx.x; i < 52 * 52 / 4; i += blockDim.x)
     reinterpret_cast<uint32_t*>(s_pre)[i] = __ldg(reinterpret_cast<const uint32_t*>(hv.pre) + i);
   __syncthreads();
-  const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= (uint32_t)batch) return;
-  deal_one(G, hv.hr, s_pre, hv.cdf, t, update_id(sched, G.N), out + t);
+  const uint32_t uid = update_id(sched, G.N);
+  for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < (uint32_t)batch; t += gridDim.x * blockDim.x)
+    deal_one(G, hv.hr, s_pre, hv.cdf, t, uid, out + t, s_deck + kDeckWords * threadIdx.x);
 }
 
 // Side-pot showdown for player `up` (cfr_gpu.cu:694-753).  The distinct non-zero
