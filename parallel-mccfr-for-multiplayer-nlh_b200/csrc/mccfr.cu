@@ -253,32 +253,26 @@ __global__ void k_advance_batched(const TableDesc* __restrict__ tables, const Ph
   D.sched->player = p;
 }
 
-// Occupied rows of the table (one atomic per warp).
-__global__ void k_count_rows(const TableView tv, unsigned long long cap_slots, unsigned int* __restrict__ on) {
-  unsigned c = 0;
-  for (unsigned long long s = blockIdx.x * (unsigned long long)blockDim.x + threadIdx.x; s < cap_slots;
-       s += (unsigned long long)gridDim.x * blockDim.x)
-    c += *row_key(tv, s) != 0;
-  c = __reduce_add_sync(0xFFFFFFFFu, c);
-  if ((threadIdx.x & 31) == 0 && c) atomicAdd(on, c);
+// Rows that a key can own (the rest of a direct-mapped table stays empty).
+__device__ __forceinline__ unsigned long long owned_rows(const TableView& tv) {
+  return min(tv.mask + 1, (unsigned long long)tv.n_words * 32);
 }
 
 // Order-independent digest of the occupied rows (mccfr_table_digest).
-__global__ void k_digest(const TableView tv, unsigned long long cap_slots, unsigned long long* __restrict__ out) {
+__global__ void k_digest(const TableView tv, unsigned long long* __restrict__ out) {
   unsigned long long sum = 0, rows = 0;
-  for (unsigned long long s = blockIdx.x * (unsigned long long)blockDim.x + threadIdx.x; s < cap_slots;
+  const unsigned long long n = owned_rows(tv);
+  for (unsigned long long s = blockIdx.x * (unsigned long long)blockDim.x + threadIdx.x; s < n;
        s += (unsigned long long)gridDim.x * blockDim.x) {
-    const unsigned long long k = *row_key(tv, s);
+    const unsigned long long k = __ldcg(row_key(tv, s));
     if (!k) continue;
-    const uint32_t* r = reinterpret_cast<const uint32_t*>(row_reg(tv, s));
-    const uint32_t* q = reinterpret_cast<const uint32_t*>(row_ssum(tv, s));
-    uint32_t rb[8], qb[8];
-#pragma unroll
-    for (int a = 0; a < 8; ++a) {
-      rb[a] = r[a];
-      qb[a] = q[a];
-    }
-    sum += row_digest(k, rb, qb, *row_visits(tv, s));
+    const Sector r = ld_sector(row_reg(tv, s)), q = ld_sector(row_ssum(tv, s));
+    const unsigned long long v = __ldcg(row_visits(tv, s));
+    const uint32_t rb[8] = {(uint32_t)r.x, (uint32_t)(r.x >> 32), (uint32_t)r.y, (uint32_t)(r.y >> 32),
+                            (uint32_t)r.z, (uint32_t)(r.z >> 32), (uint32_t)r.w, (uint32_t)(r.w >> 32)};
+    const uint32_t qb[8] = {(uint32_t)q.x, (uint32_t)(q.x >> 32), (uint32_t)q.y, (uint32_t)(q.y >> 32),
+                            (uint32_t)q.z, (uint32_t)(q.z >> 32), (uint32_t)q.w, (uint32_t)(q.w >> 32)};
+    sum += row_digest(k, rb, qb, v);
     rows++;
   }
 #pragma unroll
@@ -292,23 +286,152 @@ __global__ void k_digest(const TableView tv, unsigned long long cap_slots, unsig
   }
 }
 
-// Compacts the occupied rows into arrays of `bound` rows (unordered).
-__global__ void k_export(const TableView tv, unsigned long long cap_slots,
-                         unsigned long long* __restrict__ okeys, float4* __restrict__ oreg,
-                         float4* __restrict__ ossum, unsigned long long* __restrict__ ovis,
-                         unsigned int* __restrict__ on, unsigned bound) {
-  for (unsigned long long s = blockIdx.x * (unsigned long long)blockDim.x + threadIdx.x; s < cap_slots;
-       s += (unsigned long long)gridDim.x * blockDim.x) {
-    const unsigned long long k = *row_key(tv, s);
-    if (!k) continue;
-    const unsigned i = atomicAdd(on, 1u);
-    if (i >= bound) continue;
-    okeys[i] = k;
-    oreg[2 * i] = row_reg(tv, s)[0];
-    oreg[2 * i + 1] = row_reg(tv, s)[1];
-    ossum[2 * i] = row_ssum(tv, s)[0];
-    ossum[2 * i + 1] = row_ssum(tv, s)[1];
-    ovis[i] = *row_visits(tv, s);
+// Reading a table back: its wanted rows are counted span by span, the counts are
+// turned into offsets, and every span writes its rows at its offset, so the rows
+// come out in slot order.  In a direct-mapped table that is key order, and the
+// host neither sorts nor rearranges what it copies (2^20 rows: 130 ms of host
+// work before).
+enum { kReadRows = 0, kReadStrategy = 1, kReadActive = 2 };
+constexpr int kReadSpan = 1024;  // rows of one block: 8 warps of 4 x 32 rows
+constexpr int kReadBlock = 256;
+
+// Whether row s is wanted: occupied (rows), with a strategy that normalises
+// (strategy; `q` becomes it), or with a positive strategy sum (active).
+template <int WHAT>
+__device__ __forceinline__ bool read_wanted(const TableView& tv, unsigned long long s, unsigned long long& key,
+                                            float* q) {
+  key = __ldcg(row_key(tv, s));
+  if (!key) return false;
+  if (WHAT == kReadRows) return true;
+  const Sector v = ld_sector(row_ssum(tv, s));
+  q[0] = lo_float(v.x); q[1] = hi_float(v.x); q[2] = lo_float(v.y); q[3] = hi_float(v.y);
+  q[4] = lo_float(v.z); q[5] = hi_float(v.z); q[6] = lo_float(v.w); q[7] = hi_float(v.w);
+  if (WHAT == kReadActive) {
+    bool any = false;
+#pragma unroll
+    for (int a = 0; a < 8; ++a) any |= q[a] > 0.0f;
+    return any;
+  }
+  // the reference's normalisation and host filter (cfr_gpu.cu:1029-1058, 1399-1411)
+  float tot = 0.0f, t2 = 0.0f;
+#pragma unroll
+  for (int a = 0; a < 8; ++a) tot = __fadd_rn(tot, q[a]);
+#pragma unroll
+  for (int a = 0; a < 8; ++a) {
+    q[a] = tot > 1e-7f ? __fdiv_rn(q[a], tot) : 0.0f;
+    t2 = __fadd_rn(t2, q[a]);
+  }
+  return !(t2 < 1e-6f);
+}
+
+template <int WHAT>
+__global__ void __launch_bounds__(kReadBlock) k_read_count(const TableView tv, unsigned* __restrict__ counts) {
+  const unsigned long long n = owned_rows(tv), base = (unsigned long long)blockIdx.x * kReadSpan;
+  unsigned c = 0;
+  for (int i = threadIdx.x; i < kReadSpan; i += kReadBlock) {
+    unsigned long long key;
+    float q[8];
+    c += base + i < n && read_wanted<WHAT>(tv, base + i, key, q) ? 1u : 0u;
+  }
+  __shared__ unsigned s_c[kReadBlock / 32];
+  c = __reduce_add_sync(0xFFFFFFFFu, c);
+  if ((threadIdx.x & 31) == 0) s_c[threadIdx.x >> 5] = c;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    unsigned t = 0;
+    for (int w = 0; w < kReadBlock / 32; ++w) t += s_c[w];
+    counts[blockIdx.x] = t;
+  }
+}
+
+// counts[0..n) become their exclusive sums; *total their sum.  One block.
+__global__ void __launch_bounds__(1024) k_read_offsets(unsigned* __restrict__ counts, unsigned n,
+                                                       unsigned* __restrict__ total) {
+  __shared__ unsigned s_w[32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  unsigned carry = 0;
+  for (unsigned at = 0; at < n; at += 4096) {
+    // four consecutive counts per thread
+    const unsigned i = at + 4 * threadIdx.x;
+    unsigned v[4], t = 0;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      v[k] = i + k < n ? counts[i + k] : 0u;
+      t += v[k];
+    }
+    unsigned x = t;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const unsigned y = __shfl_up_sync(0xFFFFFFFFu, x, o);
+      if (lane >= o) x += y;
+    }
+    if (lane == 31) s_w[warp] = x;
+    __syncthreads();
+    unsigned before = carry + x - t;
+    unsigned sum = 0;
+    for (int w = 0; w < 32; ++w) {
+      if (w < warp) before += s_w[w];
+      sum += s_w[w];
+    }
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      if (i + k < n) counts[i + k] = before;
+      before += v[k];
+    }
+    carry += sum;
+    __syncthreads();
+  }
+  if (threadIdx.x == 0) *total = carry;
+}
+
+// Where k_read_write puts the rows (null: not wanted).
+struct ReadOut {
+  unsigned long long* keys;
+  unsigned* keys32;  // key32_sub: 1 where the 32-bit key is the FNV slot (key - 1)
+  Sector* regrets;
+  Sector* sums;      // strategy sums, or strategies
+  unsigned long long* visits;
+  unsigned key32_sub;
+};
+
+template <int WHAT>
+__global__ void __launch_bounds__(kReadBlock) k_read_write(const TableView tv, const unsigned* __restrict__ offsets,
+                                                           const ReadOut out) {
+  const unsigned long long n = owned_rows(tv);
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const unsigned long long base = (unsigned long long)blockIdx.x * kReadSpan + warp * 128;
+  unsigned long long key[4];
+  float q[4][8];
+  unsigned m[4], c = 0;
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    const unsigned long long s = base + 32 * k + lane;
+    key[k] = 0;
+    const bool want = s < n && read_wanted<WHAT>(tv, s, key[k], q[k]);
+    m[k] = __ballot_sync(0xFFFFFFFFu, want);
+    c += __popc(m[k]);
+  }
+  __shared__ unsigned s_c[kReadBlock / 32];
+  if (lane == 0) s_c[warp] = c;
+  __syncthreads();
+  unsigned at = offsets[blockIdx.x];
+  for (int w = 0; w < warp; ++w) at += s_c[w];
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    const unsigned i = at + __popc(m[k] & ((1u << lane) - 1u));
+    at += __popc(m[k]);
+    if (!((m[k] >> lane) & 1)) continue;
+    const unsigned long long s = base + 32 * k + lane;
+    if (out.keys) out.keys[i] = key[k];
+    if (out.keys32) out.keys32[i] = (unsigned)key[k] - out.key32_sub;
+    if (WHAT == kReadRows) {
+      if (out.regrets) out.regrets[i] = ld_sector(row_reg(tv, s));
+      if (out.sums) out.sums[i] = ld_sector(row_ssum(tv, s));
+      if (out.visits) out.visits[i] = __ldcg(row_visits(tv, s));
+    } else if (out.sums) {
+      out.sums[i] = Sector{two_floats(q[k][0], q[k][1]), two_floats(q[k][2], q[k][3]),
+                           two_floats(q[k][4], q[k][5]), two_floats(q[k][6], q[k][7])};
+    }
   }
 }
 
@@ -500,6 +623,11 @@ struct mccfr_handle {
   double traverse_ms = 0, apply_ms = 0, last_traverse_ms = 0, last_apply_ms = 0;
   long long touched_last = 0;
   long long wide_last = 0;  // of those, rows whose second line was folded
+  // scratch of calls that read the table back or stage host data, kept between
+  // calls up to kScratchKept bytes, and the span counts of table reads
+  void* d_scratch = nullptr;
+  size_t scratch_bytes = 0;
+  unsigned* d_spans = nullptr;
   int sticky_err = 0;
   std::string last_error;
   size_t persist_prev = 0;
@@ -1018,21 +1146,60 @@ struct HostRow {
 };
 static_assert(sizeof(HostRow) == 80, "a v2 checkpoint row is 80 bytes");
 
-// Occupied rows (a counting pass over the table).
-int count_rows(mccfr_handle* h, unsigned int* n) {
-  CK(cudaStreamSynchronize(h->stream));
-  unsigned int* d_n = nullptr;
-  CK(cudaMalloc(&d_n, sizeof(unsigned int)));
-  cudaError_t e = cudaMemsetAsync(d_n, 0, sizeof(unsigned int), h->stream);
-  if (e == cudaSuccess) {
-    k_count_rows<<<148 * 16, 256, 0, h->stream>>>(h->tv, h->cap, d_n);
-    e = cudaMemcpyAsync(n, d_n, sizeof(unsigned int), cudaMemcpyDeviceToHost, h->stream);
+// Device scratch of one call.  Blocks up to kScratchKept stay with the handle for
+// the next call; larger ones are freed at the end of the call.
+constexpr size_t kScratchKept = 128u << 20;
+struct Scratch {
+  mccfr_handle* h;
+  void* p = nullptr;
+  bool own = false;
+  explicit Scratch(mccfr_handle* hh) : h(hh) {}
+  Scratch(const Scratch&) = delete;
+  Scratch& operator=(const Scratch&) = delete;
+  cudaError_t take(size_t bytes) {
+    if (bytes <= h->scratch_bytes) {
+      p = h->d_scratch;
+      return cudaSuccess;
+    }
+    if (bytes > kScratchKept) {
+      own = true;
+      return cudaMalloc(&p, bytes);
+    }
+    cudaFree(h->d_scratch);
+    h->d_scratch = nullptr;
+    h->scratch_bytes = 0;
+    const size_t want = std::min(kScratchKept, std::max<size_t>(bytes + bytes / 4, 1u << 20));
+    const cudaError_t e = cudaMalloc(&h->d_scratch, want);
+    if (e != cudaSuccess) {
+      h->d_scratch = nullptr;
+      return e;
+    }
+    h->scratch_bytes = want;
+    p = h->d_scratch;
+    return cudaSuccess;
   }
-  if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
-  cudaFree(d_n);
-  if (e != cudaSuccess) return fail(h, MCCFR_ERR_CUDA, "row count: %s", cudaGetErrorString(e));
+  ~Scratch() {
+    if (own) cudaFree(p);
+  }
+};
+
+// Counts the wanted rows (kRead*) into the handle's span offsets; *n = how many.
+int count_read(mccfr_handle* h, int what, unsigned* n) {
+  const unsigned long long rows = std::min(h->cap, (unsigned long long)h->tv.n_words * 32);
+  const unsigned spans = (unsigned)((rows + kReadSpan - 1) / kReadSpan);
+  // room for every span of the table, so that a re-targeted handle keeps it
+  if (!h->d_spans) CK(cudaMalloc(&h->d_spans, ((h->cap + kReadSpan - 1) / kReadSpan + 1) * sizeof(unsigned)));
+  if (what == kReadRows) k_read_count<kReadRows><<<spans, kReadBlock, 0, h->stream>>>(h->tv, h->d_spans);
+  else if (what == kReadStrategy) k_read_count<kReadStrategy><<<spans, kReadBlock, 0, h->stream>>>(h->tv, h->d_spans);
+  else k_read_count<kReadActive><<<spans, kReadBlock, 0, h->stream>>>(h->tv, h->d_spans);
+  k_read_offsets<<<1, 1024, 0, h->stream>>>(h->d_spans, spans, h->d_spans + spans);
+  CK(cudaGetLastError());
+  CK(cudaMemcpyAsync(n, h->d_spans + spans, sizeof(unsigned), cudaMemcpyDeviceToHost, h->stream));
+  CK(cudaStreamSynchronize(h->stream));
   return MCCFR_OK;
 }
+
+int count_rows(mccfr_handle* h, unsigned int* n) { return count_read(h, kReadRows, n); }
 
 // Indices of `k` in ascending key order: LSD radix sort, 8 bits per pass,
 // skipping the bytes in which all keys agree (keys are distinct).
@@ -1057,47 +1224,88 @@ void order_by_key(const std::vector<unsigned long long>& k, std::vector<unsigned
   }
 }
 
-// Every occupied row, sorted by key: counted first, then compacted into
-// buffers of exactly that many rows and copied back.
-int read_rows(mccfr_handle* h, std::vector<HostRow>& rows) {
-  unsigned int n = 0;
-  int rc = count_rows(h, &n);
-  if (rc) return rc;
-  rows.clear();
+// The rows that count_read counted last (kReadRows or kReadStrategy, `n` of them),
+// in ascending key order, into host arrays; null arrays are skipped.  `sums`
+// receives strategy sums or strategies.
+int fetch_rows(mccfr_handle* h, int what, unsigned n, uint64_t* keys, uint32_t* keys32, float* regrets, float* sums,
+               uint64_t* visits) {
   if (n == 0) return MCCFR_OK;
-  void* block = nullptr;
-  const size_t bytes = (size_t)n * (8 + 8 + 32 + 32) + 256;
-  cudaError_t e = cudaMalloc(&block, bytes);
-  if (e != cudaSuccess) return fail(h, MCCFR_ERR_OOM, "export buffers: %s", cudaGetErrorString(e));
-  char* base = static_cast<char*>(block);
-  float4* oreg = reinterpret_cast<float4*>(base);
-  float4* ossum = reinterpret_cast<float4*>(base + (size_t)n * 32);
-  unsigned long long* okeys = reinterpret_cast<unsigned long long*>(base + (size_t)n * 64);
-  unsigned long long* ovis = reinterpret_cast<unsigned long long*>(base + (size_t)n * 72);
-  unsigned int* d_n = reinterpret_cast<unsigned int*>(base + (size_t)n * 80);
-  std::vector<unsigned long long> k(n), v(n);
-  std::vector<float> r(8ull * n), s(8ull * n);
-  e = cudaMemsetAsync(d_n, 0, sizeof(unsigned int), h->stream);
-  if (e == cudaSuccess) {
-    k_export<<<148 * 16, 256, 0, h->stream>>>(h->tv, h->cap, okeys, oreg, ossum, ovis, d_n, n);
-    e = cudaGetLastError();
+  const unsigned long long rows = std::min(h->cap, (unsigned long long)h->tv.n_words * 32);
+  const unsigned spans = (unsigned)((rows + kReadSpan - 1) / kReadSpan);
+  const bool sort = !h->tv.direct;  // slots of an open-addressed table are in no order
+  const bool k64 = keys || sort;
+  Scratch scratch(h);
+  const size_t bytes = (size_t)n * ((regrets ? 32 : 0) + (sums ? 32 : 0) + (k64 ? 8 : 0) + (visits ? 8 : 0) +
+                                    (keys32 && !sort ? 4 : 0));
+  const cudaError_t e0 = scratch.take(bytes);
+  if (e0 != cudaSuccess) {
+    cudaGetLastError();
+    return fail(h, MCCFR_ERR_OOM, "export buffers: %s", cudaGetErrorString(e0));
   }
-  if (e == cudaSuccess) e = cudaMemcpyAsync(k.data(), okeys, n * 8ull, cudaMemcpyDeviceToHost, h->stream);
-  if (e == cudaSuccess) e = cudaMemcpyAsync(v.data(), ovis, n * 8ull, cudaMemcpyDeviceToHost, h->stream);
-  if (e == cudaSuccess) e = cudaMemcpyAsync(r.data(), oreg, n * 32ull, cudaMemcpyDeviceToHost, h->stream);
-  if (e == cudaSuccess) e = cudaMemcpyAsync(s.data(), ossum, n * 32ull, cudaMemcpyDeviceToHost, h->stream);
-  if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
-  cudaFree(block);
-  if (e != cudaSuccess) return fail(h, MCCFR_ERR_CUDA, "export: %s", cudaGetErrorString(e));
+  char* p = static_cast<char*>(scratch.p);
+  const auto carve = [&](bool want, size_t width) -> void* {
+    if (!want) return nullptr;
+    void* q = p;
+    p += width * n;
+    return q;
+  };
+  ReadOut out{};
+  out.regrets = static_cast<Sector*>(carve(regrets, 32));
+  out.sums = static_cast<Sector*>(carve(sums, 32));
+  out.keys = static_cast<unsigned long long*>(carve(k64, 8));
+  out.visits = static_cast<unsigned long long*>(carve(visits, 8));
+  out.keys32 = static_cast<unsigned*>(carve(keys32 && !sort, 4));
+  out.key32_sub = h->cfg.key_mode == MCCFR_KEY_FNV26 ? 1u : 0u;
+  if (what == kReadRows) k_read_write<kReadRows><<<spans, kReadBlock, 0, h->stream>>>(h->tv, h->d_spans, out);
+  else k_read_write<kReadStrategy><<<spans, kReadBlock, 0, h->stream>>>(h->tv, h->d_spans, out);
+  CK(cudaGetLastError());
+  const auto copy = [&](void* dst, const void* src, size_t width) {
+    return dst ? cudaMemcpyAsync(dst, src, width * n, cudaMemcpyDeviceToHost, h->stream) : cudaSuccess;
+  };
+  if (!sort) {
+    CK(copy(keys, out.keys, 8));
+    CK(copy(keys32, out.keys32, 4));
+    CK(copy(regrets, out.regrets, 32));
+    CK(copy(sums, out.sums, 32));
+    CK(copy(visits, out.visits, 8));
+    CK(cudaStreamSynchronize(h->stream));
+    return MCCFR_OK;
+  }
+  std::vector<unsigned long long> k(n), v(visits ? n : 0);
+  std::vector<float> r(regrets ? 8ull * n : 0), q(sums ? 8ull * n : 0);
+  CK(copy(k.data(), out.keys, 8));
+  CK(copy(visits ? v.data() : nullptr, out.visits, 8));
+  CK(copy(regrets ? r.data() : nullptr, out.regrets, 32));
+  CK(copy(sums ? q.data() : nullptr, out.sums, 32));
+  CK(cudaStreamSynchronize(h->stream));
   std::vector<unsigned> order;
   order_by_key(k, order);
-  rows.resize(n);
   for (unsigned j = 0; j < n; ++j) {
     const unsigned i = order[j];
-    rows[j].key = k[i];
-    std::memcpy(rows[j].reg, &r[8ull * i], 32);
-    std::memcpy(rows[j].ssum, &s[8ull * i], 32);
-    rows[j].visits = v[i];
+    if (keys) keys[j] = k[i];
+    if (keys32) keys32[j] = (uint32_t)k[i] - out.key32_sub;
+    if (visits) visits[j] = v[i];
+    if (regrets) std::memcpy(regrets + 8ull * j, &r[8ull * i], 32);
+    if (sums) std::memcpy(sums + 8ull * j, &q[8ull * i], 32);
+  }
+  return MCCFR_OK;
+}
+
+// Every occupied row, sorted by key, as v2 checkpoint records.
+int read_host_rows(mccfr_handle* h, std::vector<HostRow>& rows) {
+  unsigned n = 0;
+  int rc = count_read(h, kReadRows, &n);
+  if (rc) return rc;
+  std::vector<uint64_t> keys(n), vis(n);
+  std::vector<float> reg(8ull * n), ssum(8ull * n);
+  rc = fetch_rows(h, kReadRows, n, keys.data(), nullptr, reg.data(), ssum.data(), vis.data());
+  if (rc) return rc;
+  rows.resize(n);
+  for (unsigned i = 0; i < n; ++i) {
+    rows[i].key = keys[i];
+    std::memcpy(rows[i].reg, &reg[8ull * i], 32);
+    std::memcpy(rows[i].ssum, &ssum[8ull * i], 32);
+    rows[i].visits = vis[i];
   }
   return MCCFR_OK;
 }
@@ -1126,6 +1334,8 @@ void release(mccfr_handle* h) {
   cudaFree(h->d_work);
   cudaFree(h->d_level);
   cudaFree(h->d_walk);
+  cudaFree(h->d_scratch);
+  cudaFree(h->d_spans);
   if (h->stream) cudaStreamDestroy(h->stream);
   delete h;
 }
@@ -1571,7 +1781,7 @@ int mccfr_table_digest(mccfr_handle* h, uint64_t* digest, uint64_t* rows) {
   unsigned long long out[2] = {0, 0};
   cudaError_t e = cudaMemsetAsync(d, 0, sizeof(out), h->stream);
   if (e == cudaSuccess) {
-    k_digest<<<148 * 16, 256, 0, h->stream>>>(h->tv, h->cap, d);
+    k_digest<<<148 * 16, 256, 0, h->stream>>>(h->tv, d);
     e = cudaGetLastError();
   }
   if (e == cudaSuccess) e = cudaMemcpyAsync(out, d, sizeof(out), cudaMemcpyDeviceToHost, h->stream);
@@ -1593,18 +1803,12 @@ int mccfr_export_rows(mccfr_handle* h, uint64_t* keys, float* regrets, float* st
     *count = n;
     return rc ? rc : (n ? MCCFR_ERR_CAPACITY : MCCFR_OK);
   }
-  std::vector<HostRow> rows;
-  const int rc = read_rows(h, rows);
+  unsigned n = 0;
+  const int rc = count_read(h, kReadRows, &n);
   if (rc) return rc;
-  *count = rows.size();
-  if (capacity < rows.size()) return MCCFR_ERR_CAPACITY;
-  for (size_t i = 0; i < rows.size(); ++i) {
-    if (keys) keys[i] = rows[i].key;
-    if (regrets) std::memcpy(regrets + 8 * i, rows[i].reg, 32);
-    if (strategy_sum) std::memcpy(strategy_sum + 8 * i, rows[i].ssum, 32);
-    if (visits) visits[i] = rows[i].visits;
-  }
-  return MCCFR_OK;
+  *count = n;
+  if (capacity < n) return MCCFR_ERR_CAPACITY;
+  return fetch_rows(h, kReadRows, n, keys, nullptr, regrets, strategy_sum, visits);
 }
 
 // Average strategy (cfr_gpu.cu:1029-1058 normalisation, 1399-1411 host filter).
@@ -1618,48 +1822,21 @@ int mccfr_get_strategy(mccfr_handle* h, uint32_t* keys, uint64_t* keys64, float*
     *count = n;
     return rc ? rc : (n ? MCCFR_ERR_CAPACITY : MCCFR_OK);
   }
-  std::vector<HostRow> rows;
-  const int rc = read_rows(h, rows);
+  unsigned n = 0;
+  const int rc = count_read(h, kReadStrategy, &n);
   if (rc) return rc;
-  size_t n = 0;
-  std::vector<std::pair<unsigned long long, std::array<float, 8>>> out;
-  out.reserve(rows.size());
-  for (const HostRow& r : rows) {
-    float tot = 0.0f;
-    for (int a = 0; a < 8; ++a) tot += r.ssum[a];
-    std::array<float, 8> pr;
-    for (int a = 0; a < 8; ++a) pr[a] = (tot > 1e-7f) ? r.ssum[a] / tot : 0.0f;
-    float t2 = 0.0f;
-    for (int a = 0; a < 8; ++a) t2 += pr[a];
-    if (t2 < 1e-6f) continue;
-    out.push_back({r.key, pr});
-  }
-  n = out.size();
   *count = n;
   if (capacity < n) return MCCFR_ERR_CAPACITY;
-  for (size_t i = 0; i < n; ++i) {
-    const unsigned long long k = out[i].first;
-    if (keys) keys[i] = (h->cfg.key_mode == MCCFR_KEY_FNV26) ? (uint32_t)(k - 1) : (uint32_t)k;
-    if (keys64) keys64[i] = k;
-    if (probs) std::memcpy(probs + 8 * i, out[i].second.data(), 32);
-  }
-  return MCCFR_OK;
+  return fetch_rows(h, kReadStrategy, n, keys64, keys, nullptr, probs, nullptr);
 }
 
 int mccfr_num_info_sets_active(mccfr_handle* h, long long* out) {
   if (!h || !out) return MCCFR_ERR_INVALID_ARG;
-  std::vector<HostRow> rows;
-  const int rc = read_rows(h, rows);
-  if (rc) return rc;
-  long long n = 0;
-  for (const HostRow& r : rows)
-    for (int a = 0; a < 8; ++a)
-      if (r.ssum[a] > 0.f) {
-        ++n;
-        break;
-      }
-  *out = n;
-  return MCCFR_OK;
+  CK(cudaSetDevice(h->device));
+  unsigned n = 0;
+  const int rc = count_read(h, kReadActive, &n);
+  *out = rc ? 0 : (long long)n;
+  return rc;
 }
 
 int mccfr_export_tables(mccfr_handle* h, float* regrets, float* strategy_sum, size_t n) {
@@ -1792,7 +1969,7 @@ int mccfr_save_checkpoint_v2(mccfr_handle* h, const char* path) {
   if (!h || !path) return MCCFR_ERR_INVALID_ARG;
   CK(cudaSetDevice(h->device));
   std::vector<HostRow> rows;
-  const int rc = read_rows(h, rows);
+  const int rc = read_host_rows(h, rows);
   if (rc) return rc;
   FILE* f = fopen(path, "wb");
   if (!f) return fail(h, MCCFR_ERR_IO, "cannot open %s", path);
@@ -1919,21 +2096,25 @@ int mccfr_eval7(mccfr_handle* h, const uint8_t* cards, uint16_t* ranks, size_t n
   if (!h || !cards || !ranks) return MCCFR_ERR_INVALID_ARG;
   if (!h->has_table) return fail(h, MCCFR_ERR_NO_HAND_TABLE, "load a hand-rank table first");
   if (n == 0) return MCCFR_OK;
-  for (size_t i = 0; i < 7 * n; ++i)
-    if (cards[i] > 51) return fail(h, MCCFR_ERR_INVALID_ARG, "card code %d out of range", (int)cards[i]);
+  unsigned char worst = 0;
+  for (size_t i = 0; i < 7 * n; ++i) worst = std::max(worst, cards[i]);
+  if (worst > 51)
+    for (size_t i = 0; i < 7 * n; ++i)
+      if (cards[i] > 51) return fail(h, MCCFR_ERR_INVALID_ARG, "card code %d out of range", (int)cards[i]);
   CK(cudaSetDevice(h->device));
-  uint8_t* dc = nullptr;
-  uint16_t* dr = nullptr;
-  CK(cudaMalloc(&dc, 7 * n));
-  cudaError_t e = cudaMalloc(&dr, 2 * n);
-  int rc = MCCFR_OK;
-  if (e == cudaSuccess) e = cudaMemcpyAsync(dc, cards, 7 * n, cudaMemcpyHostToDevice, h->stream);
-  if (e == cudaSuccess) rc = mccfr_eval7_device(h, dc, dr, n, nullptr);
-  if (e == cudaSuccess && !rc) e = cudaMemcpy(ranks, dr, 2 * n, cudaMemcpyDeviceToHost);
-  if (e != cudaSuccess) rc = fail(h, MCCFR_ERR_CUDA, "eval7: %s", cudaGetErrorString(e));
-  cudaFree(dc);
-  cudaFree(dr);
-  return rc;
+  Scratch scratch(h);
+  const size_t at = (7 * n + 15) & ~(size_t)15;  // the ranks, after the cards
+  const cudaError_t e = scratch.take(at + 2 * n);
+  if (e != cudaSuccess) return fail(h, e == cudaErrorMemoryAllocation ? MCCFR_ERR_OOM : MCCFR_ERR_CUDA,
+                                    "eval7 buffers: %s", cudaGetErrorString(e));
+  uint8_t* dc = static_cast<uint8_t*>(scratch.p);
+  uint16_t* dr = reinterpret_cast<uint16_t*>(dc + at);
+  CK(cudaMemcpyAsync(dc, cards, 7 * n, cudaMemcpyHostToDevice, h->stream));
+  k_eval7<<<grid_for((long long)n, 256), 256, 0, h->stream>>>(h->d_hr, dc, dr, n);
+  CK(cudaGetLastError());
+  CK(cudaMemcpyAsync(ranks, dr, 2 * n, cudaMemcpyDeviceToHost, h->stream));
+  CK(cudaStreamSynchronize(h->stream));
+  return MCCFR_OK;
 }
 
 int mccfr_level_counts(mccfr_handle* h, uint32_t* seeds, uint32_t* nodes, int cap, int* levels,
@@ -2799,15 +2980,13 @@ int mccfr_exploitability(mccfr_handle* h, const mccfr_br_options* opt, mccfr_exp
   if (!h || !out) return MCCFR_ERR_INVALID_ARG;
   if (!h->has_table) return fail(h, MCCFR_ERR_NO_HAND_TABLE, "no hand table loaded");
   CK(cudaSetDevice(h->device));
-  std::vector<HostRow> rows;
-  int rc = read_rows(h, rows);
+  unsigned n = 0;
+  int rc = count_read(h, kReadRows, &n);
   if (rc) return rc;
-  std::vector<uint64_t> keys(rows.size());
-  std::vector<float> ssum(rows.size() * 8);
-  for (size_t i = 0; i < rows.size(); ++i) {
-    keys[i] = rows[i].key;
-    std::memcpy(&ssum[8 * i], rows[i].ssum, 32);
-  }
+  std::vector<uint64_t> keys(n);
+  std::vector<float> ssum(8ull * n);
+  rc = fetch_rows(h, kReadRows, n, keys.data(), nullptr, nullptr, ssum.data(), nullptr);
+  if (rc) return rc;
   std::vector<int32_t> table(MCCFR_HAND_TABLE_ENTRIES);
   CK(cudaMemcpy(table.data(), h->d_hr, table.size() * sizeof(int32_t), cudaMemcpyDeviceToHost));
   mccfr_br_options o;
@@ -2819,7 +2998,7 @@ int mccfr_exploitability(mccfr_handle* h, const mccfr_br_options* opt, mccfr_exp
   in.T = table.data();
   in.keys = keys.data();
   in.ssum = ssum.data();
-  in.rows = rows.size();
+  in.rows = keys.size();
   if (h->gp.sub_street) {
     std::vector<uint32_t> cdf(2 * 1326);
     CK(cudaMemcpy(cdf.data(), h->d_ranges, cdf.size() * 4, cudaMemcpyDeviceToHost));

@@ -306,22 +306,22 @@ __global__ void __launch_bounds__(128) k_deal(const GameParams G, const HandView
     if (threadIdx.x == 0) *epoch += 1;
     for (int i = threadIdx.x; i < ctl_words; i += blockDim.x) ctl[i] = 0;
   }
-  if (SUB) {
+  if constexpr (SUB) {
     const uint32_t t = blockIdx.x * (128 / kDealGroup) + threadIdx.x / kDealGroup;
     if (t >= (uint32_t)batch) return;  // whole groups
     const int gl = (int)threadIdx.x & (kDealGroup - 1);
     deal_subgame(G, hv.hr, t, update_id(sched, G.N), out + t, gl,
                  ((1u << kDealGroup) - 1u) << ((threadIdx.x & 31) & ~(kDealGroup - 1)));
-    return;
+  } else {
+    __shared__ uint8_t s_pre[52 * 52];
+    __shared__ uint32_t s_deck[128 * kDeckWords];
+    for (int i = threadIdx.x; i < 52 * 52 / 4; i += blockDim.x)
+      reinterpret_cast<uint32_t*>(s_pre)[i] = __ldg(reinterpret_cast<const uint32_t*>(hv.pre) + i);
+    __syncthreads();
+    const uint32_t uid = update_id(sched, G.N);
+    for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < (uint32_t)batch; t += gridDim.x * blockDim.x)
+      deal_one(G, hv.hr, s_pre, hv.cdf, t, uid, out + t, s_deck + kDeckWords * threadIdx.x);
   }
-  __shared__ uint8_t s_pre[52 * 52];
-  __shared__ uint32_t s_deck[128 * kDeckWords];
-  for (int i = threadIdx.x; i < 52 * 52 / 4; i += blockDim.x)
-    reinterpret_cast<uint32_t*>(s_pre)[i] = __ldg(reinterpret_cast<const uint32_t*>(hv.pre) + i);
-  __syncthreads();
-  const uint32_t uid = update_id(sched, G.N);
-  for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < (uint32_t)batch; t += gridDim.x * blockDim.x)
-    deal_one(G, hv.hr, s_pre, hv.cdf, t, uid, out + t, s_deck + kDeckWords * threadIdx.x);
 }
 
 // Side-pot showdown for player `up` (cfr_gpu.cu:694-753).  The distinct non-zero
