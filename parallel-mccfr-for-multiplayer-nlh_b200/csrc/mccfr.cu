@@ -33,6 +33,7 @@
 #include "traverse_es.cuh"
 #include "traverse_levels.cuh"
 #include "traverse_walk.cuh"
+#include "traverse_path.cuh"
 #include "showdown.cuh"
 #include "batched.cuh"
 #include "best_response.h"
@@ -48,8 +49,6 @@ using namespace mccfr;
 // Small kernels
 // ---------------------------------------------------------------------------
 namespace {
-
-constexpr int kRefBlock = 128;
 
 // Folds one player-update's accumulators into the rows it touched and zeroes
 // them (the sparse equivalent of kernel_clamp_regrets, cfr_gpu.cu:1018-1022).
@@ -613,6 +612,7 @@ struct mccfr_handle {
   void* d_walk = nullptr;
   int walk_blocks = 0;    // blocks the records were allocated for
   int walk_resident = 0;  // resident blocks on this handle's device
+  int path_resident = 0;  // the same for the reference rule's kernel
   bool last_walk = false;  // the last external-sampling update ran in the walk form
   WalkBufs wb{};
   // graph of one iteration
@@ -841,6 +841,7 @@ cudaError_t launch_deals(const TableDesc* d_tables, const PhaseDesc* d_phase, co
 bool use_walk(const mccfr_handle* h);
 bool use_levels(const mccfr_handle* h);
 int enqueue_walk(mccfr_handle* h, int batch, float rscale);
+int enqueue_path(mccfr_handle* h, int batch, float rscale, mccfr_trace* d_trace);
 int enqueue_levels(mccfr_handle* h, int batch, float rscale);
 
 // Enqueues one player-update (traverse + apply) reading the device schedule;
@@ -852,8 +853,9 @@ int enqueue_update(mccfr_handle* h, int batch, mccfr_trace* d_trace, cudaEvent_t
   HandView hv{h->d_hr, h->d_pre, h->d_cdf};
   if (batch > h->deals_cap) return fail(h, MCCFR_ERR_INVALID_ARG, "deal buffer smaller than the batch");
   const bool walk = use_walk(h);
-  uint32_t* const ctl = walk ? reinterpret_cast<uint32_t*>(h->wb.ctl) : nullptr;
-  const int ctl_words = walk ? (int)(sizeof(WalkCtl) / 4) : 0;
+  // the traversal's counters, which the deal zeroes
+  uint32_t* const ctl = walk ? reinterpret_cast<uint32_t*>(h->wb.ctl) : h->d_work;
+  const int ctl_words = walk ? (int)(sizeof(WalkCtl) / 4) : 1;
   if (h->gp.sub_street)
     k_deal<true><<<(int)(((long long)batch * kDealGroup + 127) / 128), 128, 0, h->stream>>>(
         h->gp, hv, h->d_sched, batch, h->d_deals, table_epoch(h->tv), ctl, ctl_words);
@@ -863,13 +865,8 @@ int enqueue_update(mccfr_handle* h, int batch, mccfr_trace* d_trace, cudaEvent_t
   CK(cudaGetLastError());
   if (ev3 && record(h, ev3[0], capturing)) return MCCFR_ERR_CUDA;
   if (h->cfg.sampling == MCCFR_SAMPLING_REFERENCE) {
-    const int grid = (batch + kRefBlock - 1) / kRefBlock;
-    if (d_trace)
-      k_traverse_ref<kRefBlock, true><<<grid, kRefBlock, 0, h->stream>>>(h->gp, h->tv, h->d_deals, h->d_sched,
-                                                                           batch, rscale, h->d_counters, d_trace);
-    else
-      k_traverse_ref<kRefBlock, false><<<grid, kRefBlock, 0, h->stream>>>(h->gp, h->tv, h->d_deals, h->d_sched,
-                                                                            batch, rscale, h->d_counters, nullptr);
+    const int rc = enqueue_path(h, batch, rscale, d_trace);
+    if (rc) return rc;
   } else if (walk || use_levels(h)) {
     const int rc = walk ? enqueue_walk(h, batch, rscale) : enqueue_levels(h, batch, rscale);
     if (rc) return rc;
@@ -957,6 +954,24 @@ int ensure_levels(mccfr_handle* h, int batch);
 int ensure_form(mccfr_handle* h, int batch) {
   if (use_walk(h)) return ensure_walk(h, batch);
   return use_levels(h) ? ensure_levels(h, batch) : MCCFR_OK;
+}
+
+// The reference's rule: persistent lanes, as many as are resident or as the batch
+// has traversals for.
+int enqueue_path(mccfr_handle* h, int batch, float rscale, mccfr_trace* d_trace) {
+  if (!h->path_resident) {
+    int sms = 0, per = 0;
+    CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, h->device));
+    CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_path<true, false>, kPathBlock, 0));
+    h->path_resident = std::max(1, per) * sms;
+  }
+  const int blocks = std::min(h->path_resident, (batch + kPathBlock - 1) / kPathBlock);
+  auto kern = h->tv.direct ? (d_trace ? k_path<true, true> : k_path<true, false>)
+                           : (d_trace ? k_path<false, true> : k_path<false, false>);
+  kern<<<blocks, kPathBlock, 0, h->stream>>>(h->gp, h->tv, h->d_deals, h->d_sched, batch, rscale, h->d_counters,
+                                             h->d_work, d_trace);
+  CK(cudaGetLastError());
+  return MCCFR_OK;
 }
 
 int enqueue_walk(mccfr_handle* h, int batch, float rscale) {

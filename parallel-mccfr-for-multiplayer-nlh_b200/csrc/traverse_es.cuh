@@ -415,7 +415,7 @@ k_traverse_es(const GameParams G, const TableView tv, const DealRec* __restrict_
   warp_add_counters(counters, trav, c.visits, c.updates, c.terminals, trav * (unsigned)G.N);
 }
 
-// `work` must be zero when the launch starts; the launch enqueues that reset.
+// `work` must be zero when the launch starts (the deal before it zeroes it).
 // The two shallowest frames of each walk live in shared memory (measured best
 // among 0-4 staged frames and probe widths 1-2 on both presets).
 inline void launch_traverse_es(const GameParams& G, const TableView& tv, const DealRec* deals, const Sched* sched,
@@ -437,7 +437,6 @@ inline void launch_traverse_es(const GameParams& G, const TableView& tv, const D
   }
   const int resident_blocks = resident[d];
   const int grid = std::max(1, std::min(resident_blocks, (batch + B - 1) / B));
-  cudaMemsetAsync(work, 0, sizeof(unsigned), stream);
   k_traverse_es<B, K, 1><<<grid, B, smem, stream>>>(G, tv, deals, sched, batch, rscale, counters, work);
 }
 

@@ -1,24 +1,12 @@
-// traverse_ref.cuh — deal kernel and the traversal kernel of the reference's rule.
+// traverse_ref.cuh — deals, and what every traversal form shares.
 //
 // The reference runs one recursive traversal per thread, dealing and bucketing
-// at its start, with its game state in local memory (cfr_gpu.cu:644-1011).  Here:
-//   * k_deal deals every traversal of a player-update (counter-based Philox,
-//     the reference's partial Fisher-Yates) and computes its buckets and river
-//     ranks into a 64-byte record; the rank chains of all players share the
-//     3-card board prefix (the table's state depends only on the set of cards,
-//     which the tests check);
-//   * under the reference's rule every node samples one action, so a traversal
-//     is a single root-to-terminal path and every node on it returns the
-//     terminal payoff u (cfr_gpu.cu:809-818): k_traverse_ref walks the path
-//     iteratively, one thread per traversal, with per-player chip counts and
-//     buckets in shared memory (column-major [field][thread], conflict-free,
-//     indexable by player without local memory);
-//   * each node reads its regret row once (a 32-byte sector) from a snapshot
-//     that the update does not modify; the updating player's nodes are recorded
-//     in shared memory and, when u is known, folded into the row's fixed-point
-//     accumulators with three atomics (visit count, sum of u, sampled-action
-//     delta).
-// No dynamically indexed per-thread array stays alive across the walk.
+// at its start, with its game state in local memory (cfr_gpu.cu:644-1011).  Here
+// k_deal deals every traversal of a player-update (counter-based Philox, the
+// reference's partial Fisher-Yates) and computes its buckets and river ranks into a
+// 64-byte record, which the traversal kernels read; the rank chains of all players
+// share the 3-card board prefix (the table's state depends only on the set of
+// cards, which the tests check).
 #pragma once
 #include "game.cuh"
 #include "table.cuh"
@@ -59,8 +47,6 @@ static_assert(sizeof(DealRec) == 64, "deal record is one 64-byte pair of sectors
 struct Counters {
   unsigned long long traversals, visits, updates, terminals, evals;
 };
-
-constexpr int kMaxRec = 24;
 
 __device__ __forceinline__ void warp_add_counters(Counters* c, unsigned t, unsigned v, unsigned u,
                                                   unsigned x, unsigned e) {
@@ -386,241 +372,6 @@ __device__ __forceinline__ void load_regrets(const TableView& tv, long long slot
 #pragma unroll
     for (int a = 0; a < kSlots; ++a) reg[a] = 0.0f;
   }
-}
-
-template <int BLOCK, bool TRACE>
-__global__ void __launch_bounds__(BLOCK)
-k_traverse_ref(const GameParams G, const TableView tv, const DealRec* __restrict__ deals, const Sched* __restrict__ sched,
-               int batch, float rscale, Counters* __restrict__ counters, mccfr_trace* __restrict__ trace) {
-  __shared__ uint16_t s_stack[kMaxPlayers][BLOCK];
-  __shared__ uint16_t s_bet[kMaxPlayers][BLOCK];
-  __shared__ uint16_t s_inv[kMaxPlayers][BLOCK];
-  __shared__ uint16_t s_rank[kMaxPlayers][BLOCK];
-  __shared__ uint32_t s_ctx[kMaxPlayers][BLOCK];
-  // updating-player nodes of each thread's path: slot, sampled | mask << 8, q
-  __shared__ uint32_t s_rec_slot[kMaxRec][BLOCK];
-  __shared__ uint16_t s_rec_sv[kMaxRec][BLOCK];
-  __shared__ float s_rec_q[kMaxRec][BLOCK];
-
-  const int tid = threadIdx.x;
-  const uint32_t t = blockIdx.x * BLOCK + tid;
-  if (t >= (uint32_t)batch) return;
-  const int N = G.N;
-  const int up = sched->player;
-  const uint32_t uid = update_id(sched, N), epoch = *table_epoch(tv);
-
-  const DealRec& D = deals[t];
-  const int dealer = D.dealer;
-#pragma unroll
-  for (int p = 0; p < kMaxPlayers; ++p)
-    if (p < N) {
-      s_ctx[p][tid] = D.ctx[p];
-      s_rank[p][tid] = D.rank[p];
-      s_stack[p][tid] = (uint16_t)G.stack;
-      s_bet[p][tid] = 0;
-      s_inv[p][tid] = 0;
-    }
-
-  // Blinds and preflop queue (cfr_gpu.cu:954-981), or a subgame's start.
-  int pot, cb, lfr = G.bb, raises = 0, street = 0;
-  uint32_t folded = 0, allin = 0, abits = 0;
-  uint64_t path = kPathSeed;
-  uint32_t q = 0;  // action queue, 4-bit entries
-  int nq = 0;
-  if (G.sub_street) {
-#pragma unroll
-    for (int p = 0; p < kMaxPlayers; ++p)
-      if (p < N) s_inv[p][tid] = (uint16_t)(G.sub_pot / N);
-    pot = G.sub_pot;
-    cb = 0;
-    street = G.sub_street;
-    for (int i = 1; i <= N; ++i) q |= (uint32_t)seat_after(dealer, i, N) << (4 * nq++);
-  } else {
-    const int sbp = (N == 2) ? dealer : seat_after(dealer, 1, N);
-    const int bbp = (N == 2) ? seat_after(dealer, 1, N) : seat_after(seat_after(dealer, 1, N), 1, N);
-    const int sba = min(G.sb, G.stack), bba = min(G.bb, G.stack);
-    s_stack[sbp][tid] = (uint16_t)(G.stack - sba);
-    s_bet[sbp][tid] = (uint16_t)sba;
-    s_inv[sbp][tid] = (uint16_t)sba;
-    s_stack[bbp][tid] = (uint16_t)(G.stack - bba);
-    s_bet[bbp][tid] = (uint16_t)bba;
-    s_inv[bbp][tid] = (uint16_t)bba;
-    pot = sba + bba;
-    cb = bba;
-    if (G.stack - sba == 0) allin |= 1u << sbp;
-    if (G.stack - bba == 0) allin |= 1u << bbp;
-    for (int i = 0; i < N; ++i) {
-      const int p = seat_after(seat_after(bbp, 1, N), i, N);
-      if (!((allin >> p) & 1)) q |= (uint32_t)p << (4 * nq++);
-    }
-  }
-
-  int nrec = 0;
-  unsigned n_visits = 0, n_updates = 0;
-  int n_act = 0;
-  float u = 0.0f;
-  int depth = 0;
-  const uint32_t all_players = (1u << N) - 1;
-  for (;;) {
-    if (depth >= G.max_depth) {
-      u = 0.0f;
-      break;
-    }
-    const uint32_t live = all_players & ~folded;
-    if (__popc(live) == 1) {
-      const int winner = __ffs(live) - 1;
-      u = (winner == up) ? (float)(pot - (int)s_inv[up][tid]) : (float)(-(int)s_inv[up][tid]);
-      break;
-    }
-    if (nq == 0) {
-      bool showdown_now = true;
-      if (street < 3) {
-        street++;
-#pragma unroll
-        for (int p = 0; p < kMaxPlayers; ++p)
-          if (p < N) s_bet[p][tid] = 0;
-        cb = 0;
-        lfr = G.bb;
-        raises = 0;
-        q = 0;
-        nq = 0;
-        for (int i = 1; i <= N; ++i) {
-          const int p = seat_after(dealer, i, N);
-          if (!((folded >> p) & 1) && !((allin >> p) & 1)) q |= (uint32_t)p << (4 * nq++);
-        }
-        if (nq > 0) {
-          depth++;
-          showdown_now = false;
-        }
-      }
-      if (showdown_now) {
-        u = side_pot_payoff(
-            N, up, folded, [&](int x) { return (int)s_inv[x][tid]; }, [&](int x) { return (uint32_t)s_rank[x][tid]; });
-        break;
-      }
-      continue;
-    }
-    // Decision node.
-    const int player = (int)(q & 0xF);
-    const int pstack = s_stack[player][tid];
-    const int pbet = s_bet[player][tid];
-    const int to_call = cb - pbet;
-    const uint32_t vm = valid_mask(G, pot, pstack, to_call, cb, lfr, raises);
-    const uint32_t cw = s_ctx[player][tid];
-    uint32_t hb, bkt;
-    if (G.sub_street) {  // exact combo; the river card once it is dealt
-      hb = cw & 0xFFFF;
-      bkt = (street == 3 && G.sub_street == 2) ? (cw >> 16) : 0u;
-    } else {
-      hb = cw & 0xFF;
-      bkt = street ? ((cw >> (8 * street)) & 0xFF) : 0u;
-    }
-    const unsigned long long key = info_key(G, player, hb, bkt, street, abits, path);
-    const bool is_up = (player == up);
-    const long long slot = is_up ? table_insert(tv, key) : table_find(tv, key);
-    float reg[kSlots];
-    load_regrets(tv, slot, reg);
-    n_visits++;
-    const U4 d = philox(U4{t, uid, (uint32_t)path, (uint32_t)(path >> 32) | 0x80000000u}, G.seed_lo, G.seed_hi);
-    const int s = sample_action(G, reg, vm, uniform01(d.x));
-    if (is_up) {
-      n_updates++;
-      if (nrec < kMaxRec && slot >= 0) {
-        float strat[kSlots];
-        node_strategy(reg, vm, strat);
-        s_rec_slot[nrec][tid] = (uint32_t)slot;
-        s_rec_sv[nrec][tid] = (uint16_t)((uint32_t)s | (vm << 8));
-        s_rec_q[nrec][tid] = fmaxf(strat[s], 0.05f);
-        nrec++;
-      } else if (slot >= 0) {
-        atomicOr(tv.err, kErrRecordOverflow);
-      }
-    }
-    if (TRACE) {
-      if (n_act < 40) trace[t].actions[n_act] = (uint8_t)s;
-    }
-    n_act++;
-    // pop the actor, apply (cfr_gpu.cu:803-807, 543-585)
-    q >>= 4;
-    nq--;
-    const int chips = chips_for(G, s, pot, pstack, to_call, cb, lfr);
-    abits = ((abits << 3) | (uint32_t)s) & 0x3FFFFFFFu;
-    path = path_step(path, s);
-    const int k = G.kind[s];
-    if (k == 0) {
-      folded |= 1u << player;
-    } else if (k != 1) {
-      const int nstack = pstack - chips, nbet = pbet + chips;
-      s_stack[player][tid] = (uint16_t)nstack;
-      s_bet[player][tid] = (uint16_t)nbet;
-      s_inv[player][tid] = (uint16_t)(s_inv[player][tid] + chips);
-      pot += chips;
-      if (nstack == 0) allin |= 1u << player;
-      if (nbet > cb) {
-        const int prev = cb;
-        const int rs = nbet - prev;
-        if (rs >= lfr || prev == 0) lfr = rs;
-        cb = nbet;
-        raises++;
-        q = 0;
-        nq = 0;
-        for (int i = 1; i < N; ++i) {
-          const int p = seat_after(player, i, N);
-          if (!((folded >> p) & 1) && !((allin >> p) & 1)) q |= (uint32_t)p << (4 * nq++);
-        }
-      }
-    }
-    depth++;
-  }
-
-  // Fold u into the recorded nodes' accumulators.
-  const long long fu = fix_r(u, rscale);
-  for (int i = 0; i < nrec; ++i) {
-    const uint32_t slot = s_rec_slot[i][tid];
-    const uint32_t sv = s_rec_sv[i][tid];
-    const int s = (int)(sv & 0xFF);
-    const uint32_t vm = sv >> 8;
-    const long long dsamp = fix_r(__fsub_rn(__fdiv_rn(u, s_rec_q[i][tid]), u), rscale);
-    mark_wide(tv, slot);
-    if (touch_row(tv, slot, epoch, vm)) {
-      atomicAdd(row_cnt(tv, slot), (1ull << 32) | 1ull);
-      atomicAdd(row_su(tv, slot), (unsigned long long)fu);
-      atomicAdd(row_da(tv, slot) + s, (unsigned long long)(dsamp + fu));
-    } else {
-      // Mask differs from the row's canonical one (an FNV slot shared by states
-      // with different legal actions): add every term directly.
-      atomicAdd(row_cnt(tv, slot), 1ull << 32);
-      float reg[kSlots], strat[kSlots];
-      load_regrets(tv, slot, reg);
-      node_strategy(reg, vm, strat);
-      long long dr[kSlots], dw[kSlots];
-#pragma unroll
-      for (int a = 0; a < kSlots; ++a) {
-        dr[a] = (a == s) ? dsamp : -fu;
-        dw[a] = fix_s(strat[a]);
-      }
-      add_direct(tv, slot, vm, dr, dw);
-    }
-  }
-  if (TRACE) {
-    mccfr_trace& tr = trace[t];
-    for (int i = 0; i < 12; ++i) tr.hole[i] = D.hole[i];
-    for (int i = 0; i < 5; ++i) tr.board[i] = D.board[i];
-    tr.dealer = (uint8_t)dealer;
-    tr.n_actions = (uint8_t)n_act;
-    tr.n_traverser_nodes = (uint8_t)nrec;
-    for (int p = 0; p < 6; ++p) {
-      const uint32_t cw = D.ctx[p];
-      tr.hole_bucket[p] = (uint8_t)(cw & 0xFF);
-      tr.board_bucket[p][0] = 0;
-      tr.board_bucket[p][1] = (uint8_t)(cw >> 8);
-      tr.board_bucket[p][2] = (uint8_t)(cw >> 16);
-      tr.board_bucket[p][3] = (uint8_t)(cw >> 24);
-    }
-    tr.payoff = u;
-    tr.reserved = 0;
-  }
-  warp_add_counters(counters, 1u, n_visits, n_updates, 1u, (unsigned)N);
 }
 
 }  // namespace mccfr

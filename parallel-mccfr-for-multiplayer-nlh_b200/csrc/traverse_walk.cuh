@@ -232,7 +232,8 @@ __device__ __forceinline__ float walk_showdown(int N, int up, uint32_t folded, u
   const uint2 k01 = __ldg(reinterpret_cast<const uint2*>(D->rank));
   const uint32_t k2 = __ldg(reinterpret_cast<const uint32_t*>(D->rank + 4));
   const int mine = seat16(inv0, inv1, inv2, up), rank = seat16(k01.x, k01.y, k2, up);
-  bool beaten = (folded >> up) & 1, contested = false;
+  // (no chips in: the pots leave the negative zero that they start from)
+  bool beaten = ((folded >> up) & 1) || mine == 0, contested = false;
   int take = 0;
 #pragma unroll
   for (int q = 0; q < kMaxPlayers; ++q) {
@@ -244,7 +245,7 @@ __device__ __forceinline__ float walk_showdown(int N, int up, uint32_t folded, u
     contested |= live && rq >= rank;
     beaten |= live && rq > rank && iq >= mine;
   }
-  if (beaten) return (float)(-mine);
+  if (beaten) return -(float)mine;
   if (!contested) return (float)(take - mine);
   return lv_showdown(N, up, folded, inv0, inv1, inv2, D);
 }
