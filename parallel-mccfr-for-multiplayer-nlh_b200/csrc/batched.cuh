@@ -17,6 +17,7 @@
 #pragma once
 #include "traverse_es.cuh"
 #include "traverse_ref.cuh"
+#include "traverse_walk.cuh"
 
 namespace mccfr {
 
@@ -33,6 +34,11 @@ struct TableDesc {
   float rscale;
   double rinv;
   int batch;  // traversals per player-update
+  // rounds (k_walk_round): the table's deals, traversals a warp takes at a time,
+  // most decisions of its updating player on a path
+  int grab;
+  unsigned long long off;
+  int decisions;
   int pad;
 };
 
@@ -188,6 +194,34 @@ k_traverse_batched(const __grid_constant__ PhaseParams P, const DealRec* __restr
     }
   }
   flush();
+}
+
+// One player-update of several tables in the walk form.  A warp starts at a table
+// of its own (spread over the tables), walks traversals of one table at a time, and
+// goes on to the next table when no traversal of this one is left to take, so a
+// table with large trees is finished by every warp.  The table's descriptor is
+// copied to shared memory, where the whole warp reads it.  `work`: traversals
+// handed out of each table.
+template <bool DIRECT, bool FNV>
+__global__ void __launch_bounds__(kWalkBlock, 6)
+k_walk_round(const TableDesc* __restrict__ tables, int n, const DealRec* __restrict__ deals,
+             WalkNode* __restrict__ nodes, unsigned* __restrict__ work) {
+  __shared__ WalkWarp s_warp[kWalkWarps];
+  __shared__ TableDesc s_table[kWalkWarps];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int id = blockIdx.x * kWalkWarps + warp;
+  TableDesc& D = s_table[warp];
+  walk_init(s_warp[warp]);
+  for (int k = 0; k < n; ++k) {
+    const int j = (id + k) % n;
+    if (ld_volatile(work + j) >= (unsigned)tables[j].batch) continue;  // none left to take
+    for (int i = lane; i < (int)(sizeof(TableDesc) / 4); i += 32)
+      reinterpret_cast<uint32_t*>(&D)[i] = __ldg(reinterpret_cast<const uint32_t*>(tables + j) + i);
+    __syncwarp();
+    walk_update<DIRECT, FNV>(D.G, D.tv, deals + D.off, D.sched->player, update_id(D.sched, D.G.N), *table_epoch(D.tv),
+                        D.batch, D.rscale, D.grab, D.decisions, work + j, D.counters, s_warp[warp],
+                        nodes + (size_t)id * kWalkNodes, nullptr, nullptr);
+  }
 }
 
 }  // namespace mccfr

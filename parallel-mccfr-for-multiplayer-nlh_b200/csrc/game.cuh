@@ -335,15 +335,20 @@ __host__ __device__ __forceinline__ uint32_t fnv_slot(uint32_t player, uint32_t 
   return h & ((1u << 26) - 1);
 }
 
-__host__ __device__ __forceinline__ uint64_t info_key(const GameParams& G, uint32_t player, uint32_t hb,
-                                             uint32_t bb, uint32_t street, uint32_t abits,
-                                             uint64_t path) {
-  if (G.key_mode == 0) return (uint64_t)fnv_slot(player, hb, bb, street, abits) + 1;
+__host__ __device__ __forceinline__ uint64_t id64_key(const GameParams& G, uint32_t player, uint32_t hb, uint32_t bb,
+                                                      uint32_t street, uint64_t path) {
   uint64_t k = path ^ ((uint64_t)player << 56) ^ ((uint64_t)hb << 44) ^ ((uint64_t)bb << 32) ^
                ((uint64_t)street << 28);
   k = mix64(k);
   if (G.key_bits > 0) return (k & ((1ull << G.key_bits) - 1)) + 1;
   return k ? k : 1;
+}
+
+__host__ __device__ __forceinline__ uint64_t info_key(const GameParams& G, uint32_t player, uint32_t hb,
+                                             uint32_t bb, uint32_t street, uint32_t abits,
+                                             uint64_t path) {
+  if (G.key_mode == 0) return (uint64_t)fnv_slot(player, hb, bb, street, abits) + 1;
+  return id64_key(G, player, hb, bb, street, path);
 }
 
 // Fixed-point conversions of one delta (bit-exact with the oracle).

@@ -14,7 +14,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
-#include <array>
+#include <atomic>
 #include <chrono>
 #include <cmath>
 #include <cstdarg>
@@ -223,10 +223,13 @@ __global__ void __launch_bounds__(kApplyBlock) k_apply(const GameParams G, const
              blockIdx.x == 0 && threadIdx.x == 0);
 }
 
-// Apply of every table in a phase: blockIdx.y selects the table.
+// Apply of every table in a phase: blockIdx.y selects the table, whose error flag
+// goes to errors[blockIdx.y] (may be null).
 __global__ void __launch_bounds__(kApplyBlock) k_apply_batched(const TableDesc* __restrict__ tables,
-                                                       const PhaseDesc* __restrict__ phase) {
+                                                               const PhaseDesc* __restrict__ phase,
+                                                               int* __restrict__ errors) {
   const TableDesc& D = tables[phase->table[blockIdx.y]];
+  if (errors && blockIdx.x == 0 && threadIdx.x == 0) errors[blockIdx.y] = *D.tv.err;
   apply_rows(D.G, D.tv, D.sched, D.rinv, (blockIdx.x * blockDim.x + threadIdx.x) >> 5,
              (gridDim.x * blockDim.x) >> 5, blockIdx.x == 0 && threadIdx.x == 0);
 }
@@ -628,6 +631,7 @@ struct mccfr_handle {
   void* d_scratch = nullptr;
   size_t scratch_bytes = 0;
   unsigned* d_spans = nullptr;
+  bool counted = false;  // among its device's live handles
   int sticky_err = 0;
   std::string last_error;
   size_t persist_prev = 0;
@@ -921,7 +925,7 @@ int ensure_walk(mccfr_handle* h, int batch) {
   if (!h->walk_resident) {
     int sms = 0, per = 0;
     CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, h->device));
-    CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_walk<true>, kWalkBlock, 0));
+    CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, (k_walk<true, false>), kWalkBlock, 0));
     h->walk_resident = std::max(1, per) * sms;
   }
   const int want = std::min(h->walk_resident, (batch + kWalkWarps - 1) / kWalkWarps);
@@ -962,12 +966,15 @@ int enqueue_path(mccfr_handle* h, int batch, float rscale, mccfr_trace* d_trace)
   if (!h->path_resident) {
     int sms = 0, per = 0;
     CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, h->device));
-    CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_path<true, false>, kPathBlock, 0));
+    CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, (k_path<true, false, false>), kPathBlock, 0));
     h->path_resident = std::max(1, per) * sms;
   }
   const int blocks = std::min(h->path_resident, (batch + kPathBlock - 1) / kPathBlock);
-  auto kern = h->tv.direct ? (d_trace ? k_path<true, true> : k_path<true, false>)
-                           : (d_trace ? k_path<false, true> : k_path<false, false>);
+  using Kernel = decltype(&k_path<true, false, false>);
+  static const Kernel kernels[2][2][2] = {  // direct map, FNV keys, traces
+      {{k_path<false, false, false>, k_path<false, false, true>}, {k_path<false, true, false>, k_path<false, true, true>}},
+      {{k_path<true, false, false>, k_path<true, false, true>}, {k_path<true, true, false>, k_path<true, true, true>}}};
+  const Kernel kern = kernels[h->tv.direct ? 1 : 0][h->cfg.key_mode == MCCFR_KEY_FNV26][d_trace ? 1 : 0];
   kern<<<blocks, kPathBlock, 0, h->stream>>>(h->gp, h->tv, h->d_deals, h->d_sched, batch, rscale, h->d_counters,
                                              h->d_work, d_trace);
   CK(cudaGetLastError());
@@ -982,7 +989,9 @@ int enqueue_walk(mccfr_handle* h, int batch, float rscale) {
   // a warp takes up to 32 roots at a time, fewer while that would leave other
   // warps of the launch without
   wb.grab = std::max(1, std::min(32, batch / (4 * blocks * kWalkWarps)));
-  auto kern = h->tv.direct ? k_walk<true> : k_walk<false>;
+  const bool fnv = h->cfg.key_mode == MCCFR_KEY_FNV26;
+  auto kern = h->tv.direct ? (fnv ? k_walk<true, true> : k_walk<true, false>)
+                           : (fnv ? k_walk<false, true> : k_walk<false, false>);
   kern<<<blocks, kWalkBlock, 0, h->stream>>>(h->gp, h->tv, h->d_deals, h->d_sched, batch, rscale, wb, h->d_counters);
   CK(cudaGetLastError());
   return MCCFR_OK;
@@ -1325,9 +1334,14 @@ int read_host_rows(mccfr_handle* h, std::vector<HostRow>& rows) {
   return MCCFR_OK;
 }
 
+// Live handles per device; the round buffers go with a device's last one.
+std::atomic<int> g_live[64];
+void free_round_buffers(int device);
+
 void release(mccfr_handle* h) {
   if (!h) return;
   if (h->device >= 0) cudaSetDevice(h->device);
+  if (h->counted && --g_live[h->device] == 0) free_round_buffers(h->device);
   if (h->graph) cudaGraphExecDestroy(h->graph);
   if (h->persist_set) {
     cudaCtxResetPersistingL2Cache();
@@ -1544,6 +1558,10 @@ int mccfr_create(const mccfr_config* cfg, mccfr_handle** out) {
   h->tv.mask = C - 1;
   h->tv.log2cap = cfg->table_log2;
   set_direct(h);
+  if (h->device < 64) {
+    h->counted = true;
+    ++g_live[h->device];
+  }
   *out = h;
   return MCCFR_OK;
 #undef CKC
@@ -2300,7 +2318,7 @@ int batch_enqueue_iteration(mccfr_batch* b, bool capturing) {
     kern<<<grid, t.block, smem, b->stream>>>(b->params[p], b->d_deals, b->d_work + p, t.grab, t.warp_sync);
     BCK(cudaGetLastError());
     BCK(rec(b->ev_ph[2 * p + 1]));
-    k_apply_batched<<<dim3(148 * 2, P.n), 256, 0, b->stream>>>(b->d_tables, b->d_phases + p);
+    k_apply_batched<<<dim3(148 * 2, P.n), kApplyBlock, 0, b->stream>>>(b->d_tables, b->d_phases + p, nullptr);
     BCK(cudaGetLastError());
     k_advance_batched<<<1, 64, 0, b->stream>>>(b->d_tables, b->d_phases + p);
     BCK(cudaGetLastError());
@@ -2632,20 +2650,55 @@ int mccfr_batch_get_stats(mccfr_batch* b, mccfr_batch_stats* out) {
 // ---------------------------------------------------------------------------
 namespace {
 
+// What a round uploads, in one copy: the tables' descriptors and schedules, the
+// item ranges, and zeroed work counters.
+struct RoundUpload {
+  TableDesc tables[kMaxBatchTables];
+  Sched sched[kMaxBatchTables];
+  PhaseDesc phase;
+  unsigned long long persistent_work;
+  unsigned work[kMaxBatchTables];
+};
+
+// One device's round buffers.  They are shared by every trainer of the device
+// (rounds take turns) and freed with the device's last handle.
 struct RoundCtx {
-  int device = -1;
   cudaStream_t stream = nullptr;
-  TableDesc* d_tables = nullptr;
-  PhaseDesc* d_phase = nullptr;
-  DealRec* d_deals = nullptr;
-  unsigned long long* d_work = nullptr;
-  size_t deals_cap = 0;
+  RoundUpload* h_up = nullptr;  // pinned
+  RoundUpload* d_up = nullptr;
   int* h_err = nullptr;  // pinned: the tables' error flags after a round
-  PhaseParams params;
+  int* d_err = nullptr;
+  DealRec* d_deals = nullptr;
+  size_t deals_cap = 0;
+  WalkNode* d_nodes = nullptr;  // walk form: node records of `blocks` blocks
+  int blocks = 0, resident = 0;
+  PhaseParams params;  // persistent form: descriptors by value
+
+  void free_all() {
+    if (stream) cudaStreamDestroy(stream);
+    cudaFreeHost(h_up);
+    cudaFree(d_up);
+    cudaFreeHost(h_err);
+    cudaFree(d_err);
+    cudaFree(d_deals);
+    cudaFree(d_nodes);
+    stream = nullptr;
+    h_up = d_up = nullptr;
+    h_err = d_err = nullptr;
+    d_deals = nullptr;
+    d_nodes = nullptr;
+    deals_cap = 0;
+    blocks = 0;
+  }
 };
 
 RoundCtx g_round[64];
 std::mutex g_round_mu;
+
+void free_round_buffers(int device) {
+  std::lock_guard<std::mutex> lock(g_round_mu);
+  if (g_live[device] == 0) g_round[device].free_all();
+}
 
 // Range CDF on the 2^31 scale: combos that use a board card weigh 0; the last
 // combo of positive weight ends at exactly 2^31.
@@ -2833,76 +2886,109 @@ int mccfr_batch_round(mccfr_handle* const* tables, int n, const int* traversals,
   BCK(cudaSetDevice(dev));
   if (!R.stream) {
     BCK(cudaStreamCreateWithFlags(&R.stream, cudaStreamNonBlocking));
-    BCK(cudaMalloc(&R.d_tables, kMaxBatchTables * sizeof(TableDesc)));
-    BCK(cudaMalloc(&R.d_phase, sizeof(PhaseDesc)));
-    BCK(cudaMalloc(&R.d_work, sizeof(unsigned long long)));
+    BCK(cudaMalloc(&R.d_up, sizeof(RoundUpload)));
+    BCK(cudaMallocHost(&R.h_up, sizeof(RoundUpload)));
+    BCK(cudaMalloc(&R.d_err, kMaxBatchTables * sizeof(int)));
     BCK(cudaMallocHost(&R.h_err, kMaxBatchTables * sizeof(int)));
-    R.device = dev;
   }
   unsigned long long total = 0;
   for (int i = 0; i < n; ++i) total += (unsigned long long)traversals[i];
   if (total > R.deals_cap) {
     cudaFree(R.d_deals);
     R.d_deals = nullptr;
+    R.deals_cap = 0;
     BCK(cudaMalloc(&R.d_deals, total * sizeof(DealRec)));
     R.deals_cap = total;
   }
-  std::vector<TableDesc> descs(n);
-  PhaseDesc P;
-  std::memset(&P, 0, sizeof(P));
-  PhaseParams& Q = R.params;
-  std::memset(&Q, 0, sizeof(Q));
+  // The walk form, unless the caller tunes the persistent depth-first kernel or a
+  // table's config asks for another form (or has longer paths than the walk takes).
+  bool walk = !tuning, direct = true, fnv = false;
+  bool full = false, sub = false;
+  for (int i = 0; i < n; ++i) {
+    walk = walk && use_walk(tables[i]);
+    direct = direct && tables[i]->tv.direct;
+    fnv = fnv || tables[i]->cfg.key_mode == MCCFR_KEY_FNV26;
+    (tables[i]->gp.sub_street ? sub : full) = true;
+  }
+  int blocks = 0;
+  if (walk) {
+    if (!R.resident) {
+      int per = 0, sms = 0;
+      BCK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+      BCK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, (k_walk_round<true, false>), kWalkBlock, 0));
+      R.resident = std::max(1, per) * sms;
+    }
+    blocks = (int)std::min<unsigned long long>(R.resident, (total + kWalkWarps - 1) / kWalkWarps);
+    if (blocks > R.blocks) {
+      cudaFree(R.d_nodes);
+      R.d_nodes = nullptr;
+      R.blocks = 0;
+      BCK(cudaMalloc(&R.d_nodes, (size_t)blocks * kWalkWarps * kWalkNodes * sizeof(WalkNode)));
+      R.blocks = blocks;
+    }
+  }
+  RoundUpload& U = *R.h_up;
+  PhaseDesc& P = U.phase;
   unsigned long long off = 0;
+  unsigned words = 1;
   for (int i = 0; i < n; ++i) {
     mccfr_handle* h = tables[i];
-    h->h_sched->iteration = h->iterations_done + 1;
-    h->h_sched->player = h->round_player;
-    h->h_sched->pad = 0;
-    BCK(cudaMemcpyAsync(h->d_sched, h->h_sched, sizeof(Sched), cudaMemcpyHostToDevice, R.stream));
-    TableDesc& d = descs[i];
-    std::memset(&d, 0, sizeof(d));
+    U.sched[i] = Sched{h->iterations_done + 1, h->round_player, 0};
+    TableDesc& d = U.tables[i];
     d.G = h->gp;
     d.tv = h->tv;
     d.pre = h->d_pre;
     d.cdf = h->d_cdf;
-    d.sched = h->d_sched;
+    d.sched = &R.d_up->sched[i];
     d.counters = h->d_counters;
     const int rb = regret_frac_bits(h->cfg, traversals[i]);
     d.rscale = std::ldexp(1.0f, rb);
     d.rinv = std::ldexp(1.0, -rb);
     d.batch = traversals[i];
+    d.off = off;
+    d.decisions = max_decisions(h);
+    d.grab = (int)std::max(1ll, std::min(32ll, (long long)traversals[i] * n / (4ll * std::max(1, blocks) * kWalkWarps)));
     P.table[i] = i;
     P.off[i] = off;
-    Q.off[i] = off;
-    Q.T[i] = d;
+    U.work[i] = 0;
+    words = std::max(words, h->tv.n_words);
     off += (unsigned long long)traversals[i];
   }
   P.n = n;
   P.off[n] = off;
-  Q.n = n;
-  Q.off[n] = off;
-  BCK(cudaMemcpyAsync(R.d_tables, descs.data(), n * sizeof(TableDesc), cudaMemcpyHostToDevice, R.stream));
-  BCK(cudaMemcpyAsync(R.d_phase, &P, sizeof(P), cudaMemcpyHostToDevice, R.stream));
-  BCK(cudaMemsetAsync(R.d_work, 0, sizeof(unsigned long long), R.stream));
-  bool full = false, sub = false;
-  for (int i = 0; i < n; ++i) (tables[i]->gp.sub_street ? sub : full) = true;
-  BCK(launch_deals(R.d_tables, R.d_phase, tables[0]->d_hr, R.d_deals, off, full, sub, R.stream));
-  BatchedKernel kern = pick_kernel(t);
-  const size_t smem = batched_smem(t);
-  BCK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  int per_sm = 0;
-  BCK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, t.block, smem));
-  int sms = 148;
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  const unsigned long long need_blocks = (off + t.block - 1) / t.block;
-  const int grid = (int)std::max<unsigned long long>(1, std::min<unsigned long long>(need_blocks, (unsigned long long)std::max(1, per_sm) * sms));
-  kern<<<grid, t.block, smem, R.stream>>>(Q, R.d_deals, R.d_work, t.grab, t.warp_sync);
+  U.persistent_work = 0;
+  BCK(cudaMemcpyAsync(R.d_up, R.h_up, sizeof(RoundUpload), cudaMemcpyHostToDevice, R.stream));
+  BCK(launch_deals(R.d_up->tables, &R.d_up->phase, tables[0]->d_hr, R.d_deals, off, full, sub, R.stream));
+  if (walk) {
+    // any mix of tables runs the general kernel; direct-mapped tables of path-hash
+    // keys, as subgames are, the one without probing and FNV slots
+    auto kern = direct && !fnv ? k_walk_round<true, false> : k_walk_round<false, true>;
+    kern<<<blocks, kWalkBlock, 0, R.stream>>>(R.d_up->tables, n, R.d_deals, R.d_nodes, R.d_up->work);
+    BCK(cudaGetLastError());
+  } else {
+    PhaseParams& Q = R.params;
+    Q.n = n;
+    for (int i = 0; i <= n; ++i) Q.off[i] = P.off[i];
+    for (int i = 0; i < n; ++i) Q.T[i] = U.tables[i];
+    BatchedKernel kern = pick_kernel(t);
+    const size_t smem = batched_smem(t);
+    BCK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    int per_sm = 0;
+    BCK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, t.block, smem));
+    int sms = 148;
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    const unsigned long long need = (off + t.block - 1) / t.block;
+    const int grid = (int)std::max<unsigned long long>(
+        1, std::min<unsigned long long>(need, (unsigned long long)std::max(1, per_sm) * sms));
+    kern<<<grid, t.block, smem, R.stream>>>(Q, R.d_deals, &R.d_up->persistent_work, t.grab, t.warp_sync);
+    BCK(cudaGetLastError());
+  }
+  // a warp of the apply kernel per four bitmap words of the largest table
+  const int ablocks = (int)std::min(148u, (words + 31) / 32);
+  k_apply_batched<<<dim3(std::max(1, ablocks), n), kApplyBlock, 0, R.stream>>>(R.d_up->tables, &R.d_up->phase, R.d_err);
   BCK(cudaGetLastError());
-  k_apply_batched<<<dim3(std::max(1, std::min(148 * 2, (int)((off * 8 + 255) / 256) + 1)), n), 256, 0, R.stream>>>(
-      R.d_tables, R.d_phase);
-  BCK(cudaGetLastError());
-  for (int i = 0; i < n; ++i)  // every table's error flag in one synchronisation
-    BCK(cudaMemcpyAsync(R.h_err + i, tables[i]->tv.err, sizeof(int), cudaMemcpyDeviceToHost, R.stream));
+  // every table's error flag in one copy
+  BCK(cudaMemcpyAsync(R.h_err, R.d_err, n * sizeof(int), cudaMemcpyDeviceToHost, R.stream));
   BCK(cudaStreamSynchronize(R.stream));
   int worst = MCCFR_OK;
   for (int i = 0; i < n; ++i) {

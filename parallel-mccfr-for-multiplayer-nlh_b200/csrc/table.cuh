@@ -203,6 +203,20 @@ __device__ __forceinline__ void st_sector(void* p, const Sector& s) {
   asm volatile("st.global.cg.v4.u64 [%0], {%1, %2, %3, %4};"
                :: "l"(__cvta_generic_to_global(p)), "l"(s.x), "l"(s.y), "l"(s.z), "l"(s.w) : "memory");
 }
+// The same through L1, for data that only this SM's warp reads back.
+__device__ __forceinline__ Sector ld_own_sector(const void* p) {
+  Sector s;
+  asm volatile("ld.global.v4.u64 {%0, %1, %2, %3}, [%4];"
+               : "=l"(s.x), "=l"(s.y), "=l"(s.z), "=l"(s.w) : "l"(__cvta_generic_to_global(p)) : "memory");
+  return s;
+}
+__device__ __forceinline__ void st_own_sector(void* p, const Sector& s) {
+  asm volatile("st.global.v4.u64 [%0], {%1, %2, %3, %4};"
+               :: "l"(__cvta_generic_to_global(p)), "l"(s.x), "l"(s.y), "l"(s.z), "l"(s.w) : "memory");
+}
+__device__ __forceinline__ unsigned long long two_words(uint32_t lo, uint32_t hi) {
+  return (unsigned long long)lo | (unsigned long long)hi << 32;
+}
 __device__ __forceinline__ float lo_float(unsigned long long v) { return __uint_as_float((unsigned)v); }
 __device__ __forceinline__ float hi_float(unsigned long long v) { return __uint_as_float((unsigned)(v >> 32)); }
 __device__ __forceinline__ unsigned long long two_floats(float lo, float hi) {

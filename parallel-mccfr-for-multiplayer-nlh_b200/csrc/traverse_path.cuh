@@ -52,7 +52,7 @@ __device__ __forceinline__ void path_fold(const TableView& tv, uint32_t epoch, f
   }
 }
 
-template <bool DIRECT, bool TRACE>
+template <bool DIRECT, bool FNV, bool TRACE>
 __global__ void __launch_bounds__(kPathBlock, 6)
 k_path(const GameParams G, const TableView tv, const DealRec* __restrict__ deals, const Sched* __restrict__ sched,
        int batch, float rscale, Counters* __restrict__ counters, unsigned* __restrict__ work,
@@ -97,7 +97,7 @@ k_path(const GameParams G, const TableView tv, const DealRec* __restrict__ deals
     }
     if (__any_sync(0xFFFFFFFFu, st == kApply)) {
       if (st == kApply) {
-        if (pl >= 0) walk_apply(G, s, pl, pa);
+        if (pl >= 0) walk_apply<FNV>(G, s, pl, pa);
         const int r = walk_events(G, s, up, u);
         st = kFold;
         show = r == kLvShow;
@@ -158,7 +158,8 @@ k_path(const GameParams G, const TableView tv, const DealRec* __restrict__ deals
         hb = cw & 0xFF;
         bkt = street ? ((cw >> (8 * street)) & 0xFF) : 0u;
       }
-      const unsigned long long key = info_key(G, pl, hb, bkt, street, s.abits, s.path);
+      const unsigned long long key = FNV ? info_key(G, pl, hb, bkt, street, s.abits, s.path)
+                                         : id64_key(G, pl, hb, bkt, street, s.path);
       // an opponent's missing row reads as no regrets (in a direct map its stored
       // strategy is zero until training writes it); the updating player's is inserted
       const long long slot = DIRECT ? (long long)(key - 1) : isup ? table_insert(tv, key) : table_find(tv, key);

@@ -47,7 +47,7 @@ constexpr int kWalkWarps = kWalkBlock / 32;
 constexpr int kWalkNodes = 192;                  // open updating-player nodes of a warp
 constexpr int kWalkSeeds = kSlots * kWalkNodes;  // their children not yet taken
 constexpr int kWalkQueue = 64;                   // queue entries: 31 left over + 32 of one step
-constexpr int kWalkReady = 28;                   // lanes at a decision that end the filling of a step
+constexpr int kWalkReady = 24;                   // lanes at a decision that end the filling of a step
 constexpr uint32_t kWalkRoot = 0xFFFFu;          // parent of a traversal's root
 
 // Counters of one update, zeroed by the deal that precedes the walk.
@@ -73,15 +73,11 @@ struct WalkState {
 
 // An open updating-player node: its state, row, own seed, and children's values.
 struct __align__(128) WalkNode {
-  uint4 s0;  // inv0, inv1, inv2, bet0
-  uint4 s1;  // bet1, bet2, pot, cb
-  uint4 s2;  // path, lfr, abits
-  uint4 s3;  // aux, seats, prog, row slot
-  uint4 own; // parent record << 3 | action (its own seed), legal mask
-  float v[kSlots];
-  uint4 pad;
+  Sector a;   // inv0, inv1 | inv2, bet0 | bet1, bet2 | pot, cb
+  Sector b;   // path | lfr, abits | aux, seats | prog, row slot
+  Sector v;   // children's values, by action
+  uint2 own;  // parent record << 3 | action (its own seed), legal mask
 };
-static_assert(kMaxLevels == 32, "one lane per level");
 static_assert(sizeof(WalkNode) == 128, "a node record is one line");
 
 struct WalkShowdown {
@@ -96,7 +92,7 @@ struct WalkWarp {
   uint32_t out[kWalkNodes / 8];        // children still out, 4 bits per record
   WalkShowdown show[kWalkQueue];
   uint2 off[kWalkQueue];               // row slot, legal mask
-  unsigned roots;                      // traversals this warp took
+  unsigned roots, full;                // traversals taken, updating-player nodes that found no row
 };
 
 struct WalkBufs {
@@ -165,12 +161,14 @@ __device__ __forceinline__ int walk_next(uint32_t seats, int N) {
   return seat_after(from, __ffs((int)((mask | (mask << N)) >> from)) - 1, N);
 }
 
-// Applies action a of `player` (es_apply).
+// Applies action a of `player` (es_apply).  FNV: the game's keys may be FNV slots,
+// which hash the last ten actions; the walk of path-hash keys carries no abits.
+template <bool FNV>
 __device__ __forceinline__ void walk_apply(const GameParams& G, WalkState& s, int player, int a) {
   const int N = G.N;
   const uint32_t bit = 1u << player;
   const int after = seat_after(player, 1, N);
-  s.abits = ((s.abits << 3) | (uint32_t)a) & 0x3FFFFFFFu;
+  if (FNV) s.abits = ((s.abits << 3) | (uint32_t)a) & 0x3FFFFFFFu;
   s.path = path_step(s.path, a);
   s.prog += 1u << 16;  // depth
   uint32_t folded = s.seats & 0xFFu, allin = (s.seats >> 8) & 0xFFu, act = ((s.seats >> 16) & 0xFFu) & ~bit;
@@ -250,29 +248,28 @@ __device__ __forceinline__ float walk_showdown(int N, int up, uint32_t folded, u
   return lv_showdown(N, up, folded, inv0, inv1, inv2, D);
 }
 
-template <bool DIRECT>
-__global__ void __launch_bounds__(kWalkBlock, 6)
-k_walk(const GameParams G, const TableView tv, const DealRec* __restrict__ deals, const Sched* __restrict__ sched,
-       int batch, float rscale, const WalkBufs wb, Counters* __restrict__ counters) {
-  __shared__ WalkWarp s_warp[kWalkWarps];
-  __shared__ uint32_t s_nodes[kMaxLevels], s_seeds[kMaxLevels];
+// A warp's lists as walk_update expects and leaves them.
+__device__ __forceinline__ void walk_init(WalkWarp& W) {
   const int lane = threadIdx.x & 31;
-  const unsigned below = (1u << lane) - 1u;
-  WalkWarp& W = s_warp[threadIdx.x >> 5];
-  WalkNode* const pool = wb.nodes + (size_t)(blockIdx.x * kWalkWarps + (threadIdx.x >> 5)) * kWalkNodes;
-  __shared__ unsigned s_full;  // updating-player nodes that found no row
-  if (threadIdx.x < kMaxLevels) s_nodes[threadIdx.x] = s_seeds[threadIdx.x] = 0;
-  if (threadIdx.x == 0) s_full = 0;
   for (int i = lane; i < kWalkNodes; i += 32) W.spare[i] = (uint16_t)(kWalkNodes - 1 - i);
   for (int i = lane; i < kWalkNodes / 8; i += 32) W.out[i] = 0;
-  if (lane == 0) W.roots = 0;
-  __syncthreads();
+  if (lane == 0) W.roots = W.full = 0;
+  __syncwarp();
+}
+
+// The walk of one table's update by one warp, until no traversal is left to take
+// and all that it took are done.  `levels` (may be null): the block's level counts.
+template <bool DIRECT, bool FNV>
+__device__ __forceinline__ void walk_update(const GameParams& G, const TableView& tv, const DealRec* __restrict__ deals,
+                                            int up, uint32_t uid, uint32_t epoch, int batch, float rscale, int grab,
+                                            int decisions, unsigned* work, Counters* counters, WalkWarp& W,
+                                            WalkNode* const pool, uint32_t* s_nodes, uint32_t* s_seeds) {
+  const int lane = threadIdx.x & 31;
+  const unsigned below = (1u << lane) - 1u;
   const int N = G.N;
-  const int up = sched->player;
-  const uint32_t uid = update_id(sched, N), epoch = *table_epoch(tv);
   // warp-uniform list lengths and counters
   int n_seeds = 0, n_spare = kWalkNodes, n_ready = 0, n_show = 0, n_off = 0;
-  unsigned c_vis = 0;
+  unsigned c_vis = 0, c_nodes = 0, c_kids = 0;
   bool more = true;  // roots may be left
   int stalled = 0;
   // the lane's walk: idle, an action to apply, or standing at a decision
@@ -286,7 +283,7 @@ k_walk(const GameParams G, const TableView tv, const DealRec* __restrict__ deals
   // Hands lane values to their parents (ref), listing nodes whose last child it was.
   auto deliver = [&](bool on, float v) {
     const bool has = on && ref != kWalkRoot;
-    if (has) pool[ref >> 3].v[ref & 7] = v;
+    if (has) reinterpret_cast<float*>(&pool[ref >> 3].v)[ref & 7] = v;
     __syncwarp();
     bool last = false;
     if (has) {
@@ -305,7 +302,7 @@ k_walk(const GameParams G, const TableView tv, const DealRec* __restrict__ deals
     const bool starved = n_idle == 32 && n_seeds == 0 && !more;
     // seeds the pool has room for: every walking lane may still open one node,
     // and one seed walked depth first opens one per decision
-    const int room = n_spare - (32 - n_idle) - wb.decisions;
+    const int room = n_spare - (32 - n_idle) - decisions;
     const bool low = room < 1;
 
     if (n_show >= 32 || (n_show && (starved || low))) {
@@ -335,15 +332,15 @@ k_walk(const GameParams G, const TableView tv, const DealRec* __restrict__ deals
       if (on) {
         id = W.ready[n_ready + lane];
         const WalkNode* nd = pool + id;
-        const unsigned long long slot = nd->s3.w;
-        const uint4 own = nd->own;
+        const unsigned long long slot = nd->b.w >> 32;
+        const uint2 own = nd->own;
         const uint32_t vm = own.y;
         const unsigned long long k = __ldcg(row_key(tv, slot));
         float reg[kSlots], strat[kSlots], v[kSlots];
         load_regrets(tv, (long long)slot, reg);
-        const float4 v0 = *reinterpret_cast<const float4*>(nd->v), v1 = *reinterpret_cast<const float4*>(nd->v + 4);
-        v[0] = v0.x; v[1] = v0.y; v[2] = v0.z; v[3] = v0.w;
-        v[4] = v1.x; v[5] = v1.y; v[6] = v1.z; v[7] = v1.w;
+        const Sector cv = ld_own_sector(&nd->v);
+        v[0] = lo_float(cv.x); v[1] = hi_float(cv.x); v[2] = lo_float(cv.y); v[3] = hi_float(cv.y);
+        v[4] = lo_float(cv.z); v[5] = hi_float(cv.z); v[6] = lo_float(cv.w); v[7] = hi_float(cv.w);
         // a direct-mapped row's key was left to this pass
         if (DIRECT && k != slot + 1) __stcg(row_key(tv, slot), slot + 1);
         mark_wide(tv, slot);
@@ -399,12 +396,13 @@ k_walk(const GameParams G, const TableView tv, const DealRec* __restrict__ deals
         if (st == kIdle && rank < take) {
           ref = W.seeds[n_seeds + take - 1 - rank];
           const WalkNode* nd = pool + (ref >> 3);
-          const uint4 a = nd->s0, b = nd->s1, c = nd->s2, d = nd->s3;
-          s.inv0 = a.x; s.inv1 = a.y; s.inv2 = a.z; s.bet0 = a.w;
-          s.bet1 = b.x; s.bet2 = b.y; s.pot = (int)b.z; s.cb = (int)b.w;
-          s.path = (uint64_t)c.x | ((uint64_t)c.y << 32);
-          s.lfr = (int)c.z; s.abits = c.w;
-          s.aux = d.x; s.seats = d.y; s.prog = d.z;
+          const Sector a = ld_own_sector(&nd->a), b = ld_own_sector(&nd->b);
+          s.inv0 = (uint32_t)a.x; s.inv1 = (uint32_t)(a.x >> 32); s.inv2 = (uint32_t)a.y; s.bet0 = (uint32_t)(a.y >> 32);
+          s.bet1 = (uint32_t)a.z; s.bet2 = (uint32_t)(a.z >> 32); s.pot = (int)(uint32_t)a.w; s.cb = (int)(a.w >> 32);
+          s.path = b.x;
+          s.lfr = (int)(uint32_t)b.y;
+          if (FNV) s.abits = (uint32_t)(b.y >> 32);
+          s.aux = (uint32_t)b.z; s.seats = (uint32_t)(b.z >> 32); s.prog = (uint32_t)b.w;
           s.prog += 1u << 24;  // one level down
           pl = up;
           pa = (int)(ref & 7u);
@@ -412,9 +410,9 @@ k_walk(const GameParams G, const TableView tv, const DealRec* __restrict__ deals
         }
         filled = true;
       } else if (n_seeds == 0 && more && allowed > 0) {
-        const int want = min(min(n_idle, allowed), wb.grab);
+        const int want = min(min(n_idle, allowed), grab);
         unsigned base = 0;
-        if (lane == 0) base = atomicAdd(&wb.ctl->work, (unsigned)want);
+        if (lane == 0) base = atomicAdd(work, (unsigned)want);
         base = __shfl_sync(0xFFFFFFFFu, base, 0);
         const int got = base < (unsigned)batch ? min(want, (int)((unsigned)batch - base)) : 0;
         if (got < want) more = false;
@@ -435,7 +433,7 @@ k_walk(const GameParams G, const TableView tv, const DealRec* __restrict__ deals
       int r = -1;
       float v = 0.0f;
       if (st == kApply) {
-        if (pl >= 0) walk_apply(G, s, pl, pa);
+        if (pl >= 0) walk_apply<FNV>(G, s, pl, pa);
         r = walk_events(G, s, up, v);
         st = kIdle;
         if (r == kLvGoOn) {
@@ -490,25 +488,23 @@ k_walk(const GameParams G, const TableView tv, const DealRec* __restrict__ deals
         hb = cw & 0xFF;
         bkt = street ? ((cw >> (8 * street)) & 0xFF) : 0u;
       }
-      const unsigned long long key = info_key(G, player, hb, bkt, street, s.abits, s.path);
+      const unsigned long long key = FNV ? info_key(G, player, hb, bkt, street, s.abits, s.path)
+                                         : id64_key(G, player, hb, bkt, street, s.path);
       isup = player == up;
       // in a direct-mapped table the updating player's row is left to the ready pass
       slot = DIRECT ? (long long)(key - 1) : table_insert<1>(tv, key);
       if (!isup) {
         const bool ok = DIRECT || slot >= 0;
-        ulonglong2 head = make_ulonglong2(0ull, 0ull);
-        uint4 sg = make_uint4(0u, 0u, 0u, 0u);
-        if (ok) {
-          head = __ldcg(row_head(tv, (unsigned long long)slot));
-          sg = __ldcg(row_strat(tv, (unsigned long long)slot));
-        }
+        Sector row{0ull, 0ull, 0ull, 0ull};  // key, tag, strategy
+        if (ok) row = ld_sector(row_ptr(tv, (unsigned long long)slot));
         const U4 d = philox(U4{s.aux, uid, (uint32_t)s.path, (uint32_t)(s.path >> 32) | 0x80000000u}, G.seed_lo,
                             G.seed_hi);
-        if (DIRECT && head.x != key) __stcg(row_key(tv, (unsigned long long)slot), key);
-        pa = sample_stored(G, sg, vm, uniform01(d.x));
+        if (DIRECT && row.x != key) __stcg(row_key(tv, (unsigned long long)slot), key);
+        pa = sample_stored(G, make_uint4((uint32_t)row.z, (uint32_t)(row.z >> 32), (uint32_t)row.w,
+                                         (uint32_t)(row.w >> 32)), vm, uniform01(d.x));
         st = kApply;
         if (ok) {
-          if (touch_row_from(tv, (unsigned long long)slot, epoch, vm, head.y))
+          if (touch_row_from(tv, (unsigned long long)slot, epoch, vm, row.y))
             atomicAdd(row_cnt(tv, (unsigned long long)slot), (1ull << 32) | 1ull);
           else
             off = true;
@@ -538,7 +534,9 @@ k_walk(const GameParams G, const TableView tv, const DealRec* __restrict__ deals
       }
       const int cnt = __popc(upm);
       // the lanes go on with their node's first action while the pool is far from full
-      const bool go_on = n_spare - cnt - 32 >= wb.decisions;
+      const bool go_on = n_spare - cnt - 32 >= decisions;
+      c_nodes += cnt;
+      c_kids += total;
       if (go_on) {
         before -= __popc(upm & below);
         total -= cnt;
@@ -546,19 +544,21 @@ k_walk(const GameParams G, const TableView tv, const DealRec* __restrict__ deals
       if (open) {
         const uint32_t id = W.spare[n_spare - 1 - __popc(upm & below)];
         WalkNode* nd = pool + id;
-        nd->s0 = make_uint4(s.inv0, s.inv1, s.inv2, s.bet0);
-        nd->s1 = make_uint4(s.bet1, s.bet2, (uint32_t)s.pot, (uint32_t)s.cb);
-        nd->s2 = make_uint4((uint32_t)s.path, (uint32_t)(s.path >> 32), (uint32_t)s.lfr, s.abits);
-        nd->s3 = make_uint4(s.aux, s.seats, s.prog, (uint32_t)slot);
-        nd->own = make_uint4(ref, vm, 0u, 0u);
+        st_own_sector(&nd->a, Sector{two_words(s.inv0, s.inv1), two_words(s.inv2, s.bet0), two_words(s.bet1, s.bet2),
+                                     two_words((uint32_t)s.pot, (uint32_t)s.cb)});
+        st_own_sector(&nd->b, Sector{s.path, two_words((uint32_t)s.lfr, FNV ? s.abits : 0u), two_words(s.aux, s.seats),
+                                     two_words(s.prog, (uint32_t)slot)});
+        nd->own = make_uint2(ref, vm);
         atomicAdd(&W.out[id >> 3], (unsigned)k << (4u * (id & 7u)));
         int o = n_seeds + before;
         uint32_t left = vm;
         if (go_on) left &= left - 1;
         for (; left; left &= left - 1) W.seeds[o++] = (uint16_t)((id << 3) | (uint32_t)(__ffs(left) - 1));
-        const int level = (int)(s.prog >> 24);
-        atomicAdd(&s_nodes[level], 1u);
-        atomicAdd(&s_seeds[level], (unsigned)k);
+        if (s_nodes) {
+          const int level = (int)(s.prog >> 24);
+          atomicAdd(&s_nodes[level], 1u);
+          atomicAdd(&s_seeds[level], (unsigned)k);
+        }
         if (go_on) {
           pa = __ffs((int)vm) - 1;
           ref = (id << 3) | (uint32_t)pa;
@@ -570,7 +570,7 @@ k_walk(const GameParams G, const TableView tv, const DealRec* __restrict__ deals
       __syncwarp();
       if (full) {
         deliver(isup && slot < 0, 0.0f);
-        if (lane == 0) atomicAdd(&s_full, (unsigned)__popc(full));
+        if (lane == 0) W.full += __popc(full);
       }
       if (isup) st = open && go_on ? kApply : kIdle;
     }
@@ -579,21 +579,33 @@ k_walk(const GameParams G, const TableView tv, const DealRec* __restrict__ deals
     if (W.roots) {
       atomicAdd(&counters->traversals, (unsigned long long)W.roots);
       atomicAdd(&counters->evals, (unsigned long long)W.roots * (unsigned)N);
+      atomicAdd(&counters->visits, (unsigned long long)c_vis);
+      // every root and seed ended at a terminal, an updating-player node, or a node
+      // that found no row
+      atomicAdd(&counters->terminals, (unsigned long long)W.roots + c_kids - c_nodes - W.full);
+      if (c_nodes) atomicAdd(&counters->updates, (unsigned long long)c_nodes);
     }
-    if (c_vis) atomicAdd(&counters->visits, (unsigned long long)c_vis);
+    W.roots = W.full = 0;
   }
+  __syncwarp();
+  if (stalled > 8) walk_init(W);  // given up with the error flag set: nothing of this table is left in the lists
+}
+
+template <bool DIRECT, bool FNV>
+__global__ void __launch_bounds__(kWalkBlock, 6)
+k_walk(const GameParams G, const TableView tv, const DealRec* __restrict__ deals, const Sched* __restrict__ sched,
+       int batch, float rscale, const WalkBufs wb, Counters* __restrict__ counters) {
+  __shared__ WalkWarp s_warp[kWalkWarps];
+  __shared__ uint32_t s_nodes[kMaxLevels], s_seeds[kMaxLevels];
+  const int warp = threadIdx.x >> 5;
+  if (threadIdx.x < kMaxLevels) s_nodes[threadIdx.x] = s_seeds[threadIdx.x] = 0;
+  walk_init(s_warp[warp]);
   __syncthreads();
-  if (threadIdx.x < 32) {
-    // every root and seed ended at a terminal, an updating-player node, or a node
-    // that found no row
-    const unsigned nodes = __reduce_add_sync(0xFFFFFFFFu, s_nodes[threadIdx.x]);
-    const unsigned seeds = __reduce_add_sync(0xFFFFFFFFu, s_seeds[threadIdx.x]);
-    const unsigned ends = (threadIdx.x < kWalkWarps ? s_warp[threadIdx.x].roots : 0u);
-    const unsigned roots = __reduce_add_sync(0xFFFFFFFFu, ends);
-    if (threadIdx.x == 0 && roots) {
-      atomicAdd(&counters->updates, (unsigned long long)nodes);
-      atomicAdd(&counters->terminals, (unsigned long long)roots + seeds - nodes - s_full);
-    }
+  walk_update<DIRECT, FNV>(G, tv, deals, sched->player, update_id(sched, G.N), *table_epoch(tv), batch, rscale, wb.grab,
+                      wb.decisions, &wb.ctl->work, counters, s_warp[warp],
+                      wb.nodes + (size_t)(blockIdx.x * kWalkWarps + warp) * kWalkNodes, s_nodes, s_seeds);
+  __syncthreads();
+  if (threadIdx.x < kMaxLevels) {
     if (s_nodes[threadIdx.x]) atomicAdd(&wb.ctl->nodes[threadIdx.x], s_nodes[threadIdx.x]);
     if (s_seeds[threadIdx.x]) atomicAdd(&wb.ctl->seeds[threadIdx.x], s_seeds[threadIdx.x]);
   }

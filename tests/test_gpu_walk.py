@@ -109,3 +109,38 @@ def test_imported_regrets_are_sampled(hand_table):
     a.close()
     b.close()
     orc.close()
+
+
+@pytest.mark.parametrize("mixed", [False, True], ids=["path-hash-direct", "any-mix"])
+@pytest.mark.parametrize("tuning", [None, {"block": 64, "grab": 2}], ids=["walk", "persistent"])
+def test_rounds_of_uneven_tables_equal_plain(hand_table, mixed, tuning):
+    """Rounds over tables of different games and sizes (with a probed table and a
+    table of FNV slots among them: the general kernel), by the walk and by a tuned
+    persistent kernel: every table equals the same updates trained alone."""
+    cfgs = [_six(16), _hu_cap(2), _thirds()]
+    if mixed:
+        ref = L.preset(L.PRESET_REF8)
+        ref.sampling, ref.max_depth, ref.table_log2 = L.SAMPLING_EXTERNAL, 9, 22
+        cfgs += [_hu_probed(), ref]
+    counts = [50, 1, 700, 33, 20][:len(cfgs)]
+
+    def make():
+        ts = []
+        for c in cfgs:
+            t = mccfr.GPUCFRTrainer(config=c)
+            t.set_hand_table(hand_table)
+            ts.append(t)
+        return ts
+    rounds, plain = make(), make()
+    for _ in range(7):
+        mccfr.batch_round(rounds, counts, tuning)
+    for t, c, n in zip(plain, cfgs, counts):
+        for u in range(7):
+            t.step(1 + u // c.num_players, u % c.num_players, n)
+    for a, b in zip(rounds, plain):
+        assert a.digest() == b.digest()
+        sa, sb = a.stats(), b.stats()
+        assert (sa.traversals, sa.node_visits, sa.traverser_updates, sa.terminals) == (
+            sb.traversals, sb.node_visits, sb.traverser_updates, sb.terminals)
+    for t in rounds + plain:
+        t.close()
