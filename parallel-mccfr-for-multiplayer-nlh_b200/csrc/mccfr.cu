@@ -217,10 +217,41 @@ __device__ __forceinline__ void apply_rows(const GameParams& G, const TableView&
   }
 }
 
+// What ends an update inside training: the schedule moves on, and when the next
+// player's deal lies ready already (`ahead`: the iteration's first deal dealt for
+// every player), its update is begun as a deal would begin it.  Done by the last
+// block of the apply kernel, when no block reads the schedule or the epoch any more.
+struct Advance {
+  Sched* sched;  // null: the update stands alone
+  uint32_t* ctl;
+  int ctl_words;
+  int ahead;
+};
+
 __global__ void __launch_bounds__(kApplyBlock) k_apply(const GameParams G, const TableView tv,
-                                               const Sched* __restrict__ sched, double rinv) {
+                                                       const Sched* __restrict__ sched, double rinv,
+                                                       const Advance adv) {
   apply_rows(G, tv, sched, rinv, (blockIdx.x * blockDim.x + threadIdx.x) >> 5, (gridDim.x * blockDim.x) >> 5,
              blockIdx.x == 0 && threadIdx.x == 0);
+  if (!adv.sched) return;
+  __shared__ bool s_last;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    __threadfence();
+    s_last = atomicAdd(apply_ticket(tv), 1u) == gridDim.x - 1;
+  }
+  __syncthreads();
+  if (!s_last) return;
+  const int p = adv.sched->player + 1 < G.N ? adv.sched->player + 1 : 0;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    *apply_ticket(tv) = 0;
+    adv.sched->player = p;
+    if (p == 0) adv.sched->iteration += 1;
+    else if (adv.ahead) *table_epoch(tv) += 1;
+  }
+  if (adv.ahead && p)
+    for (int i = threadIdx.x; i < adv.ctl_words; i += kApplyBlock) adv.ctl[i] = 0;
 }
 
 // Apply of every table in a phase: blockIdx.y selects the table, whose error flag
@@ -232,15 +263,6 @@ __global__ void __launch_bounds__(kApplyBlock) k_apply_batched(const TableDesc* 
   if (errors && blockIdx.x == 0 && threadIdx.x == 0) errors[blockIdx.y] = *D.tv.err;
   apply_rows(D.G, D.tv, D.sched, D.rinv, (blockIdx.x * blockDim.x + threadIdx.x) >> 5,
              (gridDim.x * blockDim.x) >> 5, blockIdx.x == 0 && threadIdx.x == 0);
-}
-
-__global__ void k_advance(Sched* s, int N) {
-  int p = s->player + 1;
-  if (p >= N) {
-    p = 0;
-    s->iteration += 1;
-  }
-  s->player = p;
 }
 
 __global__ void k_advance_batched(const TableDesc* __restrict__ tables, const PhaseDesc* __restrict__ phase) {
@@ -597,7 +619,7 @@ struct mccfr_handle {
   size_t block_bytes = 0;
   Sched* d_sched = nullptr;
   DealRec* d_deals = nullptr;  // one record per traversal of an update
-  int deals_cap = 0;
+  long long deals_cap = 0;
   uint32_t* d_ranges = nullptr;  // subgame range CDFs [N][1326]
   bool shared_hr = false;        // d_hr borrowed from another handle
   int round_player = 0;          // next player of round-by-round training
@@ -621,6 +643,9 @@ struct mccfr_handle {
   // graph of one iteration
   cudaGraphExec_t graph = nullptr;
   int graph_batch = -1;
+  bool graph_timed = false;
+  long long direct_iters = 0;    // iterations enqueued without a graph since it was dropped
+  unsigned long long generation = 0;  // of the buffers and parameters that graphs hold
   long long iterations_done = 0;
   long long launches = 0;
   double traverse_ms = 0, apply_ms = 0, last_traverse_ms = 0, last_apply_ms = 0;
@@ -844,46 +869,85 @@ cudaError_t launch_deals(const TableDesc* d_tables, const PhaseDesc* d_phase, co
 
 bool use_walk(const mccfr_handle* h);
 bool use_levels(const mccfr_handle* h);
-int enqueue_walk(mccfr_handle* h, int batch, float rscale);
-int enqueue_path(mccfr_handle* h, int batch, float rscale, mccfr_trace* d_trace);
-int enqueue_levels(mccfr_handle* h, int batch, float rscale);
+int enqueue_walk(mccfr_handle* h, int batch, const DealRec* deals, float rscale);
+int enqueue_path(mccfr_handle* h, int batch, const DealRec* deals, float rscale, mccfr_trace* d_trace);
+int enqueue_levels(mccfr_handle* h, int batch, const DealRec* deals, float rscale);
 
-// Enqueues one player-update (traverse + apply) reading the device schedule;
-// `ev3` (optional) receives event records before, between and after.
-int enqueue_update(mccfr_handle* h, int batch, mccfr_trace* d_trace, cudaEvent_t* ev3, bool capturing = false) {
+// The counters of a handle's traversal kernel that must be zero when it starts.
+uint32_t* traversal_ctl(const mccfr_handle* h, int* words) {
+  const bool walk = use_walk(h);
+  *words = walk ? (int)(sizeof(WalkCtl) / 4) : 1;
+  return walk ? reinterpret_cast<uint32_t*>(h->wb.ctl) : h->d_work;
+}
+
+// Whether an iteration deals for all its players in one launch: while that is
+// little memory (2^18 deals are 16 MB), since small deals are bound by the latency
+// of their dependent lookups (1,000 heads-up deals take 9 us, like 2,000; 2^18
+// six-player deals run at the throughput of larger ones).
+bool deal_ahead(const mccfr_handle* h, int batch) {
+  return (long long)batch * h->cfg.num_players <= (1 << 18);
+}
+
+// Enqueues the deals of `players` updates, the first of which it begins.
+int enqueue_deal(mccfr_handle* h, int batch, int players) {
+  HandView hv{h->d_hr, h->d_pre, h->d_cdf};
+  const long long n = (long long)batch * players;
+  if (n > h->deals_cap) return fail(h, MCCFR_ERR_INVALID_ARG, "deal buffer smaller than the batch");
+  int words = 0;
+  uint32_t* const ctl = traversal_ctl(h, &words);
+  if (h->gp.sub_street)
+    k_deal<true><<<(int)((n * kDealGroup + 127) / 128), 128, 0, h->stream>>>(
+        h->gp, hv, h->d_sched, batch, players, h->d_deals, table_epoch(h->tv), ctl, words);
+  else
+    k_deal<false><<<(int)std::min<long long>((n + 127) / 128, kDealBlocks), 128, 0, h->stream>>>(
+        h->gp, hv, h->d_sched, batch, players, h->d_deals, table_epoch(h->tv), ctl, words);
+  CK(cudaGetLastError());
+  return MCCFR_OK;
+}
+
+// Enqueues the traversal and the apply of one player-update whose deals are at
+// `deals`, reading the device schedule; `ev3` (optional) receives event records
+// before, between and after.
+int enqueue_update(mccfr_handle* h, int batch, const DealRec* deals, mccfr_trace* d_trace, cudaEvent_t* ev3,
+                   bool capturing, const Advance& adv) {
   const int rb = regret_frac_bits(h->cfg, batch);
   const float rscale = std::ldexp(1.0f, rb);
   const double rinv = std::ldexp(1.0, -rb);
-  HandView hv{h->d_hr, h->d_pre, h->d_cdf};
-  if (batch > h->deals_cap) return fail(h, MCCFR_ERR_INVALID_ARG, "deal buffer smaller than the batch");
-  const bool walk = use_walk(h);
-  // the traversal's counters, which the deal zeroes
-  uint32_t* const ctl = walk ? reinterpret_cast<uint32_t*>(h->wb.ctl) : h->d_work;
-  const int ctl_words = walk ? (int)(sizeof(WalkCtl) / 4) : 1;
-  if (h->gp.sub_street)
-    k_deal<true><<<(int)(((long long)batch * kDealGroup + 127) / 128), 128, 0, h->stream>>>(
-        h->gp, hv, h->d_sched, batch, h->d_deals, table_epoch(h->tv), ctl, ctl_words);
-  else
-    k_deal<false><<<std::min((batch + 127) / 128, kDealBlocks), 128, 0, h->stream>>>(
-        h->gp, hv, h->d_sched, batch, h->d_deals, table_epoch(h->tv), ctl, ctl_words);
-  CK(cudaGetLastError());
   if (ev3 && record(h, ev3[0], capturing)) return MCCFR_ERR_CUDA;
   if (h->cfg.sampling == MCCFR_SAMPLING_REFERENCE) {
-    const int rc = enqueue_path(h, batch, rscale, d_trace);
+    const int rc = enqueue_path(h, batch, deals, rscale, d_trace);
     if (rc) return rc;
-  } else if (walk || use_levels(h)) {
-    const int rc = walk ? enqueue_walk(h, batch, rscale) : enqueue_levels(h, batch, rscale);
+  } else if (use_walk(h) || use_levels(h)) {
+    const int rc = use_walk(h) ? enqueue_walk(h, batch, deals, rscale) : enqueue_levels(h, batch, deals, rscale);
     if (rc) return rc;
   } else {
-    launch_traverse_es(h->gp, h->tv, h->d_deals, h->d_sched, batch, rscale, h->d_counters, h->d_work, h->stream,
-                       h->device);
+    launch_traverse_es(h->gp, h->tv, deals, h->d_sched, batch, rscale, h->d_counters, h->d_work, h->stream, h->device);
   }
   CK(cudaGetLastError());
   if (ev3 && record(h, ev3[1], capturing)) return MCCFR_ERR_CUDA;
-  k_apply<<<148 * 3, kApplyBlock, 0, h->stream>>>(h->gp, h->tv, h->d_sched, rinv);
+  // three blocks per SM are resident; a small table has fewer bitmap words than warps
+  const int blocks = (int)std::max(1u, std::min(148u * 3, (h->tv.n_words + 7) / 8));
+  k_apply<<<blocks, kApplyBlock, 0, h->stream>>>(h->gp, h->tv, h->d_sched, rinv, adv);
   CK(cudaGetLastError());
   if (ev3 && record(h, ev3[2], capturing)) return MCCFR_ERR_CUDA;
   return MCCFR_OK;
+}
+
+// Enqueues one training iteration: every player's update.  `ev` (optional): three
+// events per update.
+int enqueue_iteration(mccfr_handle* h, int batch, cudaEvent_t* ev, bool capturing) {
+  const int np = h->cfg.num_players;
+  const bool ahead = deal_ahead(h, batch);
+  Advance adv{h->d_sched, nullptr, 0, ahead ? 1 : 0};
+  adv.ctl = traversal_ctl(h, &adv.ctl_words);
+  int rc = MCCFR_OK;
+  for (int p = 0; p < np && rc == MCCFR_OK; ++p) {
+    if (p == 0 || !ahead) rc = enqueue_deal(h, batch, ahead ? np : 1);
+    if (rc == MCCFR_OK)
+      rc = enqueue_update(h, batch, h->d_deals + (ahead ? (size_t)p * batch : 0), nullptr, ev ? ev + 3 * p : nullptr,
+                          capturing, adv);
+  }
+  return rc;
 }
 
 // Most decisions of the updating player on a path: at most raise_cap + 1 per
@@ -912,10 +976,14 @@ bool use_levels(const mccfr_handle* h) {
 // kMaxLevels (the deepest level is then walked depth first).
 int level_count(const mccfr_handle* h) { return std::min(max_decisions(h) + 1, kMaxLevels); }
 
+// Drops the training graph; batches whose graphs hold this handle's updates see
+// the new generation and capture theirs again.
 void drop_graph(mccfr_handle* h) {
   if (h->graph) cudaGraphExecDestroy(h->graph);
   h->graph = nullptr;
   h->graph_batch = -1;
+  h->direct_iters = 0;
+  h->generation++;
 }
 
 // Node records of the walk form's warps: as many blocks as are resident, or as
@@ -962,7 +1030,7 @@ int ensure_form(mccfr_handle* h, int batch) {
 
 // The reference's rule: persistent lanes, as many as are resident or as the batch
 // has traversals for.
-int enqueue_path(mccfr_handle* h, int batch, float rscale, mccfr_trace* d_trace) {
+int enqueue_path(mccfr_handle* h, int batch, const DealRec* deals, float rscale, mccfr_trace* d_trace) {
   if (!h->path_resident) {
     int sms = 0, per = 0;
     CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, h->device));
@@ -975,13 +1043,13 @@ int enqueue_path(mccfr_handle* h, int batch, float rscale, mccfr_trace* d_trace)
       {{k_path<false, false, false>, k_path<false, false, true>}, {k_path<false, true, false>, k_path<false, true, true>}},
       {{k_path<true, false, false>, k_path<true, false, true>}, {k_path<true, true, false>, k_path<true, true, true>}}};
   const Kernel kern = kernels[h->tv.direct ? 1 : 0][h->cfg.key_mode == MCCFR_KEY_FNV26][d_trace ? 1 : 0];
-  kern<<<blocks, kPathBlock, 0, h->stream>>>(h->gp, h->tv, h->d_deals, h->d_sched, batch, rscale, h->d_counters,
+  kern<<<blocks, kPathBlock, 0, h->stream>>>(h->gp, h->tv, deals, h->d_sched, batch, rscale, h->d_counters,
                                              h->d_work, d_trace);
   CK(cudaGetLastError());
   return MCCFR_OK;
 }
 
-int enqueue_walk(mccfr_handle* h, int batch, float rscale) {
+int enqueue_walk(mccfr_handle* h, int batch, const DealRec* deals, float rscale) {
   h->last_walk = true;
   h->level_last_batch = batch;
   const int blocks = std::min(h->walk_blocks, (batch + kWalkWarps - 1) / kWalkWarps);
@@ -992,7 +1060,7 @@ int enqueue_walk(mccfr_handle* h, int batch, float rscale) {
   const bool fnv = h->cfg.key_mode == MCCFR_KEY_FNV26;
   auto kern = h->tv.direct ? (fnv ? k_walk<true, true> : k_walk<true, false>)
                            : (fnv ? k_walk<false, true> : k_walk<false, false>);
-  kern<<<blocks, kWalkBlock, 0, h->stream>>>(h->gp, h->tv, h->d_deals, h->d_sched, batch, rscale, wb, h->d_counters);
+  kern<<<blocks, kWalkBlock, 0, h->stream>>>(h->gp, h->tv, deals, h->d_sched, batch, rscale, wb, h->d_counters);
   CK(cudaGetLastError());
   return MCCFR_OK;
 }
@@ -1005,11 +1073,7 @@ int enqueue_walk(mccfr_handle* h, int batch, float rscale) {
 int ensure_levels(mccfr_handle* h, int batch) {
   const int nlev = level_count(h);
   if (h->d_level && h->level_batch >= batch) {
-    if (h->lb.nlev != nlev && h->graph) {  // a subgame re-targeted to another street
-      cudaGraphExecDestroy(h->graph);
-      h->graph = nullptr;
-      h->graph_batch = -1;
-    }
+    if (h->lb.nlev != nlev) drop_graph(h);  // a subgame re-targeted to another street
     h->lb.nlev = nlev;
     return MCCFR_OK;
   }
@@ -1069,32 +1133,28 @@ int ensure_levels(mccfr_handle* h, int batch) {
     CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_level_dfs<128, 2, 1>, 128, smem));
     h->grid_dfs = std::max(1, per) * sms;
   }
-  if (h->graph) {  // the graph captured the old buffers
-    cudaGraphExecDestroy(h->graph);
-    h->graph = nullptr;
-    h->graph_batch = -1;
-  }
+  drop_graph(h);  // the graph captured the old buffers
   return MCCFR_OK;
 }
 
 // One external-sampling update in the level-synchronous form: the levels
 // expanded top down, the seeds that did not fit walked depth first, the
 // recorded showdowns evaluated in one pass, the values returned bottom up.
-int enqueue_levels(mccfr_handle* h, int batch, float rscale) {
+int enqueue_levels(mccfr_handle* h, int batch, const DealRec* deals, float rscale) {
   const LevelBufs& lb = h->lb;
   h->last_walk = false;
   h->level_last_batch = batch;
   CK(cudaMemsetAsync(lb.ctl, 0, sizeof(LevelCtl), h->stream));
-  k_level_expand<128, 1, true><<<h->grid_expand, 128, 0, h->stream>>>(h->gp, h->tv, h->d_deals, h->d_sched, batch,
+  k_level_expand<128, 1, true><<<h->grid_expand, 128, 0, h->stream>>>(h->gp, h->tv, deals, h->d_sched, batch,
                                                                       lb, 0, h->d_counters);
   for (int L = 1; L < lb.nlev; ++L)
-    k_level_expand<128, 1, false><<<h->grid_expand, 128, 0, h->stream>>>(h->gp, h->tv, h->d_deals, h->d_sched,
+    k_level_expand<128, 1, false><<<h->grid_expand, 128, 0, h->stream>>>(h->gp, h->tv, deals, h->d_sched,
                                                                          batch, lb, L, h->d_counters);
   CK(cudaGetLastError());
   k_level_dfs<128, 2, 1><<<h->grid_dfs, 128, 2 * 128 * sizeof(EsFrame), h->stream>>>(
-      h->gp, h->tv, h->d_deals, h->d_sched, batch, rscale, lb, h->d_counters);
+      h->gp, h->tv, deals, h->d_sched, batch, rscale, lb, h->d_counters);
   CK(cudaGetLastError());
-  k_level_showdown<256><<<h->grid_back, 256, 0, h->stream>>>(h->gp, h->d_deals, h->d_sched, lb);
+  k_level_showdown<256><<<h->grid_back, 256, 0, h->stream>>>(h->gp, deals, h->d_sched, lb);
   CK(cudaGetLastError());
   for (int L = lb.nlev - 2; L >= 0; --L)
     k_level_back<256><<<h->grid_back, 256, 0, h->stream>>>(h->gp, h->tv, h->d_sched, batch, rscale, lb, L,
@@ -1103,45 +1163,36 @@ int enqueue_levels(mccfr_handle* h, int batch, float rscale) {
   return MCCFR_OK;
 }
 
-int ensure_deals(mccfr_handle* h, int batch) {
-  if (batch <= h->deals_cap) return MCCFR_OK;
+// Room for `n` deals.
+int ensure_deals(mccfr_handle* h, long long n) {
+  if (n <= h->deals_cap) return MCCFR_OK;
   if (h->d_deals) {
     CK(cudaStreamSynchronize(h->stream));
     cudaFree(h->d_deals);
     h->d_deals = nullptr;
     h->deals_cap = 0;
   }
-  CK(cudaMalloc(&h->d_deals, (size_t)batch * sizeof(DealRec)));
-  h->deals_cap = batch;
-  if (h->graph) {  // the graph captured the old buffer
-    cudaGraphExecDestroy(h->graph);
-    h->graph = nullptr;
-    h->graph_batch = -1;
-  }
+  drop_graph(h);  // the graph captured the old buffer
+  CK(cudaMalloc(&h->d_deals, (size_t)n * sizeof(DealRec)));
+  h->deals_cap = n;
   return MCCFR_OK;
 }
 
-int ensure_graph(mccfr_handle* h, int batch) {
-  {
-    int rc = ensure_deals(h, batch);
-    if (!rc) rc = ensure_form(h, batch);
-    if (rc) return rc;
-  }
-  if (h->graph && h->graph_batch == batch) return MCCFR_OK;
-  if (h->graph) {
-    cudaGraphExecDestroy(h->graph);
-    h->graph = nullptr;
-  }
+// Buffers of one training iteration.
+int ensure_iteration(mccfr_handle* h, int batch) {
+  const int rc = ensure_deals(h, (long long)batch * (deal_ahead(h, batch) ? h->cfg.num_players : 1));
+  return rc ? rc : ensure_form(h, batch);
+}
+
+// The graph of one iteration; `timed`: with event nodes around every update's
+// traversal and apply (three nodes per update, which cost a small update as much
+// as a kernel).
+int ensure_graph(mccfr_handle* h, int batch, bool timed) {
+  if (h->graph && h->graph_batch == batch && h->graph_timed == timed) return MCCFR_OK;
+  drop_graph(h);
   cudaGraph_t g = nullptr;
   CK(cudaStreamBeginCapture(h->stream, cudaStreamCaptureModeThreadLocal));
-  int rc = MCCFR_OK;
-  for (int p = 0; p < h->cfg.num_players && rc == MCCFR_OK; ++p) {
-    rc = enqueue_update(h, batch, nullptr, h->gev + 3 * p, true);
-    if (rc == MCCFR_OK) {
-      k_advance<<<1, 1, 0, h->stream>>>(h->d_sched, h->cfg.num_players);
-      if (cudaGetLastError() != cudaSuccess) rc = MCCFR_ERR_CUDA;
-    }
-  }
+  const int rc = enqueue_iteration(h, batch, timed ? h->gev : nullptr, true);
   const cudaError_t e = cudaStreamEndCapture(h->stream, &g);
   if (rc != MCCFR_OK) {
     if (g) cudaGraphDestroy(g);
@@ -1150,8 +1201,12 @@ int ensure_graph(mccfr_handle* h, int batch) {
   if (e != cudaSuccess) return fail(h, MCCFR_ERR_CUDA, "graph capture failed: %s", cudaGetErrorString(e));
   const cudaError_t e2 = cudaGraphInstantiate(&h->graph, g, 0);
   cudaGraphDestroy(g);
-  if (e2 != cudaSuccess) return fail(h, MCCFR_ERR_CUDA, "graph instantiate failed: %s", cudaGetErrorString(e2));
+  if (e2 != cudaSuccess) {
+    h->graph = nullptr;
+    return fail(h, MCCFR_ERR_CUDA, "graph instantiate failed: %s", cudaGetErrorString(e2));
+  }
   h->graph_batch = batch;
+  h->graph_timed = timed;
   return MCCFR_OK;
 }
 
@@ -1652,11 +1707,7 @@ int mccfr_set_hand_table(mccfr_handle* h, const int32_t* table, size_t n) {
     attr.accessPolicyWindow.hitProp = cudaAccessPropertyPersisting;
     attr.accessPolicyWindow.missProp = cudaAccessPropertyStreaming;
     CK(cudaStreamSetAttribute(h->stream, cudaStreamAttributeAccessPolicyWindow, &attr));
-    if (h->graph) {  // policies are baked into captured kernel nodes
-      cudaGraphExecDestroy(h->graph);
-      h->graph = nullptr;
-      h->graph_batch = -1;
-    }
+    drop_graph(h);  // policies are baked into captured kernel nodes
   }
   h->has_table = true;
   return MCCFR_OK;
@@ -1696,7 +1747,8 @@ int mccfr_step(mccfr_handle* h, long long iteration, int player, int batch, mccf
   int rc = ensure_deals(h, batch);
   if (rc == MCCFR_OK) rc = ensure_form(h, batch);
   if (rc == MCCFR_OK) rc = set_sched(h, iteration, player);
-  if (rc == MCCFR_OK) rc = enqueue_update(h, batch, d_trace, h->ev);
+  if (rc == MCCFR_OK) rc = enqueue_deal(h, batch, 1);
+  if (rc == MCCFR_OK) rc = enqueue_update(h, batch, h->d_deals, d_trace, h->ev, false, Advance{nullptr, nullptr, 0, 0});
   if (rc == MCCFR_OK) {
     const cudaError_t e = cudaStreamSynchronize(h->stream);
     if (e != cudaSuccess) rc = fail(h, MCCFR_ERR_CUDA, "step: %s", cudaGetErrorString(e));
@@ -1727,15 +1779,29 @@ int mccfr_train(mccfr_handle* h, long long iters, int batch, int verbose, const 
   if (!h->has_table) return fail(h, MCCFR_ERR_NO_HAND_TABLE, "load a hand-rank table first");
   if (iters == 0) return MCCFR_OK;
   CK(cudaSetDevice(h->device));
-  int rc = ensure_graph(h, batch);
+  const bool timed = (verbose & 2) != 0;
+  int rc = ensure_iteration(h, batch);
+  if (rc) return rc;
+  // The first few iterations after a change of buffers or parameters are enqueued
+  // launch by launch: capturing and instantiating a graph costs more than they do
+  // (a re-solve of two iterations), and a longer run has its graph from the start.
+  constexpr long long kDirect = 3;
+  const bool direct = !timed && h->direct_iters + iters <= kDirect &&
+                      !(h->graph && h->graph_batch == batch && !h->graph_timed);
+  if (!direct) rc = ensure_graph(h, batch, timed);
   if (rc) return rc;
   const long long base = h->iterations_done;  // iterations before this call
   rc = set_sched(h, base + 1, 0);
   if (rc) return rc;
-  const bool timed = (verbose & 2) != 0;
   const auto t0 = std::chrono::steady_clock::now();
   for (long long i = 0; i < iters; ++i) {
-    CK(cudaGraphLaunch(h->graph, h->stream));
+    if (direct) {
+      rc = enqueue_iteration(h, batch, nullptr, false);
+      if (rc) return rc;
+      h->direct_iters++;
+    } else {
+      CK(cudaGraphLaunch(h->graph, h->stream));
+    }
     if (timed) {
       // event nodes inside the graph bracket every traverse and apply kernel
       const int np = h->cfg.num_players;
@@ -2237,6 +2303,7 @@ struct mccfr_batch {
   cudaGraphExec_t graph = nullptr;
   cudaEvent_t ev_fork = nullptr;       // table-graph form: fork and joins of the tables' branches
   std::vector<cudaEvent_t> ev_join;
+  std::vector<unsigned long long> generations;  // the tables', when the graph was captured
   cudaEvent_t ev_it[2] = {nullptr, nullptr};
   cudaEvent_t ev_ph[2 * MCCFR_MAX_PLAYERS] = {};
   long long iterations = 0;
@@ -2341,12 +2408,8 @@ int batch_enqueue_table_graphs(mccfr_batch* b, bool capturing) {
   for (size_t i = 0; i < b->tables.size(); ++i) {
     mccfr_handle* h = b->tables[i];
     BCK(cudaStreamWaitEvent(h->stream, b->ev_fork, 0));
-    for (int p = 0; p < h->cfg.num_players; ++p) {
-      const int rc = enqueue_update(h, b->traversals[i], nullptr, nullptr, capturing);
-      if (rc) return bfail(b, rc, "table update in the batch graph");
-      k_advance<<<1, 1, 0, h->stream>>>(h->d_sched, h->cfg.num_players);
-      BCK(cudaGetLastError());
-    }
+    const int rc = enqueue_iteration(h, b->traversals[i], nullptr, capturing);
+    if (rc) return bfail(b, rc, "table update in the batch graph");
     BCK(cudaEventRecord(b->ev_join[i], h->stream));
     BCK(cudaStreamWaitEvent(b->stream, b->ev_join[i], 0));
   }
@@ -2363,8 +2426,7 @@ int batch_prepare_table_graphs(mccfr_batch* b) {
   }
   for (size_t i = 0; i < b->tables.size(); ++i) {
     mccfr_handle* h = b->tables[i];
-    int rc = ensure_deals(h, b->traversals[i]);
-    if (!rc) rc = ensure_form(h, b->traversals[i]);
+    const int rc = ensure_iteration(h, b->traversals[i]);
     if (rc) return bfail(b, rc, "table buffers for the batch graph");
   }
   return MCCFR_OK;
@@ -2527,10 +2589,23 @@ int mccfr_batch_train(mccfr_batch* b, long long iters, int flags) {
   int rc = batch_set_scheds(b);
   if (rc) return rc;
   const bool tgraphs = b->tuning.form == MCCFR_BATCH_TABLE_GRAPHS;
-  if (!b->graph && tgraphs) {
-    rc = batch_prepare_table_graphs(b);
-    if (rc) return rc;
-    BCK(cudaStreamSynchronize(b->stream));
+  if (tgraphs) {
+    // a table trained by itself meanwhile may have other buffers or parameters
+    // than the batch's graph was captured with
+    if (b->graph)
+      for (size_t i = 0; i < b->tables.size(); ++i)
+        if (b->tables[i]->generation != b->generations[i]) {
+          cudaGraphExecDestroy(b->graph);
+          b->graph = nullptr;
+          break;
+        }
+    if (!b->graph) {
+      rc = batch_prepare_table_graphs(b);
+      if (rc) return rc;
+      BCK(cudaStreamSynchronize(b->stream));
+      b->generations.clear();
+      for (const mccfr_handle* h : b->tables) b->generations.push_back(h->generation);
+    }
   }
   if (!b->graph) {
     cudaGraph_t g = nullptr;
@@ -2822,11 +2897,7 @@ int mccfr_subgame_reset(mccfr_handle* h, const mccfr_config* cfg, const mccfr_su
   set_direct(h);
   make_params(*cfg, h->gp);
   set_subgame_params(h, cfg, sg, nb);
-  if (h->graph) {
-    cudaGraphExecDestroy(h->graph);
-    h->graph = nullptr;
-  }
-  h->graph_batch = -1;
+  drop_graph(h);
   h->iterations_done = 0;
   h->launches = 0;
   h->round_player = 0;
@@ -2850,11 +2921,7 @@ int mccfr_share_hand_table(mccfr_handle* h, mccfr_handle* src) {
   h->d_hr = src->d_hr;
   h->shared_hr = true;
   h->has_table = true;
-  if (h->graph) {
-    cudaGraphExecDestroy(h->graph);
-    h->graph = nullptr;
-    h->graph_batch = -1;
-  }
+  drop_graph(h);
   return MCCFR_OK;
 }
 

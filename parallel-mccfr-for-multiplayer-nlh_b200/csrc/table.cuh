@@ -40,8 +40,8 @@ struct TableView {
   unsigned int* bits;        // [2][n_words] touched rows: sampled visits, wide
   unsigned int n_words;      // words of one bitmap: one bit per row that a key can own
   // counters, kCounterStride words apart, by epoch parity: touched rows (0, 1) and
-  // wide ones among them (2, 3) of the update, then the epoch (4): updates dealt
-  // since the table was cleared, advanced by the deal that starts each update
+  // wide ones among them (2, 3) of the update; the epoch (4): updates begun since
+  // the table was cleared; blocks of the apply kernel that are done (5)
   unsigned int* counters;
   unsigned long long mask;   // cap - 1
   int log2cap;
@@ -163,8 +163,11 @@ __host__ __device__ __forceinline__ unsigned int* wide_count(const TableView& tv
 __host__ __device__ __forceinline__ unsigned int* table_epoch(const TableView& tv) {
   return tv.counters + (size_t)kCounterStride * 4;
 }
-// Bytes of the counter block (the five above, then the error flag).
-constexpr size_t kCounterBytes = (size_t)kCounterStride * 4 * 5 + 128;
+__host__ __device__ __forceinline__ unsigned int* apply_ticket(const TableView& tv) {
+  return tv.counters + (size_t)kCounterStride * 5;
+}
+// Bytes of the counter block (the six above, then the error flag).
+constexpr size_t kCounterBytes = (size_t)kCounterStride * 4 * 6 + 128;
 
 __device__ __forceinline__ void mark_wide(const TableView& tv, unsigned long long slot) {
   atomicOr(tv.bits + tv.n_words + (unsigned)(slot >> 5), 1u << (slot & 31));

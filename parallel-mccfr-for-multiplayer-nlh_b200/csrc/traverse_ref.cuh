@@ -281,22 +281,28 @@ __device__ __forceinline__ void deal_one(const GameParams& G, const int32_t* __r
                           (uint32_t)board[3] << 24, (uint32_t)board[4] | dealer << 8, 0u, 0u);
 }
 
-// The deal starts an update: it advances the table's epoch and zeroes `ctl`, the
-// counters of the traversal that follows (may be null), so that neither needs a
-// launch of its own.  SUB: a subgame (eight lanes per traversal).
+// Deals of `players` successive updates (the schedule's and the following players'),
+// `batch` traversals each, update after update.  The deal starts an update: it
+// advances the table's epoch and zeroes `ctl`, the counters of the traversal that
+// follows (may be null), so that neither needs a launch of its own.  SUB: a subgame
+// (eight lanes per traversal).
 template <bool SUB>
 __global__ void __launch_bounds__(128) k_deal(const GameParams G, const HandView hv, const Sched* __restrict__ sched,
-                                              int batch, DealRec* __restrict__ out, uint32_t* __restrict__ epoch,
-                                              uint32_t* __restrict__ ctl, int ctl_words) {
+                                              int batch, int players, DealRec* __restrict__ out,
+                                              uint32_t* __restrict__ epoch, uint32_t* __restrict__ ctl,
+                                              int ctl_words) {
   if (blockIdx.x == 0) {
     if (threadIdx.x == 0) *epoch += 1;
     for (int i = threadIdx.x; i < ctl_words; i += blockDim.x) ctl[i] = 0;
   }
+  const uint32_t n = (uint32_t)batch * (uint32_t)players;
+  const uint32_t uid = update_id(sched, G.N);
   if constexpr (SUB) {
-    const uint32_t t = blockIdx.x * (128 / kDealGroup) + threadIdx.x / kDealGroup;
-    if (t >= (uint32_t)batch) return;  // whole groups
+    const uint32_t i = blockIdx.x * (128 / kDealGroup) + threadIdx.x / kDealGroup;
+    if (i >= n) return;  // whole groups
+    const uint32_t p = players > 1 ? i / (uint32_t)batch : 0u;
     const int gl = (int)threadIdx.x & (kDealGroup - 1);
-    deal_subgame(G, hv.hr, t, update_id(sched, G.N), out + t, gl,
+    deal_subgame(G, hv.hr, i - p * (uint32_t)batch, uid + p, out + i, gl,
                  ((1u << kDealGroup) - 1u) << ((threadIdx.x & 31) & ~(kDealGroup - 1)));
   } else {
     __shared__ uint8_t s_pre[52 * 52];
@@ -304,9 +310,10 @@ __global__ void __launch_bounds__(128) k_deal(const GameParams G, const HandView
     for (int i = threadIdx.x; i < 52 * 52 / 4; i += blockDim.x)
       reinterpret_cast<uint32_t*>(s_pre)[i] = __ldg(reinterpret_cast<const uint32_t*>(hv.pre) + i);
     __syncthreads();
-    const uint32_t uid = update_id(sched, G.N);
-    for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < (uint32_t)batch; t += gridDim.x * blockDim.x)
-      deal_one(G, hv.hr, s_pre, hv.cdf, t, uid, out + t, s_deck + kDeckWords * threadIdx.x);
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+      const uint32_t p = players > 1 ? i / (uint32_t)batch : 0u;
+      deal_one(G, hv.hr, s_pre, hv.cdf, i - p * (uint32_t)batch, uid + p, out + i, s_deck + kDeckWords * threadIdx.x);
+    }
   }
 }
 

@@ -108,3 +108,48 @@ def test_a_table_twice_is_refused(hand_table):
     with pytest.raises(L.MccfrError):
         mccfr.Batch([ts[0], ts[0]], [trav[0], trav[0]])
     ts[0].close()
+
+
+def test_batch_graph_follows_its_tables_buffers(hand_table):
+    """Tables trained by themselves between a batch's iterations, with larger
+    updates (other buffers) and timed: the batch's graph is captured again, and
+    everything equals plain training."""
+    cfgs, trav = small_tables()
+    plain, batched = make(cfgs, hand_table), make(cfgs, hand_table)
+    b = mccfr.Batch(batched, trav)
+    for big, timed in ((0, False), (9000, True), (40000, False), (100, True)):
+        for i, (p, q) in enumerate(zip(plain, batched)):
+            if big and i != 1:
+                p.train(2, big, verbose=False)
+                q.train(2, big, verbose=False, timed=timed)
+        b.train(1)
+        for t, n in zip(plain, trav):
+            t.train(1, n, verbose=False)
+    for p, q in zip(plain, batched):
+        assert p.digest() == q.digest()
+        assert p.stats().touched_last >= 0
+    b.close()
+
+
+@pytest.mark.parametrize("batch", [1, 43690, 43691])
+def test_calls_of_few_and_many_iterations_are_the_same_run(hand_table, batch):
+    """train() enqueues its first iterations one launch at a time and replays a
+    graph afterwards, deals an iteration's players together up to 2^18 deals
+    (6 x 43,690) and one by one above; timed graphs carry event nodes.  All the
+    same run as single steps."""
+    c = L.preset(L.PRESET_6MAX_100BB)
+    c.table_log2, c.key_bits = 18, 18
+    a, s = make([c, c], hand_table)
+    its = 0
+    for k, timed in ((1, False), (2, False), (1, False), (2, True), (2, False)):
+        a.train(k, batch, verbose=False, timed=timed)
+        for _ in range(k):
+            for p in range(6):
+                s.step(its + 1, p, batch)
+            its += 1
+        assert a.digest() == s.digest(), its
+    a.train(1, batch, verbose=False, timed=True)
+    for p in range(6):
+        s.step(its + 1, p, batch)
+    assert a.stats().touched_last == s.stats().touched_last
+    assert a.stats().wide_rows_last == s.stats().wide_rows_last
