@@ -83,8 +83,8 @@ __global__ void __launch_bounds__(128) k_deal_batched(const TableDesc* __restric
     if ((D.G.sub_street != 0) != SUB) continue;
     const uint32_t t = (uint32_t)(g - P.off[j]);
     const uint32_t uid = update_id(D.sched, D.G.N);
-    if (SUB) deal_subgame(D.G, T, t, uid, out + g, (int)threadIdx.x & (kDealGroup - 1), gmask);
-    else deal_one(D.G, T, D.pre, D.cdf, t, uid, out + g, s_deck + kDeckWords * threadIdx.x);
+    if constexpr (SUB) deal_subgame(D.G, T, t, uid, out + g, (int)threadIdx.x & (kDealGroup - 1), gmask);
+    else deal_one(D.G, T, D.pre, D.cdf, t, uid, out + g, Deck<128>{s_deck + threadIdx.x});
   }
 }
 

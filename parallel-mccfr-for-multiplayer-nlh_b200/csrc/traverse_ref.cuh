@@ -196,51 +196,69 @@ __device__ __forceinline__ void deal_subgame(const GameParams& G, const int32_t*
   }
 }
 
-// Deal, buckets and river ranks of traversal t of update `uid`
-// (cfr_gpu.cu:460-470, 476-489, 942-952, 963).  `pre` is the 52x52 preflop LUT
-// (shared or global memory), `cdf` the rank-CDF LUTs, `row` this thread's 13 words
-// of shared memory for the deck: a shuffle indexes it by card, and as an array of
-// the thread it lived in local memory (2^18 six-player deals: 98 us).
-constexpr int kDeckWords = 13;  // an odd stride: a warp's decks lie in different banks
+// One thread's 52-card deck in shared memory, as 13 words of four cards, a block's
+// width apart: whatever cards a warp's threads touch, each works in its own bank.
+// (As a thread's own array the shuffle's indexing put it in local memory, and as
+// rows of 13 words the threads' banks met at random.)
+constexpr int kDeckWords = 13;
+template <int STRIDE>
+struct Deck {
+  uint32_t* col;
+  __device__ __forceinline__ uint8_t& at(int i) const {
+    return reinterpret_cast<uint8_t*>(col + (i >> 2) * STRIDE)[i & 3];
+  }
+  __device__ __forceinline__ uint32_t word(int w) const { return col[w * STRIDE]; }
 
-__device__ __forceinline__ void deal_one(const GameParams& G, const int32_t* __restrict__ T, const uint8_t* pre,
-                                         const uint8_t* __restrict__ cdf, uint32_t t, uint32_t uid,
-                                         DealRec* __restrict__ out, uint32_t* row) {
-  uint8_t* const deck = reinterpret_cast<uint8_t*>(row);
-  const int N = G.N;
-  const int n_deal = 2 * N + 5;
+  // The first `n_deal` cards of traversal t's shuffle in update `uid`
+  // (cfr_gpu.cu:460-470): partial Fisher-Yates by multiply-shift, four draws per
+  // Philox block; returns the word after the last draw.
+  __device__ __forceinline__ uint32_t shuffle(const GameParams& G, uint32_t t, uint32_t uid, int n_deal) const {
 #pragma unroll
-  for (int w = 0; w < kDeckWords; ++w) row[w] = 0x03020100u + 0x04040404u * (uint32_t)w;  // cards 4w .. 4w+3
-  uint32_t dealer = 0;
-  for (int blk = 0; 4 * blk <= n_deal; ++blk) {
-    const U4 o = philox(U4{t, uid, 0u, (uint32_t)blk}, G.seed_lo, G.seed_hi);
-    const uint32_t wv[4] = {o.x, o.y, o.z, o.w};
+    for (int w = 0; w < kDeckWords; ++w) col[w * STRIDE] = 0x03020100u + 0x04040404u * (uint32_t)w;  // cards 4w .. 4w+3
+    uint32_t next = 0;
+    for (int blk = 0; 4 * blk <= n_deal; ++blk) {
+      const U4 o = philox(U4{t, uid, 0u, (uint32_t)blk}, G.seed_lo, G.seed_hi);
+      const uint32_t wv[4] = {o.x, o.y, o.z, o.w};
 #pragma unroll
-    for (int e = 0; e < 4; ++e) {
-      const int i = 4 * blk + e;
-      if (i < n_deal) {
-        const int j = i + (int)__umulhi(wv[e], (uint32_t)(52 - i));
-        const uint8_t tmp = deck[i];
-        deck[i] = deck[j];
-        deck[j] = tmp;
-      } else if (i == n_deal) {
-        dealer = wv[e] % (uint32_t)N;
+      for (int e = 0; e < 4; ++e) {
+        const int i = 4 * blk + e;
+        if (i < n_deal) {
+          uint8_t& mine = at(i);
+          uint8_t& drawn = at(i + (int)__umulhi(wv[e], (uint32_t)(52 - i)));
+          const uint8_t tmp = mine;
+          mine = drawn;
+          drawn = tmp;
+        } else if (i == n_deal) {
+          next = wv[e];
+        }
       }
     }
+    return next;
   }
+};
+
+// Deal, buckets and river ranks of traversal t of update `uid`
+// (cfr_gpu.cu:460-470, 476-489, 942-952, 963).  `pre` is the 52x52 preflop LUT
+// (shared or global memory), `cdf` the rank-CDF LUTs.
+template <int STRIDE>
+__device__ __forceinline__ void deal_one(const GameParams& G, const int32_t* __restrict__ T, const uint8_t* pre,
+                                         const uint8_t* __restrict__ cdf, uint32_t t, uint32_t uid,
+                                         DealRec* __restrict__ out, const Deck<STRIDE> deck) {
+  const int N = G.N;
+  const uint32_t dealer = deck.shuffle(G, t, uid, 2 * N + 5) % (uint32_t)N;
   int board[5];
 #pragma unroll
-  for (int i = 0; i < 5; ++i) board[i] = deck[2 * N + i];
+  for (int i = 0; i < 5; ++i) board[i] = deck.at(2 * N + i);
   int32_t b = __ldg(T + 53 + to_rm(board[0]));
   b = __ldg(T + b + to_rm(board[1]));
   b = __ldg(T + b + to_rm(board[2]));
   int32_t s5[kMaxPlayers], s6[kMaxPlayers], r7[kMaxPlayers], s4[kMaxPlayers];
 #pragma unroll
   for (int p = 0; p < kMaxPlayers; ++p)
-    if (p < N) s4[p] = __ldg(T + b + to_rm(deck[2 * p]));
+    if (p < N) s4[p] = __ldg(T + b + to_rm(deck.at(2 * p)));
 #pragma unroll
   for (int p = 0; p < kMaxPlayers; ++p)
-    if (p < N) s5[p] = __ldg(T + s4[p] + to_rm(deck[2 * p + 1]));
+    if (p < N) s5[p] = __ldg(T + s4[p] + to_rm(deck.at(2 * p + 1)));
   const int rm3 = to_rm(board[3]), rm4 = to_rm(board[4]);
 #pragma unroll
   for (int p = 0; p < kMaxPlayers; ++p)
@@ -254,7 +272,7 @@ __device__ __forceinline__ void deal_one(const GameParams& G, const int32_t* __r
     ctx[p] = 0;
     rank[p] = 0;
     if (p >= N) continue;
-    const uint32_t hb = pre[deck[2 * p] * 52 + deck[2 * p + 1]];
+    const uint32_t hb = pre[deck.at(2 * p) * 52 + deck.at(2 * p + 1)];
     const uint32_t rr = decode16((uint32_t)r7[p] & 0xFFFF);
     uint32_t b1, b2, b3;
     if (G.postflop_mode == 0) {
@@ -274,9 +292,9 @@ __device__ __forceinline__ void deal_one(const GameParams& G, const int32_t* __r
   uint4* const dst = reinterpret_cast<uint4*>(out);
   dst[0] = make_uint4(ctx[0], ctx[1], ctx[2], ctx[3]);
   dst[1] = make_uint4(ctx[4], ctx[5], rank[0] | rank[1] << 16, rank[2] | rank[3] << 16);
-  const uint32_t h1 = N == 2 ? 0u : N == 3 ? row[1] & 0xFFFFu : row[1];
-  const uint32_t h2 = N <= 4 ? 0u : N == 5 ? row[2] & 0xFFFFu : row[2];
-  dst[2] = make_uint4(rank[4] | rank[5] << 16, row[0], h1, h2);
+  const uint32_t h1 = N == 2 ? 0u : N == 3 ? deck.word(1) & 0xFFFFu : deck.word(1);
+  const uint32_t h2 = N <= 4 ? 0u : N == 5 ? deck.word(2) & 0xFFFFu : deck.word(2);
+  dst[2] = make_uint4(rank[4] | rank[5] << 16, deck.word(0), h1, h2);
   dst[3] = make_uint4((uint32_t)board[0] | (uint32_t)board[1] << 8 | (uint32_t)board[2] << 16 |
                           (uint32_t)board[3] << 24, (uint32_t)board[4] | dealer << 8, 0u, 0u);
 }
@@ -312,7 +330,8 @@ __global__ void __launch_bounds__(128) k_deal(const GameParams G, const HandView
     __syncthreads();
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
       const uint32_t p = players > 1 ? i / (uint32_t)batch : 0u;
-      deal_one(G, hv.hr, s_pre, hv.cdf, i - p * (uint32_t)batch, uid + p, out + i, s_deck + kDeckWords * threadIdx.x);
+      deal_one(G, hv.hr, s_pre, hv.cdf, i - p * (uint32_t)batch, uid + p, out + i,
+               Deck<128>{s_deck + threadIdx.x});
     }
   }
 }
