@@ -130,27 +130,30 @@ __device__ __forceinline__ void deal_subgame(const GameParams& G, const int32_t*
     if (fit) winner = __ffs((int)fit) - 1;
   }
   if (winner < 0) {
+    // player by player from the first attempt's draws (the group's first lane's),
+    // eight combos of the search at a time: neighbours share their higher card, so a
+    // search often passes dozens
     winner = __ffs((int)gmask) - 1;
-    if (gl == 0) {
-      used = used_board;
+    used = used_board;
 #pragma unroll
-      for (int p = 0; p < kMaxPlayers; ++p) {
-        if (p >= N) break;
-        const uint32_t* cdf = G.range_cdf + 1326 * p;
-        const int start = first[p];  // attempt 0 is this lane's
-        int pick = -1;
-        for (int k = 0; k < 1326 && pick < 0; ++k) {
-          const int c = start + k < 1326 ? start + k : start + k - 1326;
-          const uint32_t prev = c ? __ldg(cdf + c - 1) : 0u;
-          if (__ldg(cdf + c) == prev) continue;  // zero weight
-          if (!(used & combo_bits(c))) pick = c;
+    for (int p = 0; p < kMaxPlayers; ++p) {
+      if (p >= N) break;
+      const uint32_t* cdf = G.range_cdf + 1326 * p;
+      const int start = __shfl_sync(gmask, first[p], winner);
+      int pick = start;  // kept when the range is exhausted by card removal
+      for (int k = 0; k < 1326; k += kDealGroup) {
+        const int c = start + k + gl < 1326 ? start + k + gl : start + k + gl - 1326;
+        bool fits = false;
+        if (k + gl < 1326) fits = __ldg(cdf + c) != (c ? __ldg(cdf + c - 1) : 0u) && !(used & combo_bits(c));
+        const unsigned fit = __ballot_sync(gmask, fits) & gmask;
+        if (fit) {
+          pick = __shfl_sync(gmask, c, __ffs((int)fit) - 1);
+          break;
         }
-        if (pick < 0) pick = start;  // range exhausted by card removal: keep the draw
-        combo[p] = pick;
-        used |= combo_bits(pick);
       }
+      combo[p] = pick;
+      used |= combo_bits(pick);
     }
-    __syncwarp(gmask);
   }
   int mine = 0;
 #pragma unroll
