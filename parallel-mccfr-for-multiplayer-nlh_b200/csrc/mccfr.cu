@@ -418,6 +418,8 @@ struct ReadOut {
   unsigned key32_sub;
 };
 
+// A span writes no more rows than were counted in it: a table that another thread
+// trains meanwhile may have gained some.
 template <int WHAT>
 __global__ void __launch_bounds__(kReadBlock) k_read_write(const TableView tv, const unsigned* __restrict__ offsets,
                                                            const ReadOut out) {
@@ -439,12 +441,13 @@ __global__ void __launch_bounds__(kReadBlock) k_read_write(const TableView tv, c
   if (lane == 0) s_c[warp] = c;
   __syncthreads();
   unsigned at = offsets[blockIdx.x];
+  const unsigned end = offsets[blockIdx.x + 1];
   for (int w = 0; w < warp; ++w) at += s_c[w];
 #pragma unroll
   for (int k = 0; k < 4; ++k) {
     const unsigned i = at + __popc(m[k] & ((1u << lane) - 1u));
     at += __popc(m[k]);
-    if (!((m[k] >> lane) & 1)) continue;
+    if (!((m[k] >> lane) & 1) || i >= end) continue;
     const unsigned long long s = base + 32 * k + lane;
     if (out.keys) out.keys[i] = key[k];
     if (out.keys32) out.keys32[i] = (unsigned)key[k] - out.key32_sub;
@@ -652,7 +655,9 @@ struct mccfr_handle {
   long long touched_last = 0;
   long long wide_last = 0;  // of those, rows whose second line was folded
   // scratch of calls that read the table back or stage host data, kept between
-  // calls up to kScratchKept bytes, and the span counts of table reads
+  // calls up to kScratchKept bytes, and the span counts of table reads; such calls
+  // on one handle from several threads take turns
+  std::mutex read_mu;
   void* d_scratch = nullptr;
   size_t scratch_bytes = 0;
   unsigned* d_spans = nullptr;
@@ -1249,9 +1254,11 @@ struct Scratch {
     h->scratch_bytes = 0;
     const size_t want = std::min(kScratchKept, std::max<size_t>(bytes + bytes / 4, 1u << 20));
     const cudaError_t e = cudaMalloc(&h->d_scratch, want);
-    if (e != cudaSuccess) {
+    if (e != cudaSuccess) {  // no room to spare: this call's bytes alone
       h->d_scratch = nullptr;
-      return e;
+      cudaGetLastError();
+      own = true;
+      return cudaMalloc(&p, bytes);
     }
     h->scratch_bytes = want;
     p = h->d_scratch;
@@ -1372,6 +1379,7 @@ int fetch_rows(mccfr_handle* h, int what, unsigned n, uint64_t* keys, uint32_t* 
 
 // Every occupied row, sorted by key, as v2 checkpoint records.
 int read_host_rows(mccfr_handle* h, std::vector<HostRow>& rows) {
+  std::lock_guard<std::mutex> lock(h->read_mu);
   unsigned n = 0;
   int rc = count_read(h, kReadRows, &n);
   if (rc) return rc;
@@ -1896,6 +1904,7 @@ int mccfr_export_rows(mccfr_handle* h, uint64_t* keys, float* regrets, float* st
                       size_t capacity, size_t* count) {
   if (!h || !count) return MCCFR_ERR_INVALID_ARG;
   CK(cudaSetDevice(h->device));
+  std::lock_guard<std::mutex> lock(h->read_mu);
   if (capacity == 0) {  // size query: a counting pass only
     unsigned int n = 0;
     const int rc = count_rows(h, &n);
@@ -1915,6 +1924,7 @@ int mccfr_get_strategy(mccfr_handle* h, uint32_t* keys, uint64_t* keys64, float*
                        size_t* count) {
   if (!h || !count) return MCCFR_ERR_INVALID_ARG;
   CK(cudaSetDevice(h->device));
+  std::lock_guard<std::mutex> lock(h->read_mu);
   if (capacity == 0) {  // size query: occupied rows, an upper bound of the rows written
     unsigned int n = 0;
     const int rc = count_rows(h, &n);
@@ -1932,6 +1942,7 @@ int mccfr_get_strategy(mccfr_handle* h, uint32_t* keys, uint64_t* keys64, float*
 int mccfr_num_info_sets_active(mccfr_handle* h, long long* out) {
   if (!h || !out) return MCCFR_ERR_INVALID_ARG;
   CK(cudaSetDevice(h->device));
+  std::lock_guard<std::mutex> lock(h->read_mu);
   unsigned n = 0;
   const int rc = count_read(h, kReadActive, &n);
   *out = rc ? 0 : (long long)n;
@@ -2201,6 +2212,7 @@ int mccfr_eval7(mccfr_handle* h, const uint8_t* cards, uint16_t* ranks, size_t n
     for (size_t i = 0; i < 7 * n; ++i)
       if (cards[i] > 51) return fail(h, MCCFR_ERR_INVALID_ARG, "card code %d out of range", (int)cards[i]);
   CK(cudaSetDevice(h->device));
+  std::lock_guard<std::mutex> lock(h->read_mu);
   Scratch scratch(h);
   const size_t at = (7 * n + 15) & ~(size_t)15;  // the ranks, after the cards
   const cudaError_t e = scratch.take(at + 2 * n);
@@ -3149,12 +3161,18 @@ int mccfr_exploitability(mccfr_handle* h, const mccfr_br_options* opt, mccfr_exp
   if (!h->has_table) return fail(h, MCCFR_ERR_NO_HAND_TABLE, "no hand table loaded");
   CK(cudaSetDevice(h->device));
   unsigned n = 0;
-  int rc = count_read(h, kReadRows, &n);
-  if (rc) return rc;
-  std::vector<uint64_t> keys(n);
-  std::vector<float> ssum(8ull * n);
-  rc = fetch_rows(h, kReadRows, n, keys.data(), nullptr, nullptr, ssum.data(), nullptr);
-  if (rc) return rc;
+  int rc = MCCFR_OK;
+  std::vector<uint64_t> keys;
+  std::vector<float> ssum;
+  {
+    std::lock_guard<std::mutex> lock(h->read_mu);
+    rc = count_read(h, kReadRows, &n);
+    if (rc) return rc;
+    keys.resize(n);
+    ssum.resize(8ull * n);
+    rc = fetch_rows(h, kReadRows, n, keys.data(), nullptr, nullptr, ssum.data(), nullptr);
+    if (rc) return rc;
+  }
   std::vector<int32_t> table(MCCFR_HAND_TABLE_ENTRIES);
   CK(cudaMemcpy(table.data(), h->d_hr, table.size() * sizeof(int32_t), cudaMemcpyDeviceToHost));
   mccfr_br_options o;

@@ -4,6 +4,7 @@ the oracle's; sizes and capacities as declared."""
 from __future__ import annotations
 
 import ctypes
+from concurrent.futures import ThreadPoolExecutor
 
 import numpy as np
 import pytest
@@ -83,4 +84,36 @@ def test_eval7_staging_sizes(hand_table, n):
     bad[n - 1, 6] = 52
     with pytest.raises(mccfr.MccfrError, match="52"):
         tr.eval7(bad)
+    tr.close()
+
+
+@pytest.mark.parametrize("threads", [2, 6])
+def test_reads_of_one_handle_from_several_threads(hand_table, threads):
+    """Rows, strategies and staged hands of one handle, read by several threads at
+    once: each gets what it gets alone, though the reads share the handle's scratch."""
+    tr = mccfr.GPUCFRTrainer(config=_cfg(16, 13))
+    tr.set_hand_table(hand_table)
+    tr.train(2, 2000, verbose=False)
+    rng = np.random.default_rng(threads)
+    hands = [rng.random((m, 52)).argpartition(7, axis=1)[:, :7].astype(np.uint8) for m in (16, 9_001, 150_001)]
+    ranks = [binding.eval7(hand_table, c) for c in hands]
+    rows, strat, active = tr.export_rows(), tr.strategy_arrays(), tr.num_info_sets_active()
+
+    def read(i):
+        for k in range(12):
+            w = (i + k) % 4
+            if w == 0:
+                c = (i + k) // 4 % 3
+                assert np.array_equal(tr.eval7(hands[c]), ranks[c])
+            elif w == 1:
+                got = tr.export_rows()
+                assert all(np.array_equal(got[f].view(np.uint8), rows[f].view(np.uint8)) for f in rows)
+            elif w == 2:
+                assert all(np.array_equal(a.view(np.uint8), b.view(np.uint8)) for a, b in
+                           zip(tr.strategy_arrays(), strat))
+            else:
+                assert tr.num_info_sets_active() == active
+
+    with ThreadPoolExecutor(threads) as pool:
+        list(pool.map(read, range(threads)))
     tr.close()
