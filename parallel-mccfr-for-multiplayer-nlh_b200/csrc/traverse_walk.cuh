@@ -33,6 +33,14 @@
 // Every sum that reaches the table is an integer (fixed point) and every draw is
 // keyed by the node's action path, so the rows after an update are those of the
 // other forms, bit for bit, whatever the order of the walks.
+//
+// What bounds it: the dependent issue of a step's code (about 1,450 instructions for
+// 23 decisions; 41% of issue slots, no unit above half its rate) and, in tables far
+// beyond L2, random 64-byte accesses: 16 G visits/s in a 33 MB table, 10 G in one of
+// 17 GB.  6-max 100BB at 2^20 traversals per update took the level kernels 14.4 ms
+// (expand 10.8, back 3.0, showdowns 0.5) and takes this one 5.8-6.1 ms; a 1,000-
+// traversal heads-up update 220 us and 60 us.  Six blocks of 80 registers per SM:
+// five and seven are within 3%, eight spill and are 5% slower.
 #pragma once
 #include "game.cuh"
 #include "table.cuh"
@@ -44,10 +52,10 @@ namespace mccfr {
 
 constexpr int kWalkBlock = 128;
 constexpr int kWalkWarps = kWalkBlock / 32;
-constexpr int kWalkNodes = 192;                  // open updating-player nodes of a warp
+constexpr int kWalkNodes = 192;                  // open updating-player nodes of a warp (128: heads-up 15% slower)
 constexpr int kWalkSeeds = kSlots * kWalkNodes;  // their children not yet taken
 constexpr int kWalkQueue = 64;                   // queue entries: 31 left over + 32 of one step
-constexpr int kWalkReady = 24;                   // lanes at a decision that end the filling of a step
+constexpr int kWalkReady = 24;                   // lanes at a decision that end the filling of a step (28: up to 7% slower, 20: equal)
 constexpr uint32_t kWalkRoot = 0xFFFFu;          // parent of a traversal's root
 
 // Counters of one update, zeroed by the deal that precedes the walk.

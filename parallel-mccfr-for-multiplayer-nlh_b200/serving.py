@@ -105,8 +105,8 @@ def request_config(req: Request) -> L.Config:
 
 
 def table_bytes(req: Request) -> int:
-    """Device bytes of a request's table: 256-byte rows and a 4-byte touched-list
-    entry per row, plus its small buffers."""
+    """Device bytes a request's table is counted as: 256-byte rows with 4 bytes each
+    for bitmaps and read-back, plus its small buffers."""
     return (1 << req.table_log2) * (256 + 4) + (1 << 20)
 
 
