@@ -57,7 +57,7 @@ namespace {
 // time, one lane per row in nearly ascending address order.  The bytes of the rows
 // are what it costs: a lane has its row's whole first line in flight at once (and
 // da for a wide row), and writes only what changed.  At 2^20 traversals of 6-max
-// 100BB it folds 26.7 M rows in 1.85 ms, 14.4 rows/ns (79% of the measured copy
+// 100BB it folds 26.7 M rows in 1.85 ms, 14.4 rows/ns (58% of the measured copy
 // bandwidth by the bytes it needs); eight lanes per row over a list of touched rows
 // in random order, the second line read for every row, folded 8.5 rows/ns.
 // `group` of `ngroups`: the warps working on this table.
