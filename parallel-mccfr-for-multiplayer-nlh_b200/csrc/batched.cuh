@@ -214,7 +214,11 @@ k_walk_round(const TableDesc* __restrict__ tables, int n, const DealRec* __restr
   walk_init(s_warp[warp]);
   for (int k = 0; k < n; ++k) {
     const int j = (id + k) % n;
-    if (ld_volatile(work + j) >= (unsigned)tables[j].batch) continue;  // none left to take
+    // Lane 0 reads for the warp: other warps count the word up meanwhile, and lanes
+    // that read for themselves could part at the branch and wait for each other in
+    // different tables' collectives.
+    const unsigned taken = __shfl_sync(0xFFFFFFFFu, lane == 0 ? ld_volatile(work + j) : 0u, 0);
+    if (taken >= (unsigned)tables[j].batch) continue;  // none left to take
     for (int i = lane; i < (int)(sizeof(TableDesc) / 4); i += 32)
       reinterpret_cast<uint32_t*>(&D)[i] = __ldg(reinterpret_cast<const uint32_t*>(tables + j) + i);
     __syncwarp();
