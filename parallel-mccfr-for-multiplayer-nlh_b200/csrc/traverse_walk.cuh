@@ -522,6 +522,8 @@ __device__ __forceinline__ void walk_update(const GameParams& G, const TableView
     const unsigned offm = __ballot_sync(0xFFFFFFFFu, off);
     if (off) W.off[n_off + __popc(offm & below)] = make_uint2((uint32_t)slot, vm);
     n_off += __popc(offm);
+    // other lanes read the entries, and the votes on the way there order no memory
+    if (offm) __syncwarp();
     // ---- updating-player nodes: a record and one seed per legal action
     if (__any_sync(0xFFFFFFFFu, isup)) {
       const unsigned full = __ballot_sync(0xFFFFFFFFu, isup && slot < 0);  // no row: nothing to update
