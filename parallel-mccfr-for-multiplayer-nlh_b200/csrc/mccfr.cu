@@ -831,7 +831,8 @@ int check_device_error(mccfr_handle* h) {
   CK(cudaMemcpy(&e, h->tv.err, sizeof(int), cudaMemcpyDeviceToHost));
   if (e) {
     h->sticky_err |= e;
-    CK(cudaMemset(h->tv.err, 0, sizeof(int)));
+    CK(cudaMemsetAsync(h->tv.err, 0, sizeof(int), h->stream));
+    CK(cudaStreamSynchronize(h->stream));
     if (e & kErrTableFull)
       return fail(h, MCCFR_ERR_TABLE_FULL, "info-set table full (capacity %llu rows); raise table_log2", h->cap);
     return fail(h, MCCFR_ERR_DEVICE, "kernel error flags 0x%x", e);
@@ -1599,22 +1600,26 @@ int mccfr_create(const mccfr_config* cfg, mccfr_handle** out) {
   uint8_t pre[52 * 52];
   build_preflop_lut(cfg->preflop_mode, cfg->preflop_buckets, pre);
   CKC(cudaMalloc(&h->d_pre, sizeof(pre)));
-  CKC(cudaMemcpy(h->d_pre, pre, sizeof(pre), cudaMemcpyHostToDevice));
+  CKC(cudaMemcpyAsync(h->d_pre, pre, sizeof(pre), cudaMemcpyHostToDevice, h->stream));
   CKC(cudaMalloc(&h->d_cdf, kCdfBytes));
-  CKC(cudaMemset(h->d_cdf, 0, kCdfBytes));
+  CKC(cudaMemsetAsync(h->d_cdf, 0, kCdfBytes, h->stream));
   CKC(cudaMalloc(&h->d_sched, sizeof(Sched)));
   CKC(cudaMallocHost(&h->h_sched, sizeof(Sched)));
   CKC(cudaMalloc(&h->d_counters, sizeof(Counters)));
-  CKC(cudaMemset(h->d_counters, 0, sizeof(Counters)));
+  CKC(cudaMemsetAsync(h->d_counters, 0, sizeof(Counters), h->stream));
   CKC(cudaMalloc(&h->d_work, 256));
-  CKC(cudaMemset(h->d_work, 0, 256));
+  CKC(cudaMemsetAsync(h->d_work, 0, 256, h->stream));
   // Table rows, the touched-row bitmaps and small counters in one allocation.
   h->cap = 1ull << cfg->table_log2;
   const unsigned long long C = h->cap;
   const size_t bytes_rows = C * kRowBytes, bytes_bits = C / 4, bytes_misc = kCounterBytes;
   h->block_bytes = bytes_rows + bytes_bits + bytes_misc;
   CKC(cudaMalloc(&h->d_block, h->block_bytes));
-  CKC(cudaMemset(h->d_block, 0, h->block_bytes));
+  // On the handle's own stream and waited for: no stream of the library waits for the
+  // default one, a table of many GB takes milliseconds to clear, and rounds and
+  // batches read it on streams of theirs.
+  CKC(cudaMemsetAsync(h->d_block, 0, h->block_bytes, h->stream));
+  CKC(cudaStreamSynchronize(h->stream));
   char* base = static_cast<char*>(h->d_block);
   h->tv.rows = reinterpret_cast<unsigned char*>(base);
   h->tv.bits = reinterpret_cast<unsigned int*>(base + bytes_rows);
@@ -1668,14 +1673,17 @@ int mccfr_set_hand_table(mccfr_handle* h, const int32_t* table, size_t n) {
   CK(cudaSetDevice(h->device));
   const size_t bytes = n * sizeof(int32_t);
   if (!h->d_hr) CK(cudaMalloc(&h->d_hr, bytes));
-  CK(cudaMemcpy(h->d_hr, table, bytes, cudaMemcpyHostToDevice));
+  // copied on the stream whose kernels read it, and waited for (other handles'
+  // streams may read it too)
+  CK(cudaMemcpyAsync(h->d_hr, table, bytes, cudaMemcpyHostToDevice, h->stream));
+  CK(cudaStreamSynchronize(h->stream));
   // Rank-CDF bucket LUTs from exact histograms.
   if (h->cfg.postflop_mode == MCCFR_POSTFLOP_RANK_CDF) {
     unsigned long long* d_hist = nullptr;
     CK(cudaMalloc(&d_hist, 7463 * sizeof(unsigned long long)));
     uint8_t lut[3][7463];
     for (int s = 0; s < 3; ++s) {
-      CK(cudaMemset(d_hist, 0, 7463 * sizeof(unsigned long long)));
+      CK(cudaMemsetAsync(d_hist, 0, 7463 * sizeof(unsigned long long), h->stream));
       k_rank_hist<<<(52 * 52 * 52 + 127) / 128, 128, 0, h->stream>>>(h->d_hr, 5 + s, d_hist);
       CK(cudaGetLastError());
       unsigned long long hist[7463];
@@ -1684,7 +1692,7 @@ int mccfr_set_hand_table(mccfr_handle* h, const int32_t* table, size_t n) {
       build_cdf_lut(hist, h->cfg.postflop_buckets[s], lut[s]);
     }
     cudaFree(d_hist);
-    CK(cudaMemcpy(h->d_cdf, lut, sizeof(lut), cudaMemcpyHostToDevice));
+    CK(cudaMemcpyAsync(h->d_cdf, lut, sizeof(lut), cudaMemcpyHostToDevice, h->stream));
     k_state_buckets<<<148 * 8, 256, 0, h->stream>>>(h->d_hr, h->d_cdf);
     CK(cudaGetLastError());
     CK(cudaStreamSynchronize(h->stream));
@@ -2555,9 +2563,11 @@ int mccfr_batch_create(mccfr_handle* const* tables, int n, const int* traversals
       cudaMalloc(&b->d_work, b->max_players * sizeof(unsigned long long)) != cudaSuccess ||
       cudaMalloc(&b->d_deals, b->max_items * sizeof(DealRec)) != cudaSuccess)
     return bad(MCCFR_ERR_OOM, "batch buffers");
-  if (cudaMemcpy(b->d_tables, descs.data(), n * sizeof(TableDesc), cudaMemcpyHostToDevice) != cudaSuccess ||
-      cudaMemcpy(b->d_phases, b->phases.data(), b->max_players * sizeof(PhaseDesc), cudaMemcpyHostToDevice) !=
-          cudaSuccess)
+  if (cudaMemcpyAsync(b->d_tables, descs.data(), n * sizeof(TableDesc), cudaMemcpyHostToDevice, b->stream) !=
+          cudaSuccess ||
+      cudaMemcpyAsync(b->d_phases, b->phases.data(), b->max_players * sizeof(PhaseDesc), cudaMemcpyHostToDevice,
+                      b->stream) != cudaSuccess ||
+      cudaStreamSynchronize(b->stream) != cudaSuccess)
     return bad(MCCFR_ERR_CUDA, "batch upload");
   *out = b;
   return MCCFR_OK;
@@ -2880,7 +2890,8 @@ int mccfr_create_subgame(const mccfr_config* cfg, const mccfr_subgame* sg, mccfr
   mccfr_handle* h = *out;
   // room for any player count, so a reset can take a different one
   if (cudaMalloc(&h->d_ranges, (size_t)MCCFR_MAX_PLAYERS * 1326 * 4) != cudaSuccess ||
-      cudaMemcpy(h->d_ranges, cdf.data(), cdf.size() * 4, cudaMemcpyHostToDevice) != cudaSuccess) {
+      cudaMemcpyAsync(h->d_ranges, cdf.data(), cdf.size() * 4, cudaMemcpyHostToDevice, h->stream) != cudaSuccess ||
+      cudaStreamSynchronize(h->stream) != cudaSuccess) {
     mccfr_destroy(h);
     *out = nullptr;
     return MCCFR_ERR_OOM;
@@ -2931,7 +2942,8 @@ int mccfr_share_hand_table(mccfr_handle* h, mccfr_handle* src) {
     if (src->cfg.postflop_mode != MCCFR_POSTFLOP_RANK_CDF ||
         std::memcmp(src->cfg.postflop_buckets, h->cfg.postflop_buckets, sizeof(h->cfg.postflop_buckets)))
       return fail(h, MCCFR_ERR_INVALID_ARG, "rank-CDF buckets differ from the source table's");
-    CK(cudaMemcpy(h->d_cdf, src->d_cdf, kCdfBytes, cudaMemcpyDeviceToDevice));
+    CK(cudaMemcpyAsync(h->d_cdf, src->d_cdf, kCdfBytes, cudaMemcpyDeviceToDevice, h->stream));
+    CK(cudaStreamSynchronize(h->stream));
   }
   if (h->d_hr && !h->shared_hr) cudaFree(h->d_hr);
   h->d_hr = src->d_hr;
