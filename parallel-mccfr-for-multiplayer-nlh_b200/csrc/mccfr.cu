@@ -25,6 +25,7 @@
 #include <vector>
 
 #include "../../include/mccfr.h"
+#include "block_pool.h"
 #include "game.cuh"
 #include "handtable.h"
 #include "table.cuh"
@@ -639,8 +640,7 @@ struct mccfr_handle {
   LevelBufs lb{};
   int grid_expand = 0, grid_back = 0, grid_dfs = 0;  // resident blocks on this handle's device
   // walk form: every resident warp's node records, and the update's counters
-  void* d_walk = nullptr;
-  int walk_blocks = 0;    // blocks the records were allocated for
+  BlockPool walk;
   int walk_resident = 0;  // resident blocks on this handle's device
   int path_resident = 0;  // the same for the reference rule's kernel
   bool last_walk = false;  // the last external-sampling update ran in the walk form
@@ -997,7 +997,7 @@ void drop_graph(mccfr_handle* h) {
 
 // Node records of the walk form's warps: as many blocks as are resident, or as
 // the batch has traversals for.  Fewer are tried when the device is short of
-// memory; any number gives the same rows.
+// memory (BlockPool); any number gives the same rows.
 int ensure_walk(mccfr_handle* h, int batch) {
   if (!h->walk_resident) {
     int sms = 0, per = 0;
@@ -1007,27 +1007,14 @@ int ensure_walk(mccfr_handle* h, int batch) {
   }
   const int want = std::min(h->walk_resident, (batch + kWalkWarps - 1) / kWalkWarps);
   h->wb.decisions = max_decisions(h);
-  if (h->d_walk && h->walk_blocks >= want) return MCCFR_OK;
-  if (h->d_walk) {
-    CK(cudaStreamSynchronize(h->stream));
-    cudaFree(h->d_walk);
-    h->d_walk = nullptr;
-    h->walk_blocks = 0;
-  }
+  if (h->walk.holds(want)) return MCCFR_OK;
+  if (h->walk.p) CK(cudaStreamSynchronize(h->stream));
   drop_graph(h);  // the graph captured the old buffers
-  for (int blocks = want;; blocks = (blocks + 1) / 2) {
-    const size_t nodes = (size_t)blocks * kWalkWarps * kWalkNodes;
-    const cudaError_t e = cudaMalloc(&h->d_walk, nodes * sizeof(WalkNode) + sizeof(WalkCtl));
-    if (e == cudaSuccess) {
-      h->wb.nodes = static_cast<WalkNode*>(h->d_walk);
-      h->wb.ctl = reinterpret_cast<WalkCtl*>(h->wb.nodes + nodes);
-      h->walk_blocks = blocks;
-      return MCCFR_OK;
-    }
-    cudaGetLastError();  // clear the allocation error
-    if (e != cudaErrorMemoryAllocation || blocks == 1)
-      return fail(h, MCCFR_ERR_OOM, "walk buffers: %s", cudaGetErrorString(e));
-  }
+  const cudaError_t e = h->walk.take(want, kWalkWarps * kWalkNodes * sizeof(WalkNode), sizeof(WalkCtl));
+  if (e != cudaSuccess) return fail(h, MCCFR_ERR_OOM, "walk buffers: %s", cudaGetErrorString(e));
+  h->wb.nodes = static_cast<WalkNode*>(h->walk.p);
+  h->wb.ctl = reinterpret_cast<WalkCtl*>(h->wb.nodes + (size_t)h->walk.blocks * kWalkWarps * kWalkNodes);
+  return MCCFR_OK;
 }
 
 // Buffers of the handle's external-sampling form for updates of `batch` traversals.
@@ -1061,7 +1048,7 @@ int enqueue_path(mccfr_handle* h, int batch, const DealRec* deals, float rscale,
 int enqueue_walk(mccfr_handle* h, int batch, const DealRec* deals, float rscale) {
   h->last_walk = true;
   h->level_last_batch = batch;
-  const int blocks = std::min(h->walk_blocks, (batch + kWalkWarps - 1) / kWalkWarps);
+  const int blocks = std::min(h->walk.blocks, (batch + kWalkWarps - 1) / kWalkWarps);
   WalkBufs wb = h->wb;
   // a warp takes up to 32 roots at a time, fewer while that would leave other
   // warps of the launch without
@@ -1429,7 +1416,7 @@ void release(mccfr_handle* h) {
   cudaFree(h->d_counters);
   cudaFree(h->d_work);
   cudaFree(h->d_level);
-  cudaFree(h->d_walk);
+  h->walk.free();
   cudaFree(h->d_scratch);
   cudaFree(h->d_spans);
   if (h->stream) cudaStreamDestroy(h->stream);
@@ -2245,7 +2232,7 @@ int mccfr_level_counts(mccfr_handle* h, uint32_t* seeds, uint32_t* nodes, int ca
   if (!h || !levels || cap < 0 || (cap && (!seeds || !nodes))) return MCCFR_ERR_INVALID_ARG;
   *levels = 0;
   if (deferred) *deferred = 0;
-  if (h->last_walk ? !h->d_walk : !h->d_level) return MCCFR_OK;
+  if (h->last_walk ? !h->walk.p : !h->d_level) return MCCFR_OK;
   CK(cudaSetDevice(h->device));
   if (h->last_walk) {
     WalkCtl w;
