@@ -22,7 +22,7 @@ ORACLE_DIR = ROOT / "oracle"
 SOURCES = ["mccfr.cu", "eval_static.cu", "best_response.cu", "handtable.cpp", "abstraction.cpp"]
 HEADERS = ["game.cuh", "table.cuh", "traverse_ref.cuh", "traverse_es.cuh", "traverse_levels.cuh",
            "traverse_walk.cuh", "traverse_path.cuh", "showdown.cuh", "batched.cuh",
-           "block_pool.h", "handtable.h", "best_response.h"]
+           "block_pool.h", "round_buffers.h", "handtable.h", "best_response.h"]
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a",

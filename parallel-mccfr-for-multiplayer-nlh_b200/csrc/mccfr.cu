@@ -28,6 +28,7 @@
 #include "block_pool.h"
 #include "game.cuh"
 #include "handtable.h"
+#include "round_buffers.h"
 #include "table.cuh"
 #include "traverse_ref.cuh"
 #include "traverse_es.cuh"
@@ -2751,28 +2752,22 @@ struct RoundUpload {
 // One device's round buffers.  They are shared by every trainer of the device
 // (rounds take turns) and freed with the device's last handle.
 struct RoundCtx {
-  cudaStream_t stream = nullptr;
-  RoundUpload* h_up = nullptr;  // pinned
-  RoundUpload* d_up = nullptr;
-  int* h_err = nullptr;  // pinned: the tables' error flags after a round
-  int* d_err = nullptr;
+  RoundParts parts;
   DealRec* d_deals = nullptr;
   size_t deals_cap = 0;
   WalkNode* d_nodes = nullptr;  // walk form: node records of `blocks` blocks
   int blocks = 0, resident = 0;
   PhaseParams params;  // persistent form: descriptors by value
 
+  RoundUpload* h_up() const { return static_cast<RoundUpload*>(parts.h_up); }
+  RoundUpload* d_up() const { return static_cast<RoundUpload*>(parts.d_up); }
+  int* h_err() const { return static_cast<int*>(parts.h_err); }  // the tables' error flags after a round
+  int* d_err() const { return static_cast<int*>(parts.d_err); }
+
   void free_all() {
-    if (stream) cudaStreamDestroy(stream);
-    cudaFreeHost(h_up);
-    cudaFree(d_up);
-    cudaFreeHost(h_err);
-    cudaFree(d_err);
+    parts.free_all();
     cudaFree(d_deals);
     cudaFree(d_nodes);
-    stream = nullptr;
-    h_up = d_up = nullptr;
-    h_err = d_err = nullptr;
     d_deals = nullptr;
     d_nodes = nullptr;
     deals_cap = 0;
@@ -2966,13 +2961,8 @@ int mccfr_batch_round(mccfr_handle* const* tables, int n, const int* traversals,
   RoundCtx& R = g_round[dev];
   mccfr_batch* b = nullptr;  // for BCK error reporting
   BCK(cudaSetDevice(dev));
-  if (!R.stream) {
-    BCK(cudaStreamCreateWithFlags(&R.stream, cudaStreamNonBlocking));
-    BCK(cudaMalloc(&R.d_up, sizeof(RoundUpload)));
-    BCK(cudaMallocHost(&R.h_up, sizeof(RoundUpload)));
-    BCK(cudaMalloc(&R.d_err, kMaxBatchTables * sizeof(int)));
-    BCK(cudaMallocHost(&R.h_err, kMaxBatchTables * sizeof(int)));
-  }
+  BCK(R.parts.make(sizeof(RoundUpload), kMaxBatchTables * sizeof(int)));
+  const cudaStream_t stream = R.parts.stream;
   unsigned long long total = 0;
   for (int i = 0; i < n; ++i) total += (unsigned long long)traversals[i];
   if (total > R.deals_cap) {
@@ -3009,7 +2999,7 @@ int mccfr_batch_round(mccfr_handle* const* tables, int n, const int* traversals,
       R.blocks = blocks;
     }
   }
-  RoundUpload& U = *R.h_up;
+  RoundUpload& U = *R.h_up();
   PhaseDesc& P = U.phase;
   unsigned long long off = 0;
   unsigned words = 1;
@@ -3021,7 +3011,7 @@ int mccfr_batch_round(mccfr_handle* const* tables, int n, const int* traversals,
     d.tv = h->tv;
     d.pre = h->d_pre;
     d.cdf = h->d_cdf;
-    d.sched = &R.d_up->sched[i];
+    d.sched = &R.d_up()->sched[i];
     d.counters = h->d_counters;
     const int rb = regret_frac_bits(h->cfg, traversals[i]);
     d.rscale = std::ldexp(1.0f, rb);
@@ -3039,13 +3029,13 @@ int mccfr_batch_round(mccfr_handle* const* tables, int n, const int* traversals,
   P.n = n;
   P.off[n] = off;
   U.persistent_work = 0;
-  BCK(cudaMemcpyAsync(R.d_up, R.h_up, sizeof(RoundUpload), cudaMemcpyHostToDevice, R.stream));
-  BCK(launch_deals(R.d_up->tables, &R.d_up->phase, tables[0]->d_hr, R.d_deals, off, full, sub, R.stream));
+  BCK(cudaMemcpyAsync(R.parts.d_up, R.parts.h_up, sizeof(RoundUpload), cudaMemcpyHostToDevice, stream));
+  BCK(launch_deals(R.d_up()->tables, &R.d_up()->phase, tables[0]->d_hr, R.d_deals, off, full, sub, stream));
   if (walk) {
     // any mix of tables runs the general kernel; direct-mapped tables of path-hash
     // keys, as subgames are, the one without probing and FNV slots
     auto kern = direct && !fnv ? k_walk_round<true, false> : k_walk_round<false, true>;
-    kern<<<blocks, kWalkBlock, 0, R.stream>>>(R.d_up->tables, n, R.d_deals, R.d_nodes, R.d_up->work);
+    kern<<<blocks, kWalkBlock, 0, stream>>>(R.d_up()->tables, n, R.d_deals, R.d_nodes, R.d_up()->work);
     BCK(cudaGetLastError());
   } else {
     PhaseParams& Q = R.params;
@@ -3062,16 +3052,17 @@ int mccfr_batch_round(mccfr_handle* const* tables, int n, const int* traversals,
     const unsigned long long need = (off + t.block - 1) / t.block;
     const int grid = (int)std::max<unsigned long long>(
         1, std::min<unsigned long long>(need, (unsigned long long)std::max(1, per_sm) * sms));
-    kern<<<grid, t.block, smem, R.stream>>>(Q, R.d_deals, &R.d_up->persistent_work, t.grab, t.warp_sync);
+    kern<<<grid, t.block, smem, stream>>>(Q, R.d_deals, &R.d_up()->persistent_work, t.grab, t.warp_sync);
     BCK(cudaGetLastError());
   }
   // a warp of the apply kernel per four bitmap words of the largest table
   const int ablocks = (int)std::min(148u, (words + 31) / 32);
-  k_apply_batched<<<dim3(std::max(1, ablocks), n), kApplyBlock, 0, R.stream>>>(R.d_up->tables, &R.d_up->phase, R.d_err);
+  k_apply_batched<<<dim3(std::max(1, ablocks), n), kApplyBlock, 0, stream>>>(R.d_up()->tables, &R.d_up()->phase,
+                                                                             R.d_err());
   BCK(cudaGetLastError());
   // every table's error flag in one copy
-  BCK(cudaMemcpyAsync(R.h_err, R.d_err, n * sizeof(int), cudaMemcpyDeviceToHost, R.stream));
-  BCK(cudaStreamSynchronize(R.stream));
+  BCK(cudaMemcpyAsync(R.h_err(), R.d_err(), n * sizeof(int), cudaMemcpyDeviceToHost, stream));
+  BCK(cudaStreamSynchronize(stream));
   int worst = MCCFR_OK;
   for (int i = 0; i < n; ++i) {
     mccfr_handle* h = tables[i];
@@ -3080,7 +3071,7 @@ int mccfr_batch_round(mccfr_handle* const* tables, int n, const int* traversals,
       h->round_player = 0;
       h->iterations_done++;
     }
-    if (R.h_err[i]) {
+    if (R.h_err()[i]) {
       const int rc = check_device_error(h);
       if (rc && !worst) worst = rc;
     }
