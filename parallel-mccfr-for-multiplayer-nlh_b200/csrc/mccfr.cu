@@ -2755,8 +2755,8 @@ struct RoundCtx {
   RoundParts parts;
   DealRec* d_deals = nullptr;
   size_t deals_cap = 0;
-  WalkNode* d_nodes = nullptr;  // walk form: node records of `blocks` blocks
-  int blocks = 0, resident = 0;
+  BlockPool nodes;  // walk form: node records
+  int resident = 0;
   PhaseParams params;  // persistent form: descriptors by value
 
   RoundUpload* h_up() const { return static_cast<RoundUpload*>(parts.h_up); }
@@ -2767,11 +2767,9 @@ struct RoundCtx {
   void free_all() {
     parts.free_all();
     cudaFree(d_deals);
-    cudaFree(d_nodes);
+    nodes.free();
     d_deals = nullptr;
-    d_nodes = nullptr;
     deals_cap = 0;
-    blocks = 0;
   }
 };
 
@@ -2991,13 +2989,8 @@ int mccfr_batch_round(mccfr_handle* const* tables, int n, const int* traversals,
       R.resident = std::max(1, per) * sms;
     }
     blocks = (int)std::min<unsigned long long>(R.resident, (total + kWalkWarps - 1) / kWalkWarps);
-    if (blocks > R.blocks) {
-      cudaFree(R.d_nodes);
-      R.d_nodes = nullptr;
-      R.blocks = 0;
-      BCK(cudaMalloc(&R.d_nodes, (size_t)blocks * kWalkWarps * kWalkNodes * sizeof(WalkNode)));
-      R.blocks = blocks;
-    }
+    if (!R.nodes.holds(blocks)) BCK(R.nodes.take(blocks, kWalkWarps * kWalkNodes * sizeof(WalkNode), 0));
+    blocks = std::min(blocks, R.nodes.blocks);  // fewer on a device short of memory: the same rows
   }
   RoundUpload& U = *R.h_up();
   PhaseDesc& P = U.phase;
@@ -3035,7 +3028,8 @@ int mccfr_batch_round(mccfr_handle* const* tables, int n, const int* traversals,
     // any mix of tables runs the general kernel; direct-mapped tables of path-hash
     // keys, as subgames are, the one without probing and FNV slots
     auto kern = direct && !fnv ? k_walk_round<true, false> : k_walk_round<false, true>;
-    kern<<<blocks, kWalkBlock, 0, stream>>>(R.d_up()->tables, n, R.d_deals, R.d_nodes, R.d_up()->work);
+    kern<<<blocks, kWalkBlock, 0, stream>>>(R.d_up()->tables, n, R.d_deals, static_cast<WalkNode*>(R.nodes.p),
+                                             R.d_up()->work);
     BCK(cudaGetLastError());
   } else {
     PhaseParams& Q = R.params;

@@ -44,3 +44,38 @@ def test_rounds_whose_tables_run_out_while_warps_enter(hand_table, tables, most)
         assert a.stats().node_visits == b.stats().node_visits
     for t in plain[::-1] + rounds[::-1]:
         t.close()
+
+
+def test_a_round_on_a_device_short_of_memory(hand_table):
+    """Node records for every resident warp do not fit: the round runs with fewer."""
+    import torch
+
+    cfgs = [_game(2, 14, 70), _game(6, 14, 71)]
+    counts = [9000, 3000]
+    rounds, plain = _make(cfgs, hand_table), _make(cfgs, hand_table)
+    mccfr.batch_round(rounds, [3, 3])  # kernels loaded
+    mccfr.batch_round(rounds, counts, {"block": 128})  # deals sized, by the form without node records
+    for t, c, n in zip(plain, cfgs, counts):
+        t.step(1, 0, 3)
+        t.step(1, 1, n)
+        t.step(1 + 2 // c.num_players, 2 % c.num_players, n)
+    torch.cuda.init()
+    held, chunk, left = [], 1 << 30, 32 << 20
+    while chunk >= 8 << 20:
+        if torch.cuda.mem_get_info()[0] < left + chunk:
+            chunk //= 2
+            continue
+        try:
+            held.append(torch.empty(chunk, dtype=torch.uint8, device="cuda"))
+        except torch.OutOfMemoryError:
+            chunk //= 2
+    assert torch.cuda.mem_get_info()[0] < 64 << 20  # 87 MB of records do not fit
+    try:
+        mccfr.batch_round(rounds, counts)
+    finally:
+        held.clear()
+        torch.cuda.empty_cache()
+    for a, b in zip(rounds, plain):
+        assert a.digest() == b.digest()
+    for t in plain[::-1] + rounds[::-1]:
+        t.close()
