@@ -1302,19 +1302,16 @@ void order_by_key(const std::vector<unsigned long long>& k, std::vector<unsigned
   }
 }
 
-// The rows that count_read counted last (kReadRows or kReadStrategy, `n` of them),
-// in ascending key order, into host arrays; null arrays are skipped.  `sums`
-// receives strategy sums or strategies.
-int fetch_rows(mccfr_handle* h, int what, unsigned n, uint64_t* keys, uint32_t* keys32, float* regrets, float* sums,
-               uint64_t* visits) {
-  if (n == 0) return MCCFR_OK;
+// The rows that count_read counted last (kReadRows or kReadStrategy, `n` of them), in
+// slot order, into host arrays; null arrays are skipped.  `sums` receives strategy
+// sums or strategies.
+int fetch_slots(mccfr_handle* h, int what, unsigned n, unsigned long long* keys, uint32_t* keys32, float* regrets,
+                float* sums, unsigned long long* visits) {
   const unsigned long long rows = std::min(h->cap, (unsigned long long)h->tv.n_words * 32);
   const unsigned spans = (unsigned)((rows + kReadSpan - 1) / kReadSpan);
-  const bool sort = !h->tv.direct;  // slots of an open-addressed table are in no order
-  const bool k64 = keys || sort;
   Scratch scratch(h);
-  const size_t bytes = (size_t)n * ((regrets ? 32 : 0) + (sums ? 32 : 0) + (k64 ? 8 : 0) + (visits ? 8 : 0) +
-                                    (keys32 && !sort ? 4 : 0));
+  const size_t bytes = (size_t)n * ((regrets ? 32 : 0) + (sums ? 32 : 0) + (keys ? 8 : 0) + (visits ? 8 : 0) +
+                                    (keys32 ? 4 : 0));
   const cudaError_t e0 = scratch.take(bytes);
   if (e0 != cudaSuccess) {
     cudaGetLastError();
@@ -1330,9 +1327,9 @@ int fetch_rows(mccfr_handle* h, int what, unsigned n, uint64_t* keys, uint32_t* 
   ReadOut out{};
   out.regrets = static_cast<Sector*>(carve(regrets, 32));
   out.sums = static_cast<Sector*>(carve(sums, 32));
-  out.keys = static_cast<unsigned long long*>(carve(k64, 8));
+  out.keys = static_cast<unsigned long long*>(carve(keys, 8));
   out.visits = static_cast<unsigned long long*>(carve(visits, 8));
-  out.keys32 = static_cast<unsigned*>(carve(keys32 && !sort, 4));
+  out.keys32 = static_cast<unsigned*>(carve(keys32, 4));
   out.key32_sub = h->cfg.key_mode == MCCFR_KEY_FNV26 ? 1u : 0u;
   if (what == kReadRows) k_read_write<kReadRows><<<spans, kReadBlock, 0, h->stream>>>(h->tv, h->d_spans, out);
   else k_read_write<kReadStrategy><<<spans, kReadBlock, 0, h->stream>>>(h->tv, h->d_spans, out);
@@ -1340,28 +1337,36 @@ int fetch_rows(mccfr_handle* h, int what, unsigned n, uint64_t* keys, uint32_t* 
   const auto copy = [&](void* dst, const void* src, size_t width) {
     return dst ? cudaMemcpyAsync(dst, src, width * n, cudaMemcpyDeviceToHost, h->stream) : cudaSuccess;
   };
-  if (!sort) {
-    CK(copy(keys, out.keys, 8));
-    CK(copy(keys32, out.keys32, 4));
-    CK(copy(regrets, out.regrets, 32));
-    CK(copy(sums, out.sums, 32));
-    CK(copy(visits, out.visits, 8));
-    CK(cudaStreamSynchronize(h->stream));
-    return MCCFR_OK;
-  }
+  CK(copy(keys, out.keys, 8));
+  CK(copy(keys32, out.keys32, 4));
+  CK(copy(regrets, out.regrets, 32));
+  CK(copy(sums, out.sums, 32));
+  CK(copy(visits, out.visits, 8));
+  CK(cudaStreamSynchronize(h->stream));
+  return MCCFR_OK;
+}
+
+// The same in ascending key order: slot order in a direct-mapped table; the slots of an
+// open-addressed one are in no order and their rows are sorted on the host.
+int fetch_rows(mccfr_handle* h, int what, unsigned n, uint64_t* keys, uint32_t* keys32, float* regrets, float* sums,
+               uint64_t* visits) {
+  if (n == 0) return MCCFR_OK;
+  static_assert(sizeof(uint64_t) == sizeof(unsigned long long), "one 64-bit word");
+  if (h->tv.direct)
+    return fetch_slots(h, what, n, reinterpret_cast<unsigned long long*>(keys), keys32, regrets, sums,
+                       reinterpret_cast<unsigned long long*>(visits));
   std::vector<unsigned long long> k(n), v(visits ? n : 0);
   std::vector<float> r(regrets ? 8ull * n : 0), q(sums ? 8ull * n : 0);
-  CK(copy(k.data(), out.keys, 8));
-  CK(copy(visits ? v.data() : nullptr, out.visits, 8));
-  CK(copy(regrets ? r.data() : nullptr, out.regrets, 32));
-  CK(copy(sums ? q.data() : nullptr, out.sums, 32));
-  CK(cudaStreamSynchronize(h->stream));
+  const int rc = fetch_slots(h, what, n, k.data(), nullptr, regrets ? r.data() : nullptr, sums ? q.data() : nullptr,
+                             visits ? v.data() : nullptr);
+  if (rc) return rc;
   std::vector<unsigned> order;
   order_by_key(k, order);
+  const unsigned sub = h->cfg.key_mode == MCCFR_KEY_FNV26 ? 1u : 0u;
   for (unsigned j = 0; j < n; ++j) {
     const unsigned i = order[j];
     if (keys) keys[j] = k[i];
-    if (keys32) keys32[j] = (uint32_t)k[i] - out.key32_sub;
+    if (keys32) keys32[j] = (uint32_t)k[i] - sub;
     if (visits) visits[j] = v[i];
     if (regrets) std::memcpy(regrets + 8ull * j, &r[8ull * i], 32);
     if (sums) std::memcpy(sums + 8ull * j, &q[8ull * i], 32);
@@ -1375,16 +1380,21 @@ int read_host_rows(mccfr_handle* h, std::vector<HostRow>& rows) {
   unsigned n = 0;
   int rc = count_read(h, kReadRows, &n);
   if (rc) return rc;
-  std::vector<uint64_t> keys(n), vis(n);
-  std::vector<float> reg(8ull * n), ssum(8ull * n);
-  rc = fetch_rows(h, kReadRows, n, keys.data(), nullptr, reg.data(), ssum.data(), vis.data());
+  rows.clear();
+  if (n == 0) return MCCFR_OK;
+  std::vector<unsigned long long> k(n), v(n);
+  std::vector<float> r(8ull * n), q(8ull * n);
+  rc = fetch_slots(h, kReadRows, n, k.data(), nullptr, r.data(), q.data(), v.data());
   if (rc) return rc;
+  std::vector<unsigned> order;
+  if (!h->tv.direct) order_by_key(k, order);
   rows.resize(n);
-  for (unsigned i = 0; i < n; ++i) {
-    rows[i].key = keys[i];
-    std::memcpy(rows[i].reg, &reg[8ull * i], 32);
-    std::memcpy(rows[i].ssum, &ssum[8ull * i], 32);
-    rows[i].visits = vis[i];
+  for (unsigned j = 0; j < n; ++j) {
+    const unsigned i = h->tv.direct ? j : order[j];
+    rows[j].key = k[i];
+    std::memcpy(rows[j].reg, &r[8ull * i], 32);
+    std::memcpy(rows[j].ssum, &q[8ull * i], 32);
+    rows[j].visits = v[i];
   }
   return MCCFR_OK;
 }
