@@ -104,10 +104,21 @@ def request_config(req: Request) -> L.Config:
     return c
 
 
+def capacity_bytes(table_log2: int) -> int:
+    """Device bytes that a re-solve handle of this capacity may hold: per row 256 of
+    the table, 1/4 of the touched-row bitmaps and the read-back scratch that the
+    handle keeps (36 bytes per exported row and a quarter more, over the half of the
+    rows that keys can own: 22.5 bytes), rounded up to 280; and 6 MB for the bucket
+    LUTs, the smallest scratch and other small buffers, and for the allocator's
+    rounding of table and scratch to 2 MB each.  Buffers that all rounds of a device
+    share (87 MB of node records, 64 bytes per traversal of a round) are not a
+    table's and are not counted."""
+    return (1 << table_log2) * 280 + (6 << 20)
+
+
 def table_bytes(req: Request) -> int:
-    """Device bytes a request's table is counted as: 256-byte rows with 4 bytes each
-    for bitmaps and read-back, plus its small buffers."""
-    return (1 << req.table_log2) * (256 + 4) + (1 << 20)
+    """Device bytes a request's table is counted as."""
+    return capacity_bytes(req.table_log2)
 
 
 @dataclass
@@ -204,7 +215,7 @@ class ReSolveServer:
         return int(torch.cuda.mem_get_info()[0])
 
     def pooled_bytes(self) -> int:
-        return sum((1 << log2) * (256 + 4) + (1 << 20) for log2, ts in self.pool.items() for _ in ts)
+        return sum(capacity_bytes(log2) * len(ts) for log2, ts in self.pool.items())
 
     def _evict(self, need: int, held: int) -> None:
         """Frees pooled tables of other capacities until `need` more bytes fit."""
