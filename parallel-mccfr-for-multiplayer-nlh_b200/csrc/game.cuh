@@ -28,7 +28,7 @@ struct GameParams {
   const uint32_t* range_cdf;    // [N][1326] cumulative range weights, 2^31 scale
   // action slots
   int8_t kind[kSlots];
-  int16_t num[kSlots];
+  int16_t num[kSlots], den[kSlots];  // den 0: not a pot raise
   uint8_t m_fold, m_check, m_call, m_allin, m_raise, m_check_kind;
   uint8_t n_fallback;
   uint8_t fallback[kSlots];
@@ -141,14 +141,21 @@ __host__ __device__ __forceinline__ void frac_factors(int den, uint32_t& mul, ui
   sh = (uint8_t)l;
 }
 
+// Makes action slot a a raise of num / den of the pot.
+__host__ __device__ __forceinline__ void set_pot_fraction(GameParams& G, int a, int num, int den) {
+  G.num[a] = (int16_t)num;
+  G.den[a] = (int16_t)imax(1, den);
+  frac_factors(G.den[a], G.frac_mul[a], G.frac_sh[a]);
+}
+
 __host__ __device__ __forceinline__ int raise_target(const GameParams& G, int a, int pot, int cb, int mrt) {
-  const uint32_t x = 2u * (uint32_t)(G.num[a] * pot);
 #ifdef __CUDA_ARCH__
-  const uint32_t q = __umulhi(x, G.frac_mul[a]);
+  const int frac = (int)(__umulhi(2u * (uint32_t)(G.num[a] * pot), G.frac_mul[a]) >> G.frac_sh[a]);
 #else
-  const uint32_t q = (uint32_t)(((uint64_t)x * G.frac_mul[a]) >> 32);
+  // the host's best response takes pots beyond the multiplier's range
+  const int frac = G.den[a] > 0 ? G.num[a] * pot / G.den[a] : 0;
 #endif
-  return imax(mrt, cb + imax(1, (int)(q >> G.frac_sh[a])));
+  return imax(mrt, cb + imax(1, frac));
 }
 
 __host__ __device__ __forceinline__ uint32_t valid_mask(const GameParams& G, int pot, int stack, int to_call,

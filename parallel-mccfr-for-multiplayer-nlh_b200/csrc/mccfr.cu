@@ -792,7 +792,7 @@ void make_params(const mccfr_config& c, GameParams& g) {
     if (k == MCCFR_ACT_RAISE_MIN || k == MCCFR_ACT_RAISE_POT) {
       g.m_raise |= 1u << a;
       g.raise_slot[g.n_raise++] = (uint8_t)a;
-      if (k == MCCFR_ACT_RAISE_POT) frac_factors((int16_t)std::max(1, c.action_den[a]), g.frac_mul[a], g.frac_sh[a]);
+      if (k == MCCFR_ACT_RAISE_POT) set_pot_fraction(g, a, c.action_num[a], c.action_den[a]);
     }
   }
   // Passive fallback order (cfr_gpu.cu:498-508): check, check/call, call, fold,
