@@ -76,6 +76,18 @@ def make_config(L, workload: str, rank: int = 0):
     return cfg, batch
 
 
+def traversal_form(cfg) -> str:
+    """The kernels that a config's updates run: the default form walks while a path
+    holds at most 31 decisions of the updating player (raise_cap + 1 per street, or
+    the depth cut's nodes), and takes the level kernels for longer ones."""
+    if cfg.sampling != 1:
+        return "reference"
+    if cfg.traversal_form == 0:
+        decisions = min(cfg.max_depth, 4 * (cfg.raise_cap + 1)) if cfg.raise_cap > 0 else cfg.max_depth
+        return "walk" if decisions < 32 else "levels"
+    return "lanes" if cfg.traversal_form == 1 else "levels"
+
+
 def apply_roofline(s0, s1, launches: int, peak: float, row_bytes: float = 420.0, wide_bytes: float = 96.0) -> dict:
     """The apply kernel's share of a step against the HBM roofline, at `row_bytes`
     per touched row and `wide_bytes` more per row of the updating player; rows
@@ -898,8 +910,7 @@ def main():
     achieved = bytes_per_launch / (kernel_ms / 1e3) / 1e9 if kernel_ms else None
     has_levels = isinstance(levels, dict) and "seeds" in levels
     nlev = len(levels["seeds"]) if has_levels else 0
-    form_name = ("reference" if cfg.sampling != 1 else "lanes" if cfg.traversal_form == 1
-                 else "levels" if cfg.traversal_form == 2 else "walk")
+    form_name = traversal_form(cfg)
     tr_prof = profiled_traffic(args.workload, form_name)
     traffic = None
     if tr_prof and "dram_bytes_per_node_visit" in tr_prof:
