@@ -88,20 +88,22 @@ def traversal_form(cfg) -> str:
     return "lanes" if cfg.traversal_form == 1 else "levels"
 
 
-def apply_roofline(s0, s1, launches: int, peak: float, row_bytes: float = 420.0, wide_bytes: float = 96.0) -> dict:
+def apply_roofline(s0, s1, launches: int, peak: float, row_bytes: float = 420.0, wide_bytes: float = 96.0,
+                   last: bool = False) -> dict:
     """The apply kernel's share of a step against the HBM roofline, at `row_bytes`
-    per touched row and `wide_bytes` more per row of the updating player; rows
-    counted on the device for the last player-update.  The defaults are a whole
+    per touched row and `wide_bytes` more per row whose second line was folded; rows
+    counted on the device for the last player-update, over the mean time of a launch
+    or, with `last`, the time of that update's own.  The defaults are a whole
     256-byte record read, 160 bytes of it written and a 4-byte list entry, plus 96
     bytes of accumulators."""
-    ms = (s1.apply_ms - s0.apply_ms) / max(1, launches)
+    ms = s1.last_apply_ms if last else (s1.apply_ms - s0.apply_ms) / max(1, launches)
     rows = int(s1.touched_last)
     wide = int(getattr(s1, "wide_rows_last", 0))
     nbytes = rows * row_bytes + wide * wide_bytes
     gbs = nbytes / (ms / 1e3) / 1e9 if ms > 0 else None
     return {"kernel": "k_apply", "kernel_ms_per_launch": ms, "touched_rows_last_update": rows,
             "wide_rows_last_update": wide, "bytes_per_launch": nbytes,
-            "bytes_per_row": f"{row_bytes:.0f} + {wide_bytes:.0f} for the updating player's rows",
+            "bytes_per_row": f"{row_bytes:.0f} + {wide_bytes:.0f} for rows whose second line was folded",
             "achieved": gbs, "unit": "GB/s", "frac": gbs / peak if gbs else None}
 
 
@@ -948,9 +950,11 @@ def main():
                      "traffic_source": tr_prof.get("source") if tr_prof else None,
                      "algorithmic_bytes": "40*V + 96*U per launch (V node visits, U updating-player updates)",
                      "V_per_traversal": visits / max(1, trav), "U_per_traversal": updates / max(1, trav)},
-        # k_apply: a row's first 128-byte line read and two of its sectors written; for a row of the
-        # updating player its accumulators read and zeroed, its regrets and strategy written
-        "apply": apply_roofline(s0, s1, launches, peak, row_bytes=192.0, wide_bytes=192.0),
+        # k_apply: a row's first 128-byte line read, its counters and sums written (192 B); for a row of
+        # the updating player its accumulators read and zeroed and its regrets and strategy written, but
+        # most of them leave the sums as they are (160 more); the strategy weights of off-mask visits
+        # read and zeroed (128 more).  The last update's rows over the last update's time.
+        "apply": apply_roofline(s0, s1, launches, peak, row_bytes=192.0, wide_bytes=160.0, last=True),
         "table": {"rows_used": rows_used, "capacity": int(s1.table_capacity),
                   "load": rows_used / max(1, s1.table_capacity), "record_bytes": 256,
                   "span_gb": s1.table_capacity * 256 / 1e9},
