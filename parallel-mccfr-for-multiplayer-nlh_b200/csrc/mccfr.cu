@@ -150,6 +150,9 @@ __device__ __forceinline__ void fold_row(const GameParams& G, const TableView& t
   wide_rows += WIDE || has_ds ? 1u : 0u;
 }
 
+// RUNS: the table's runs of rows may be marked (TableView::runs); without, the kernel
+// keeps its registers for the rows.
+template <bool RUNS>
 __device__ __forceinline__ void apply_rows(const GameParams& G, const TableView& tv, const Sched* sched, double rinv,
                                            unsigned group, unsigned ngroups, bool leader) {
   __shared__ unsigned s_rows[kApplyBlock / 32][kApplyList];
@@ -164,18 +167,43 @@ __device__ __forceinline__ void apply_rows(const GameParams& G, const TableView&
   unsigned run = 32;
   while (run > 1 && (unsigned long long)run * ngroups > n_words) run >>= 1;
   const unsigned runs = (n_words + run - 1) / run;
-  unsigned q = group;
+  // This warp's next run.  Where runs are marked (32 words each: such a table has far
+  // more than 32 words per warp) it looks its next 32 up at once, one per lane, clears
+  // their marks and takes the marked ones in turn.
+  unsigned seen = group, marked = 0;
+  bool first = true;
+  const auto next = [&](unsigned after) -> unsigned {
+    if constexpr (RUNS) {
+      if (tv.runs) {
+        while (!marked) {
+          if (!first) seen += 32 * ngroups;
+          first = false;
+          if (seen >= runs) return runs;
+          const unsigned mine = seen + (unsigned)lane * ngroups;
+          const bool m = mine < runs && __ldcg(tv.runs + mine) != 0;
+          if (m) __stcg(tv.runs + mine, (unsigned char)0);
+          marked = __ballot_sync(0xFFFFFFFFu, m);
+        }
+        const unsigned k = __ffs((int)marked) - 1;
+        marked &= marked - 1;
+        return seen + k * ngroups;
+      }
+    }
+    return after + ngroups;
+  };
+  unsigned q = RUNS && tv.runs ? next(0) : group;
   unsigned word = q * run + lane;
   bool on = q < runs && lane < run && word < n_words;
   unsigned b = on ? __ldcg(tv.bits + word) : 0u, bw = on ? __ldcg(wide_bits + word) : 0u;
   int n_s = 0, n_w = 0;  // rows listed: sampled only, wide
-  for (; q < runs; q += ngroups) {
+  while (q < runs) {
     const unsigned cur = word;
     const unsigned cb = b & ~bw, cw = bw;
     if (b) __stcg(tv.bits + cur, 0u);
     if (bw) __stcg(wide_bits + cur, 0u);
-    word = (q + ngroups) * run + lane;
-    on = q + ngroups < runs && lane < run && word < n_words;
+    q = next(q);
+    word = q * run + lane;
+    on = q < runs && lane < run && word < n_words;
     b = on ? __ldcg(tv.bits + word) : 0u;
     bw = on ? __ldcg(wide_bits + word) : 0u;
     const unsigned mine = (unsigned)__popc(cb) | (unsigned)__popc(cw) << 16;
@@ -232,11 +260,12 @@ struct Advance {
   int ahead;
 };
 
+template <bool RUNS>
 __global__ void __launch_bounds__(kApplyBlock) k_apply(const GameParams G, const TableView tv,
                                                        const Sched* __restrict__ sched, double rinv,
                                                        const Advance adv) {
-  apply_rows(G, tv, sched, rinv, (blockIdx.x * blockDim.x + threadIdx.x) >> 5, (gridDim.x * blockDim.x) >> 5,
-             blockIdx.x == 0 && threadIdx.x == 0);
+  apply_rows<RUNS>(G, tv, sched, rinv, (blockIdx.x * blockDim.x + threadIdx.x) >> 5, (gridDim.x * blockDim.x) >> 5,
+                   blockIdx.x == 0 && threadIdx.x == 0);
   if (!adv.sched) return;
   __shared__ bool s_last;
   __syncthreads();
@@ -259,14 +288,15 @@ __global__ void __launch_bounds__(kApplyBlock) k_apply(const GameParams G, const
 }
 
 // Apply of every table in a phase: blockIdx.y selects the table, whose error flag
-// goes to errors[blockIdx.y] (may be null).
+// goes to errors[blockIdx.y] (may be null).  RUNS: some of the tables mark runs.
+template <bool RUNS>
 __global__ void __launch_bounds__(kApplyBlock) k_apply_batched(const TableDesc* __restrict__ tables,
                                                                const PhaseDesc* __restrict__ phase,
                                                                int* __restrict__ errors) {
   const TableDesc& D = tables[phase->table[blockIdx.y]];
   if (errors && blockIdx.x == 0 && threadIdx.x == 0) errors[blockIdx.y] = *D.tv.err;
-  apply_rows(D.G, D.tv, D.sched, D.rinv, (blockIdx.x * blockDim.x + threadIdx.x) >> 5,
-             (gridDim.x * blockDim.x) >> 5, blockIdx.x == 0 && threadIdx.x == 0);
+  apply_rows<RUNS>(D.G, D.tv, D.sched, D.rinv, (blockIdx.x * blockDim.x + threadIdx.x) >> 5,
+                   (gridDim.x * blockDim.x) >> 5, blockIdx.x == 0 && threadIdx.x == 0);
 }
 
 __global__ void k_advance_batched(const TableDesc* __restrict__ tables, const PhaseDesc* __restrict__ phase) {
@@ -623,6 +653,7 @@ struct mccfr_handle {
   unsigned long long cap = 0;
   TableView tv{};
   void* d_block = nullptr;  // one allocation for the table arrays
+  unsigned char* d_runs = nullptr;  // marks of runs of rows, in a table that may need them
   size_t block_bytes = 0;
   Sched* d_sched = nullptr;
   DealRec* d_deals = nullptr;  // one record per traversal of an update
@@ -820,6 +851,7 @@ void set_direct(mccfr_handle* h) {
   const int kb = h->cfg.key_mode == MCCFR_KEY_FNV26 ? 26 : h->cfg.key_bits;
   const unsigned long long rows = h->tv.direct ? 1ull << kb : h->cap;
   h->tv.n_words = (unsigned)((rows + 31) / 32);
+  h->tv.runs = rows > kRunRows ? h->d_runs : nullptr;
 }
 
 int grid_for(long long work, int block) {
@@ -936,7 +968,8 @@ int enqueue_update(mccfr_handle* h, int batch, const DealRec* deals, mccfr_trace
   if (ev3 && record(h, ev3[1], capturing)) return MCCFR_ERR_CUDA;
   // three blocks per SM are resident; a small table has fewer bitmap words than warps
   const int blocks = (int)std::max(1u, std::min(148u * 3, (h->tv.n_words + 7) / 8));
-  k_apply<<<blocks, kApplyBlock, 0, h->stream>>>(h->gp, h->tv, h->d_sched, rinv, adv);
+  const auto apply = h->tv.runs ? k_apply<true> : k_apply<false>;
+  apply<<<blocks, kApplyBlock, 0, h->stream>>>(h->gp, h->tv, h->d_sched, rinv, adv);
   CK(cudaGetLastError());
   if (ev3 && record(h, ev3[2], capturing)) return MCCFR_ERR_CUDA;
   return MCCFR_OK;
@@ -1611,7 +1644,8 @@ int mccfr_create(const mccfr_config* cfg, mccfr_handle** out) {
   h->cap = 1ull << cfg->table_log2;
   const unsigned long long C = h->cap;
   const size_t bytes_rows = C * kRowBytes, bytes_bits = C / 4, bytes_misc = kCounterBytes;
-  h->block_bytes = bytes_rows + bytes_bits + bytes_misc;
+  const size_t bytes_runs = C > kRunRows ? C >> 10 : 0;
+  h->block_bytes = bytes_rows + bytes_bits + bytes_misc + bytes_runs;
   CKC(cudaMalloc(&h->d_block, h->block_bytes));
   // On the handle's own stream and waited for: no stream of the library waits for the
   // default one, a table of many GB takes milliseconds to clear, and rounds and
@@ -1624,6 +1658,7 @@ int mccfr_create(const mccfr_config* cfg, mccfr_handle** out) {
   char* misc = base + bytes_rows + bytes_bits;
   h->tv.counters = reinterpret_cast<unsigned int*>(misc);
   h->tv.err = reinterpret_cast<int*>(misc + kCounterBytes - 128);
+  if (bytes_runs) h->d_runs = reinterpret_cast<unsigned char*>(misc + bytes_misc);
   h->tv.mask = C - 1;
   h->tv.log2cap = cfg->table_log2;
   set_direct(h);
@@ -2407,7 +2442,10 @@ int batch_enqueue_iteration(mccfr_batch* b, bool capturing) {
     kern<<<grid, t.block, smem, b->stream>>>(b->params[p], b->d_deals, b->d_work + p, t.grab, t.warp_sync);
     BCK(cudaGetLastError());
     BCK(rec(b->ev_ph[2 * p + 1]));
-    k_apply_batched<<<dim3(148 * 2, P.n), kApplyBlock, 0, b->stream>>>(b->d_tables, b->d_phases + p, nullptr);
+    bool runs = false;
+    for (int j = 0; j < P.n; ++j) runs = runs || b->params[p].T[j].tv.runs;
+    const auto apply = runs ? k_apply_batched<true> : k_apply_batched<false>;
+    apply<<<dim3(148 * 2, P.n), kApplyBlock, 0, b->stream>>>(b->d_tables, b->d_phases + p, nullptr);
     BCK(cudaGetLastError());
     k_advance_batched<<<1, 64, 0, b->stream>>>(b->d_tables, b->d_phases + p);
     BCK(cudaGetLastError());
@@ -2982,13 +3020,14 @@ int mccfr_batch_round(mccfr_handle* const* tables, int n, const int* traversals,
   }
   // The walk form, unless the caller tunes the persistent depth-first kernel or a
   // table's config asks for another form (or has longer paths than the walk takes).
-  bool walk = !tuning, direct = true, fnv = false;
+  bool walk = !tuning, direct = true, fnv = false, runs = false;
   bool full = false, sub = false;
   for (int i = 0; i < n; ++i) {
     walk = walk && use_walk(tables[i]);
     direct = direct && tables[i]->tv.direct;
     fnv = fnv || tables[i]->cfg.key_mode == MCCFR_KEY_FNV26;
     (tables[i]->gp.sub_street ? sub : full) = true;
+    runs = runs || tables[i]->tv.runs;
   }
   int blocks = 0;
   if (walk) {
@@ -3061,8 +3100,8 @@ int mccfr_batch_round(mccfr_handle* const* tables, int n, const int* traversals,
   }
   // a warp of the apply kernel per four bitmap words of the largest table
   const int ablocks = (int)std::min(148u, (words + 31) / 32);
-  k_apply_batched<<<dim3(std::max(1, ablocks), n), kApplyBlock, 0, stream>>>(R.d_up()->tables, &R.d_up()->phase,
-                                                                             R.d_err());
+  const auto apply = runs ? k_apply_batched<true> : k_apply_batched<false>;
+  apply<<<dim3(std::max(1, ablocks), n), kApplyBlock, 0, stream>>>(R.d_up()->tables, &R.d_up()->phase, R.d_err());
   BCK(cudaGetLastError());
   // every table's error flag in one copy
   BCK(cudaMemcpyAsync(R.h_err(), R.d_err(), n * sizeof(int), cudaMemcpyDeviceToHost, stream));
