@@ -121,6 +121,12 @@ def table_bytes(req: Request) -> int:
     return capacity_bytes(req.table_log2)
 
 
+def alone_bytes(table_log2: int) -> int:
+    """Of those, the bytes of the table itself and its small buffers: what a budget
+    has to hold for a request to be served at all."""
+    return (1 << table_log2) * 260 + (1 << 20)
+
+
 @dataclass
 class Solve:
     req: Request
@@ -150,7 +156,9 @@ class ReSolveServer:
     """Continuous-batching re-solver.
 
     hbm_budget: device bytes the server may hold in request tables, pooled ones
-    included (admission also requires that much free device memory);
+    included (admission also requires that much free device memory); a request whose
+    table fits the budget, but not with the scratch that reading it back leaves, is
+    served alone;
     max_active: requests batched per round (the persistent kernel takes up to 64
     tables); traversals: per player-update of each request.  Finished requests'
     tables are kept in a pool by capacity and reset for new requests of the
@@ -228,9 +236,11 @@ class ReSolveServer:
             return False
         if self.pool.get(req.table_log2):
             return True  # a pooled table of this capacity is reset, nothing is allocated
-        need = table_bytes(req)
+        need, alone = table_bytes(req), alone_bytes(req.table_log2)
         self._evict(need, held)
-        return held + self.pooled_bytes() + need <= self.hbm_budget and need + (1 << 30) <= self.free_memory()
+        others = held + self.pooled_bytes()
+        fits = others + need <= self.hbm_budget or (others == 0 and alone <= self.hbm_budget)
+        return fits and alone + (1 << 30) <= self.free_memory()
 
     def _start(self, req: Request, now: float) -> Solve:
         cfg = request_config(req)

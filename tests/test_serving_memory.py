@@ -30,6 +30,32 @@ def test_counted_bytes_cover_rows_bitmaps_and_kept_scratch(log2):
                                   else sv.table_bytes(req))
 
 
+@pytest.mark.parametrize("log2", [10, 14, 21])
+def test_a_table_that_fits_the_budget_is_served_alone(log2):
+    """The budget holds the table but not the scratch that it may leave: accepted on
+    an idle server (pooled tables freed for it), not beside another one."""
+    req = sv.make_request(np.random.default_rng(1), 0)
+    req.table_log2 = log2
+    own = (1 << log2) * 260 + (1 << 20)
+    assert own < sv.table_bytes(req)
+    for budget in (own, sv.table_bytes(req) - 1):
+        srv = sv.ReSolveServer(None, hbm_budget=budget, free_memory=lambda: own + (1 << 30))
+        assert srv.admit_ok(req, 0, 0)
+        assert not srv.admit_ok(req, 1, 1)
+        assert not sv.ReSolveServer(None, hbm_budget=own - 1, free_memory=lambda: 1 << 40).admit_ok(req, 0, 0)
+        assert not sv.ReSolveServer(None, hbm_budget=budget, free_memory=lambda: own + (1 << 30) - 1).admit_ok(req, 0, 0)
+
+        class Pooled:
+            closed = False
+
+            def close(self):
+                self.closed = True
+
+        other = Pooled()
+        srv.pool[9] = [other]
+        assert srv.admit_ok(req, 0, 0) and other.closed
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("log2", [18, 20])
 def test_device_memory_of_solved_tables_is_counted(hand_table, log2):
