@@ -296,9 +296,9 @@ int mccfr_eval7_device(mccfr_handle* h, const uint8_t* dev_cards,
                        uint16_t* dev_ranks, size_t n, float* ms);
 
 /* Level counts of the handle's last external-sampling update in the default or
-   the level-synchronous form: seeds[L] (level 0: the update's traversals) and updating-player
-   nodes[L] reached from level L, for L < min(cap, *levels), and the seeds left
-   to the depth-first walk because the buffers were full.  *levels = 0 before
+   the level-synchronous form: seeds[L] (level 0: the update's traversals) and
+   updating-player nodes[L] reached from level L, for L < min(cap, *levels), and
+   the seeds left to the depth-first walk because the buffers were full.  *levels = 0 before
    the first such update.  No reference counterpart (a tuning aid). */
 int mccfr_level_counts(mccfr_handle* h, uint32_t* seeds, uint32_t* nodes, int cap, int* levels,
                        uint32_t* deferred);
@@ -339,8 +339,8 @@ typedef struct mccfr_batch_tuning {
   int32_t warp_sync;      /* lanes that refill together share one grab of lanes x grab
                              traversals; 1: interleaved (neighbouring lanes take neighbouring
                              traversals), 0: each lane a contiguous run of `grab` */
-  int32_t form;           /* MCCFR_BATCH_* (mccfr_batch_train only; rounds always run the
-                             persistent kernel) */
+  int32_t form;           /* MCCFR_BATCH_* (mccfr_batch_train only; a round given a tuning
+                             runs the persistent kernel) */
   int32_t reserved[2];
 } mccfr_batch_tuning;
 /* Batch forms.  PERSISTENT: per phase one persistent traversal launch over all
@@ -405,10 +405,12 @@ int mccfr_subgame_reset(mccfr_handle* h, const mccfr_config* cfg, const mccfr_su
    outlive h).  Valid for subgames and for tables without rank-CDF buckets or
    with the same bucket counts as src. */
 int mccfr_share_hand_table(mccfr_handle* h, mccfr_handle* src);
-/* One player-update of each listed table, all in one persistent traversal
-   launch: the serving step of continuous batching.  Each table advances its
+/* One player-update of each listed table, all in one traversal launch: the
+   serving step of continuous batching.  Each table advances its
    own (iteration, player) and its iteration count after its last player.
-   traversals[i] = traversals of table i's update; tuning may be NULL. */
+   traversals[i] = traversals of table i's update.  tuning NULL: the walk form
+   where every table's config runs it (MCCFR_FORM_AUTO); otherwise, and with a
+   tuning, the persistent depth-first kernel. */
 int mccfr_batch_round(mccfr_handle* const* tables, int n, const int* traversals,
                       const mccfr_batch_tuning* tuning);
 /* The (iteration, player) the table's next update will run, and the number of

@@ -59,8 +59,9 @@ namespace {
 // time, one lane per row in nearly ascending address order.  The bytes of the rows
 // are what it costs: a lane has its row's whole first line in flight at once (and
 // da for a wide row), and writes only what changed.  At 2^20 traversals of 6-max
-// 100BB it folds 26.7 M rows in 1.85 ms, 14.4 rows/ns (58% of the measured copy
-// bandwidth by the bytes it needs); eight lanes per row over a list of touched rows
+// 100BB it folds the 26.5 M rows (10.0 M wide) of iteration 6's last update in 1.79 ms,
+// 14.8 rows/ns, and iteration 25's 33.9 M (17.3 M) in 2.50: 58% of the measured copy
+// bandwidth by the bytes they need (192 a row, 160 more a wide one); eight lanes per row over a list of touched rows
 // in random order, the second line read for every row, folded 8.5 rows/ns.
 // `group` of `ngroups`: the warps working on this table.
 constexpr int kApplyBlock = 256;
@@ -1002,8 +1003,8 @@ int max_decisions(const mccfr_handle* h) {
 }
 
 // Traversal form of an external-sampling update.  The walk form unless the
-// config asks for another (6-max at 2^20 traversals per update: 5.8 ms against the
-// level kernels' 14.4; 1,000 heads-up traversals: 60 us against 220).  It keeps one
+// config asks for another (6-max at 2^20 traversals per update, iterations 6-25: 7.0 ms
+// against the level kernels' 16.4; 1,000 heads-up traversals: 60 us against 220).  It keeps one
 // node record per decision in reserve, so paths longer than its level counters (no
 // raise cap and a deep depth cut) take the level-synchronous kernels, which leave
 // the deepest level to the depth-first walk.

@@ -37,9 +37,9 @@
 // What bounds it: the dependent issue of a step's code (about 1,450 instructions for
 // 23 decisions; 41% of issue slots, no unit above half its rate) and, in tables far
 // beyond L2, random 64-byte accesses: 16 G visits/s in a 33 MB table, 10 G in one of
-// 17 GB.  6-max 100BB at 2^20 traversals per update took the level kernels 14.4 ms
-// (expand 10.8, back 3.0, showdowns 0.5) and takes this one 5.8-6.1 ms; a 1,000-
-// traversal heads-up update 220 us and 60 us.  Six blocks of 80 registers per SM:
+// 17 GB.  6-max 100BB at 2^20 traversals per update takes the level kernels 12.5 ms
+// in iteration 6 and 16.4 in the mean of iterations 6-25, this one 5.6 and 7.0; a
+// 1,000-traversal heads-up update took them 220 us and takes this one 60 us.  Six blocks of 80 registers per SM:
 // five and seven are within 3%, eight spill and are 5% slower.
 #pragma once
 #include "game.cuh"

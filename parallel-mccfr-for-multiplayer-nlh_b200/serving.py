@@ -4,7 +4,7 @@ Requests are turn or river subgames (board, 2-6 players, pot, one 1326-combo
 range per player, bet sizes, iteration budget).  The server keeps every admitted
 request's regret table resident on the device and runs rounds: each round is
 one mccfr_batch_round call, i.e. one player-update of every active request in a
-single persistent traversal launch.  Requests that arrive while others run are
+single traversal launch.  Requests that arrive while others run are
 admitted between rounds as soon as a slot and device memory are free, and a
 request retires (its strategy is copied to the host) as soon as its budget is
 spent, so solves overlap on the device.  A request's result depends only on its
@@ -158,8 +158,7 @@ class ReSolveServer:
     hbm_budget: device bytes the server may hold in request tables, pooled ones
     included (admission also requires that much free device memory); a request whose
     table fits the budget, but not with the scratch that reading it back leaves, is
-    served alone;
-    max_active: requests batched per round (the persistent kernel takes up to 64
+    served alone; max_active: requests batched per round (a round takes up to 64
     tables); traversals: per player-update of each request.  Finished requests'
     tables are kept in a pool by capacity and reset for new requests of the
     same capacity (mccfr_subgame_reset), so a steady stream of requests
@@ -176,8 +175,8 @@ class ReSolveServer:
     host logic can run against stand-ins.
 
     retire_workers > 0 moves retiring off the round loop: a finished request's
-    strategy is exported (a counting pass, a compaction and a copy on its own
-    handle's stream, then the host sort) by a worker thread while the loop goes
+    strategy is exported (a counting pass, a pass that writes the rows in key order
+    and a copy, on its own handle's stream) by a worker thread while the loop goes
     on running rounds for the others; its table counts against the budget until
     the export is done and then returns to the pool.  0 retires in the loop."""
 

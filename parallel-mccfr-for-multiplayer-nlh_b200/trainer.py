@@ -213,7 +213,7 @@ class GPUCFRTrainer:
 
     def level_counts(self) -> dict:
         """Per-level seeds and updating-player nodes of the last external-sampling
-        update in the level-synchronous form (mccfr_level_counts)."""
+        update in the walk or the level-synchronous form (mccfr_level_counts)."""
         seeds = np.zeros(64, np.uint32)
         nodes = np.zeros(64, np.uint32)
         n, deferred = ctypes.c_int(), ctypes.c_uint32()
@@ -322,7 +322,7 @@ class Batch:
 
 
 def batch_round(trainers: list, traversals: list[int], tuning: dict | None = None) -> None:
-    """One player-update of every listed trainer in one persistent launch
+    """One player-update of every listed trainer in one traversal launch
     (continuous batching step, mccfr_batch_round)."""
     lib = L.load()
     arr = (ctypes.c_void_p * len(trainers))(*[t.handle.value for t in trainers])
