@@ -705,7 +705,10 @@ struct mccfr_handle {
 
 namespace {
 
+// A call that failed for want of memory leaves its error with the runtime, where the
+// next call's check of its launches would find it: it is taken back here.
 int fail(mccfr_handle* h, int code, const char* fmt, ...) {
+  if (code == MCCFR_ERR_OOM || code == MCCFR_ERR_CUDA) cudaGetLastError();
   if (h) {
     char buf[512];
     va_list ap;
@@ -2372,6 +2375,7 @@ struct mccfr_batch {
 namespace {
 
 int bfail(mccfr_batch* b, int code, const char* msg) {
+  if (code == MCCFR_ERR_OOM || code == MCCFR_ERR_CUDA) cudaGetLastError();
   if (b) b->last_error = msg;
   fprintf(stderr, "mccfr_batch: %s\n", msg);
   return code;
@@ -2921,6 +2925,7 @@ int mccfr_create_subgame(const mccfr_config* cfg, const mccfr_subgame* sg, mccfr
   if (cudaMalloc(&h->d_ranges, (size_t)MCCFR_MAX_PLAYERS * 1326 * 4) != cudaSuccess ||
       cudaMemcpyAsync(h->d_ranges, cdf.data(), cdf.size() * 4, cudaMemcpyHostToDevice, h->stream) != cudaSuccess ||
       cudaStreamSynchronize(h->stream) != cudaSuccess) {
+    cudaGetLastError();
     mccfr_destroy(h);
     *out = nullptr;
     return MCCFR_ERR_OOM;
